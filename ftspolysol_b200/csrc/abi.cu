@@ -626,6 +626,7 @@ unsigned char* g_noalloc_base[NA_MAX_DEVICES] = {};
 struct NoallocTables {
     ftsp::FftPlan1 plans[3];                 // x, y, z
     double2 tw[3][NOALLOC_MAX_EXTENT];       // exp(-2 pi i j / m_d)
+    double2 split[5 * NOALLOC_MAX_EXTENT];   // twiddle tables of the split-y passes
     double phi[3 * NOALLOC_MAX_EXTENT];      // separable exp(-b^2 k_d^2 / 6)
     double qsum[2];                          // sum of q_N (combine output)
 };
@@ -691,6 +692,17 @@ extern "C" int ftsp_propagate_chain_noalloc(int m1, int m2, int m3, double L1, d
                 ht.tw[d][j] = make_double2((double)cosl(ang), (double)sinl(ang));
             }
         }
+        SplitGeom sg{};
+        if (split_setup(sg, m1, m2, m3, (int)sizeof(double2))) {
+            const int first[3] = {m1, m2, m3};
+            const std::vector<double2> t = split_tables<double2>(sg, [&](int n, int j) {
+                for (int d = 0; d < 3; ++d)
+                    if (first[d] == n) return ht.tw[d][j];
+                return make_double2(1.0, 0.0);   // not reached: n is an extent
+            });
+            std::copy(t.begin(), t.end(), ht.split);
+            split_point_tables(sg, (const double2*)dtab->split);
+        }
         int off = 0;
         for (int d = 0; d < 3; ++d)
             for (int i = 0; i < ms[d]; ++i) {
@@ -729,7 +741,7 @@ extern "C" int ftsp_propagate_chain_noalloc(int m1, int m2, int m3, double L1, d
         const size_t y_smem = std::max(sizeof(double2) * ((size_t)m2 * W + m2), (size_t)4096);
         const size_t z_smem = std::max(sizeof(double2) * ((size_t)B * (m3 + 1) + m3), (size_t)4096);
         if (x_threads > 256 || y_threads > 256 || z_threads > 256) throw std::runtime_error("ftsp_propagate_chain_noalloc: mesh too large for the line passes");
-        const int parts = plane_ok ? m1 : m1 * m2 / B;
+        const int parts = sg.ok ? m1 * (sg.Y2 / sg.G) : plane_ok ? m1 : m1 * m2 / B;
         if ((size_t)parts > NA_PARTIALS_N) throw std::runtime_error("ftsp_propagate_chain_noalloc: too many reduction partials");
         const double2* tw1 = dtab->tw[0];
         const double2* tw2 = dtab->tw[1];
@@ -737,10 +749,30 @@ extern "C" int ftsp_propagate_chain_noalloc(int m1, int m2, int m3, double L1, d
         auto smem_attr = [&](auto kernel, size_t bytes) {
             if (bytes > 48 * 1024) FTSP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
         };
-        // real-space pass of one segment (plane, or y / z-line / y)
+        // dependent launch: the kernel's prologue overlaps the one before it
+        auto launch = [&](auto kernel, int grid, int threads, size_t smem, const double2* src, double2* dst, const auto& op) {
+            smem_attr(kernel, smem);
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(grid);
+            cfg.blockDim = dim3(threads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = stream;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            FTSP_CUDA(cudaLaunchKernelEx(&cfg, kernel, sg, src, dst, V, op));
+        };
+        // real-space pass of one segment (split-y pass, plane, or y / z-line / y)
         auto seg = [&](auto s1c, auto s2c, const double2* src, double2* dst, const auto& op) {
             constexpr int S1 = decltype(s1c)::value, S2 = decltype(s2c)::value;
             using Op = std::decay_t<decltype(op)>;
+            if (sg.ok) {
+                if (sg.big) launch(k_split_real<double, RtBigPlan, S1, S2, Op>, parts, sg.r_threads, split_real_smem<RtBigPlan, double2>(sg), src, dst, op);
+                else launch(k_split_real<double, RtPlan, S1, S2, Op>, parts, sg.r_threads, split_real_smem<RtPlan, double2>(sg), src, dst, op);
+                return;
+            }
             if (plane_ok) {
                 auto k = k_plane<double, EP, S1, S2, Op>;
                 smem_attr(k, plane_smem);
@@ -766,8 +798,17 @@ extern "C" int ftsp_propagate_chain_noalloc(int m1, int m2, int m3, double L1, d
         ob.phiy = dtab->phi + m1;
         ob.phiz = dtab->phi + m1 + m2;
         ob.invV = 1.0 / (double)V;
-        auto kb = k_strided<double, EL, 0, -1, +1, OpBond<double, true, false>>;
-        smem_attr(kb, x_smem);
+        auto bond = [&] {
+            using OB = OpBond<double, true, false>;
+            if (sg.ok) {
+                if (sg.big) launch(k_split_k<double, RtBigPlan, -1, +1, OB>, sg.Y1 * sg.nzb, sg.k_threads, split_k_smem<RtBigPlan, double2>(sg), Gb, Gb, ob);
+                else launch(k_split_k<double, RtPlan, -1, +1, OB>, sg.Y1 * sg.nzb, sg.k_threads, split_k_smem<RtPlan, double2>(sg), Gb, Gb, ob);
+                return;
+            }
+            auto kb = k_strided<double, EL, 0, -1, +1, OB>;
+            smem_attr(kb, x_smem);
+            kb<<<dim3(m2 * (m3 / W), 1), x_threads, x_smem, stream>>>(gx, Gb, Gb, V, tw1, ob);
+        };
 
         const double2* wp = reinterpret_cast<const double2*>(w);
         double2* qe = reinterpret_cast<double2*>(q_end);
@@ -790,7 +831,7 @@ extern "C" int ftsp_propagate_chain_noalloc(int m1, int m2, int m3, double L1, d
             op0.E = Eb; op0.qstore = qe;
             seg(I0{}, Im{}, nullptr, Gb, op0);
             for (int b = 0; b < N - 1; ++b) {
-                kb<<<dim3(m2 * (m3 / W), 1), x_threads, x_smem, stream>>>(gx, Gb, Gb, V, tw1, ob);
+                bond();
                 if (b + 1 < N - 1) {
                     OpProp<double, FWD_MID> op{};
                     op.E = Eb; op.qstore = qe;

@@ -26,6 +26,7 @@
 
 #include "passes.cuh"
 #include "chain_pairs.cuh"
+#include "split_passes.cuh"
 #include "learned.cuh"
 #include "ftsp.h"
 
@@ -932,6 +933,11 @@ struct Engine : EngineBase {
     Buf<V> si_inc;       // semi-implicit increments (nm + 1 fields)
     Buf<V> ck;           // device checkpoint of (omega, psi) for rollback
     Buf<float> pmax;     // per-CTA propagator maxima, two slots (ping-pong by segment parity)
+    SplitGeom sg{};      // split-y passes of the chain sweeps (split_passes.cuh)
+    Buf<V> split_tw;     // their twiddle tables
+    bool use_split = false;
+    Buf<float> smax;     // their propagator maxima: per species, forward [N], backward [N]; zeroed by eval
+    std::vector<size_t> smax0;   // first slot of each species
     Buf<double> spart;   // stress partials [ncta_x * 6] complex
     // mirror-symmetric species: pair tables of the density and stress kernels
     Buf<int2> pair_ix;
@@ -945,8 +951,7 @@ struct Engine : EngineBase {
     std::vector<SymTables> sym;
     bool chain_sym = true;       // use the pair kernels for mirror-symmetric species
     bool fused_strided = true;   // bond passes with register-resident middle stages (k_strided_fused)
-    bool fused_plane = true;     // mid segment passes with register-resident end stages (k_plane_fused)
-    bool zreg_plane = true;      // forward mid passes of 128^2 complex64 planes: z pair in registers (k_plane_zreg)
+    bool fused_plane = true;     // field loads with a register-resident first stage (k_plane_load_fused)
     // every ion smeared like the beads (and at most 3 ion species): the ion
     // potentials are psi_s itself, and the ion charge is one combined field
     // sum_j z_j (n_j/V)/Q_j exp(-i z_j psi_s), transformed once (see eval)
@@ -995,6 +1000,7 @@ struct Engine : EngineBase {
         plans.release();
         kx.release(); ky.release(); kz.release(); phi.release(); gam.release(); gion.release(); eta.release();
         part.release(); spart.release(); stage.release(); expo.release(); pmax.release();
+        split_tw.release(); smax.release();
         pair_ix.release(); pair_wt.release(); pair_run.release();
         si_G.release(); si_inc.release(); ck.release();
         avg.acc.release();
@@ -1066,6 +1072,8 @@ struct Engine : EngineBase {
         z_threads = round32((B * m3 + EL - 1) / EL);
         z_smem = std::max(sizeof(V) * ((size_t)B * (m3 + 1) + m3), (size_t)32 * 16 * 8);
         if (x_threads > 256 || y_threads > 256 || z_threads > 256) throw std::runtime_error("grid dimension too large for the line passes");
+        if (!sg.m1) split_setup(sg, m1, m2, m3, (int)sizeof(V));
+        use_split = sg.ok;
     }
 
     void allocate()
@@ -1099,6 +1107,13 @@ struct Engine : EngineBase {
         part.alloc((size_t)std::max(RED_BLOCKS, std::max(c.m1, c.m1 * c.m2)) * 32);
         expo.alloc((size_t)2 * Nmax);
         pmax.alloc((size_t)2 * std::max(c.m1, c.m1 * c.m2));
+        size_t slots = 0;
+        for (auto& s : c.sp) {
+            smax0.push_back(slots);
+            slots += 2 * (size_t)s.N;
+        }
+        smax.alloc(std::max<size_t>(1, slots));
+        split_tw.alloc((size_t)2 * c.m1 + c.m2 + 2 * c.m3);
         spart.alloc((size_t)c.m2 * c.m3 * 12);
         if (c.restart_interval > 0) ck.alloc((size_t)(std::max(1, c.nm) + 1) * V_);
         FTSP_CUDA(cudaMalloc(&ds, sizeof(DevScal)));
@@ -1234,6 +1249,16 @@ struct Engine : EngineBase {
             }
             return t;
         };
+        if (sg.ok) {
+            upload(split_tw, split_tables<V>(sg, [&](int n, int j) {
+                const long double ang = -2.0L * 3.141592653589793238462643383279502884L * j / n;
+                V w;
+                w.x = (T)cosl(ang);
+                w.y = (T)sinl(ang);
+                return w;
+            }));
+            split_point_tables(sg, (const V*)split_tw.p);
+        }
         upload(tw1, tw(c.m1));
         upload(tw2, tw(c.m2));
         upload(tw3, tw(c.m3));
@@ -2075,26 +2100,6 @@ struct Engine : EngineBase {
                 return;
             }
         }
-        if constexpr (S1 != 0 && S2 != 0 && F32 && N == 128 && NT == 1024 && op_loads<Op>::value <= 1) {
-            if (zreg_plane) {
-                auto k = k_plane_zreg<T, S1, S2, Op>;
-                // tile of 128 x ZREG_P values, the twiddles, the [t][i] and [t][b] twiddle tables
-                const size_t zsmem = sizeof(V) * ((size_t)128 * ZREG_P + 128 + 128 + 128);
-                set_smem(k, zsmem);
-                launch_pass(k, dim3(c.m1, nf), NT, zsmem, src, dst, (size_t)V_, (const V*)tw3.p, op);
-                ++launches;
-                return;
-            }
-        }
-        if constexpr (S1 != 0 && S2 != 0 && plane_fused_ok<N, RMAX, NT, E>()) {
-            if (fused_plane) {
-                auto k = k_plane_fused<T, N, RMAX, NT, E, S1, S2, Op>;
-                set_smem(k, smem);
-                launch_pass(k, dim3(c.m1, nf), NT, smem, src, dst, (size_t)V_, (const V*)tw3.p, op);
-                ++launches;
-                return;
-            }
-        }
         auto k = k_plane_ct<T, N, RMAX, NT, E, S1, S2, Op>;
         set_smem(k, smem);
         launch_pass(k, dim3(c.m1, nf), NT, smem, src, dst, (size_t)V_, (const V*)tw3.p, op);
@@ -2112,6 +2117,12 @@ struct Engine : EngineBase {
             if constexpr (plane_ct_ok<32>())
                 if (c.m3 == 32) return plane_ct<32, S1, S2>(src, dst, nf, op);
         }
+        plane_rt<S1, S2>(src, dst, nf, op);
+    }
+    // the run-time plan (the only one that the sweeps of a grid without split passes use)
+    template <int S1, int S2, class Op>
+    void plane_rt(const V* src, V* dst, int nf, const Op& op)
+    {
         auto kp = k_plane<T, EP, S1, S2, Op>;
         set_smem(kp, plane_smem);
         kp<<<dim3(c.m1, nf), plane_threads, plane_smem, stream>>>(pg, src, dst, V_, tw2.p, tw3.p, op);
@@ -2186,6 +2197,11 @@ struct Engine : EngineBase {
                 return strided_ct<DIM, 32, S1, S2>(src, dst, nf, op);
             }
         }
+        strided_rt<DIM, S1, S2>(src, dst, nf, op);
+    }
+    template <int DIM, int S1, int S2, class Op>
+    void strided_rt(const V* src, V* dst, int nf, const Op& op)
+    {
         if constexpr (op_has_src<Op>::value) {
             throw std::runtime_error("pencil op with a source map needs the fused pencil pass");
         } else {
@@ -2214,6 +2230,11 @@ struct Engine : EngineBase {
                 return;
             }
         }
+        zline_rt<S1, S2>(src, dst, nf, op);
+    }
+    template <int S1, int S2, class Op>
+    void zline_rt(const V* src, V* dst, int nf, const Op& op)
+    {
         auto k = k_zline<T, EL, S1, S2, Op>;
         set_smem(k, z_smem);
         k<<<dim3(c.m1 * c.m2 / gz.B, nf), z_threads, z_smem, stream>>>(gz, src, dst, V_, tw3.p, op);
@@ -2243,6 +2264,59 @@ struct Engine : EngineBase {
         strided<0, 0, S>(nullptr, dst, nf, self);
         // two passes (three without the plane pass), each reading and writing every field
         prof_end(ev, "field_fft", (plane_ok ? 4.0 : 6.0) * nf * sizeof(V) * (double)V_);
+    }
+
+    // ---- split-y passes (split_passes.cuh) ----
+    template <class P, int S1, int S2, class Op>
+    void split_real_plan(const V* src, V* dst, int nf, const Op& op)
+    {
+        auto k = k_split_real<T, P, S1, S2, Op>;
+        const SplitGeom& p = P::CT ? P::G : sg;
+        const size_t smem = split_real_smem<P, V>(p);
+        set_smem(k, smem);
+        launch_pass(k, dim3(p.m1 * (p.Y2 / p.G), nf), p.r_threads, smem, sg, src, dst, (size_t)V_, op);
+        ++launches;
+    }
+    template <class P, int S1, int S2, class Op>
+    void split_k_plan(const V* src, V* dst, int nf, const Op& op)
+    {
+        auto k = k_split_k<T, P, S1, S2, Op>;
+        const SplitGeom& p = P::CT ? P::G : sg;
+        const size_t smem = split_k_smem<P, V>(p);
+        set_smem(k, smem);
+        launch_pass(k, dim3(p.Y1 * p.nzb, nf), p.k_threads, smem, sg, src, dst, (size_t)V_, op);
+        ++launches;
+    }
+    int cube() const { return c.m1 == c.m2 && c.m2 == c.m3 ? c.m1 : 0; }
+    template <int S1, int S2, class Op>
+    void split_real(const V* src, V* dst, int nf, const Op& op)
+    {
+        // the passes at the ends of a sweep (one transform) run once: the
+        // run-time plan serves them
+        if constexpr (S1 != 0 && S2 != 0) switch (cube()) {
+            case 32: return split_real_plan<CubePlan<32, T>, S1, S2>(src, dst, nf, op);
+            case 48: return split_real_plan<CubePlan<48, T>, S1, S2>(src, dst, nf, op);
+            case 64: return split_real_plan<CubePlan<64, T>, S1, S2>(src, dst, nf, op);
+            case 96: return split_real_plan<CubePlan<96, T>, S1, S2>(src, dst, nf, op);
+            case 128: return split_real_plan<CubePlan<128, T>, S1, S2>(src, dst, nf, op);
+            default: break;
+        }
+        if (sg.big) return split_real_plan<RtBigPlan, S1, S2>(src, dst, nf, op);
+        split_real_plan<RtPlan, S1, S2>(src, dst, nf, op);
+    }
+    template <int S1, int S2, class Op>
+    void split_k(const V* src, V* dst, int nf, const Op& op)
+    {
+        switch (cube()) {
+            case 32: return split_k_plan<CubePlan<32, T>, S1, S2>(src, dst, nf, op);
+            case 48: return split_k_plan<CubePlan<48, T>, S1, S2>(src, dst, nf, op);
+            case 64: return split_k_plan<CubePlan<64, T>, S1, S2>(src, dst, nf, op);
+            case 96: return split_k_plan<CubePlan<96, T>, S1, S2>(src, dst, nf, op);
+            case 128: return split_k_plan<CubePlan<128, T>, S1, S2>(src, dst, nf, op);
+            default: break;
+        }
+        if (sg.big) return split_k_plan<RtBigPlan, S1, S2>(src, dst, nf, op);
+        split_k_plan<RtPlan, S1, S2>(src, dst, nf, op);
     }
 
     // Real-space pass of one segment: [inverse S1] op [forward S2] with the
@@ -2281,28 +2355,39 @@ struct Engine : EngineBase {
     void seg_pass_launch(const V* src, V* dst, const OpProp<T, KIND>& op)
     {
         using OpLoadOne = ftsp::OpLoadOne<T>;
+        if (use_split) {
+            split_real<S1, S2>(src, dst, 1, op);
+            return;
+        }
         if (plane_ok) {
-            plane<S1, S2>(src, dst, 1, op);
+            plane_rt<S1, S2>(src, dst, 1, op);
             return;
         }
         if (S1 != 0) strided<1, 0, S1>(nullptr, const_cast<V*>(src), 1, OpLoadOne{src});   // y-lines, in place
-        zline<S1, S2>(src, dst, 1, op);
+        zline_rt<S1, S2>(src, dst, 1, op);
         if (S2 != 0) strided<1, 0, S2>(nullptr, dst, 1, OpLoadOne{dst});                    // y-lines, in place
     }
 
     int seg_pass_ctas() const
     {
+        if (use_split) return sg.m1 * (sg.Y2 / sg.G);
         if (plane_ok) return c.m1;
-        if (!F32 && c.m3 == 128 && (c.m1 * c.m2) % 16 == 0) return c.m1 * c.m2 / 16;
         return c.m1 * c.m2 / gz.B;
     }
+    // blocks that write connectivity-stress partials: the pair kernel's (x_ctas)
+    // and, with the split passes, the backward bond pass's
+    int stress_parts() const { return std::max(x_ctas(), use_split ? sg.Y1 * sg.nzb : 0); }
     int x_ctas() const { return c.m2 * (c.m3 / (strided_is_ct(c.m1) ? WCT : gx.W)); }
 
     template <int S1, int S2, bool FWD, bool STRESS>
     void bond_pass(const V* src, V* dst, const OpBond<T, FWD, STRESS>& op)
     {
         cudaEvent_t ev = prof_begin();
-        strided<0, S1, S2>(src, dst, 1, op);
+        if (use_split) {
+            split_k<S1, S2>(src, dst, 1, op);
+        } else {
+            strided_rt<0, S1, S2>(src, dst, 1, op);
+        }
         // G in, H out, plus the stored/read forward spectrum when the stress is on
         const bool extra = FWD ? op.Fstore != nullptr : STRESS;
         prof_end(ev, std::string("bond_") + (FWD ? "fwd" : "bwd") + (extra ? (FWD ? "_storeF" : "_stress") : ""),
@@ -2321,7 +2406,7 @@ struct Engine : EngineBase {
         double2* factor = &ds->factor[isp];
         double* qpart = part.p;
         // renormalisation bookkeeping (see Renorm in passes.cuh)
-        const int nparts = seg_pass_ctas();
+        const int nparts = use_split ? 0 : seg_pass_ctas();
         const size_t pslot = (size_t)std::max(c.m1, c.m1 * c.m2);
         auto pm = [&](int s) { return pmax.p + (size_t)(s & 1) * pslot; };
         auto rn = [&](int s) {
@@ -2333,6 +2418,18 @@ struct Engine : EngineBase {
             r.N = N;
             r.pmax_cur = pm(s);
             r.pmax_prev = pm(s + 1);   // the pass before: segment s-1 (forward) or s+1 (backward), other parity
+            if (use_split) {
+                r.pmax_cur = smax.p + smax0[isp] + s;
+                r.pmax_prev = r.pmax_cur - 1;
+            }
+            return r;
+        };
+        auto rnb = [&](int s) {   // the same of the backward sweep
+            Renorm r = rn(s);
+            if (use_split) {
+                r.pmax_cur = smax.p + smax0[isp] + N + s;
+                r.pmax_prev = r.pmax_cur + 1;
+            }
             return r;
         };
         // ---- forward sweep ----
@@ -2395,14 +2492,14 @@ struct Engine : EngineBase {
         if (N == 1) {
             OpProp<T, BWD_SINGLE> op{};
             op.qread = qf(0); op.rho_type = rho_of(0); op.rho_charge = rchg(0); op.z = (T)s.charge[0]; op.factor = factor;
-            op.rn = rn(0);
+            op.rn = rnb(0);
             seg_pass<0, 0, BWD_SINGLE>(nullptr, nullptr, op);
             return;
         }
         {
             OpProp<T, BWD_START> op{};
             op.E = Ec(N - 1); op.qread = qf(N - 1); op.rho_type = rho_of(N - 1); op.rho_charge = rchg(N - 1);
-            op.z = (T)s.charge[N - 1]; op.factor = factor; op.rn = rn(N - 1);
+            op.z = (T)s.charge[N - 1]; op.factor = factor; op.rn = rnb(N - 1);
             seg_pass<0, +1, BWD_START>(nullptr, G.p, op);
         }
         for (int b = N - 2; b >= 0; --b) {
@@ -2426,12 +2523,12 @@ struct Engine : EngineBase {
             if (b > 0) {
                 OpProp<T, BWD_MID> op{};
                 op.E = Ec(b); op.qread = qf(b); op.rho_type = rho_of(b); op.rho_charge = rchg(b);
-                op.z = (T)s.charge[b]; op.factor = factor; op.rn = rn(b);
+                op.z = (T)s.charge[b]; op.factor = factor; op.rn = rnb(b);
                 seg_pass<-1, +1, BWD_MID>(H.p, G.p, op);
             } else {
                 OpProp<T, BWD_LAST> op{};
                 op.qread = qf(0); op.rho_type = rho_of(0); op.rho_charge = rchg(0);
-                op.z = (T)s.charge[0]; op.factor = factor; op.rn = rn(0);
+                op.z = (T)s.charge[0]; op.factor = factor; op.rn = rnb(0);
                 seg_pass<-1, 0, BWD_LAST>(H.p, nullptr, op);
             }
         }
@@ -2742,6 +2839,8 @@ struct Engine : EngineBase {
             const V* kBp = kB.p;
             V* Ep = E.p;
             V* dBp = dB.p;
+            float* slot = smax.p;
+            const size_t slots = use_split ? smax.n : 0;
             if (ion_common) {
                 // the Boltzmann factors exp(-i z_j psi_s) are only summed here
                 // (Q_j); the combined ion charge is formed after the sweeps
@@ -2749,6 +2848,7 @@ struct Engine : EngineBase {
                 const int t0 = ct.type[0];
                 const T z0 = (T)ct.z[0];
                 reduce<6>(Vn, [=] __device__(size_t i, double* acc) {
+                    for (size_t k = i; k < slots; k += Vn) slot[k] = 0.0f;
                     const V ps_ = __ldg(kBp + (size_t)M * Vn + i);
                     {
                         V w = __ldg(kBp + (size_t)t0 * Vn + i);
@@ -2789,6 +2889,7 @@ struct Engine : EngineBase {
                 ++launches;
             } else {
                 foreach(Vn, [=] __device__(size_t i) {
+                    for (size_t k = i; k < slots; k += Vn) slot[k] = 0.0f;
                     const V ps_ = kBp[(size_t)M * Vn + i];
                     for (int k = 0; k < ncls; ++k) {
                         V w = kBp[(size_t)ct.type[k] * Vn + i];
@@ -2808,7 +2909,7 @@ struct Engine : EngineBase {
                 }, (double)(2 * (c.M + 1 + J) + (int)c.cls.size()) * sizeof(V));
             }
         }
-        if (stress) FTSP_CUDA(cudaMemsetAsync(spart.p, 0, sizeof(double) * 12 * (size_t)x_ctas(), stream));
+        if (stress) FTSP_CUDA(cudaMemsetAsync(spart.p, 0, sizeof(double) * 12 * (size_t)stress_parts(), stream));
         // 4. chain propagators of every species
         for (int isp = 0; isp < (int)c.sp.size(); ++isp) solve_species(isp, stress);
         if (!fx) charge_fold();
@@ -3378,7 +3479,7 @@ struct Engine : EngineBase {
     void finalize_record(bool with_stress)
     {
         if (with_stress) {
-            k_combine<false><<<12, COMBINE_THREADS, 0, stream>>>(spart.p, x_ctas(), 12, ds->sconn);
+            k_combine<false><<<12, COMBINE_THREADS, 0, stream>>>(spart.p, stress_parts(), 12, ds->sconn);
             ++launches;
         }
         const int S = (int)c.sp.size(), J = (int)c.ions.size(), nm = c.nm;

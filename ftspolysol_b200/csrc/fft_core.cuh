@@ -182,7 +182,7 @@ struct FastDiv {
     unsigned d, m, s;
 };
 __device__ __forceinline__ unsigned fdiv(unsigned n, const FastDiv& f) { return (__umulhi(n, f.m) + n) >> f.s; }
-inline FastDiv make_fastdiv(unsigned d)
+constexpr FastDiv make_fastdiv(unsigned d)
 {
     FastDiv f{d, 0u, 0u};
     if (d <= 1) return f;

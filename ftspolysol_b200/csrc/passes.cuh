@@ -318,7 +318,9 @@ struct OpIdentity {
 
 // Power-of-two renormalisation of the propagators (all optional: a null eF
 // turns it off).  Each real-space segment pass records, per CTA, the largest
-// component magnitude of the propagator it wrote (pmax_cur); the next pass of
+// component magnitude of the propagator it wrote (pmax_cur), or one maximum
+// over the grid (nparts = 0: an atomic maximum into a slot of the segment, which
+// the evaluation has zeroed; order-independent); the next pass of
 // the same sweep reduces those maxima, scales its output by 2^-d with
 // d = floor(log2 max), and accumulates d into a per-segment exponent:
 //   qF[s] is stored as qF_true[s] 2^-aF[s],  qB[s] as qB_true[s] 2^-aB[s].
@@ -331,10 +333,12 @@ struct Renorm {
     int* eB;                 // backward exponents aB[0..N)
     const float* pmax_prev;  // per-CTA maxima written by the previous pass of this sweep
     float* pmax_cur;         // per-CTA maxima of this pass
-    int nparts;              // number of entries of pmax_prev
+    int nparts;              // number of entries of pmax_prev (0: one slot per segment)
     int s;                   // segment index of this pass
     int N;                   // segments of the species
 };
+
+__device__ __forceinline__ int max_exponent(float M) { return (M > 0.0f && isfinite(M)) ? ilogbf(M) : 0; }
 
 // the exponent floor(log2 max) of the previous pass's per-CTA maxima; m is
 // this thread's share of them (its strided elements), loaded beforehand
@@ -353,7 +357,7 @@ __device__ __forceinline__ int reduce_exponent_local(float m)
     __syncthreads();
     const float M = s_red[0];
     __syncthreads();
-    return (M > 0.0f && isfinite(M)) ? ilogbf(M) : 0;
+    return max_exponent(M);
 }
 
 __device__ __forceinline__ float local_max(const float* pm, int n)
@@ -420,9 +424,14 @@ struct OpProp {
     {
         preloaded = false;
         if ((KIND == FWD_MID || KIND == FWD_LAST || KIND == BWD_MID) && rn.eF) {
-            pm_local = local_max(rn.pmax_prev, rn.nparts);
+            pm_local = rn.nparts ? local_max(rn.pmax_prev, rn.nparts) : *rn.pmax_prev;
             preloaded = true;
         }
+    }
+    __device__ __forceinline__ int prev_exponent() const
+    {
+        if (rn.nparts == 0) return max_exponent(preloaded ? pm_local : *rn.pmax_prev);
+        return preloaded ? reduce_exponent_local(pm_local) : reduce_exponent(rn.pmax_prev, rn.nparts);
     }
     __device__ __forceinline__ void begin()
     {
@@ -435,13 +444,13 @@ struct OpProp {
             if (KIND == FWD_START || KIND == FWD_SINGLE) {
                 if (first) rn.eF[0] = 0;
             } else if (KIND == FWD_MID || KIND == FWD_LAST) {
-                const int d = preloaded ? reduce_exponent_local(pm_local) : reduce_exponent(rn.pmax_prev, rn.nparts);
+                const int d = prev_exponent();
                 oscale = (T)ldexp(1.0, -d);
                 if (first) rn.eF[rn.s] = rn.eF[rn.s - 1] + d;
             } else if (KIND == BWD_START || KIND == BWD_SINGLE) {
                 if (first) rn.eB[rn.s] = 0;
             } else if (KIND == BWD_MID) {
-                const int d = preloaded ? reduce_exponent_local(pm_local) : reduce_exponent(rn.pmax_prev, rn.nparts);
+                const int d = prev_exponent();
                 oscale = (T)ldexp(1.0, -d);
                 if (first) rn.eB[rn.s] = rn.eB[rn.s + 1] + d;
                 dens_exp = rn.eF[rn.s] + rn.eB[rn.s + 1] - rn.eF[rn.N - 1];
@@ -534,7 +543,9 @@ struct OpProp {
             if (threadIdx.x == 0) {
                 float r = 0.0f;
                 for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w) r = fmaxf(r, sm[w]);
-                rn.pmax_cur[cta] = r;
+                // non-negative floats order like their bits
+                if (rn.nparts == 0) atomicMax(reinterpret_cast<int*>(rn.pmax_cur), __float_as_int(r));
+                else rn.pmax_cur[cta] = r;
             }
         }
     }
@@ -571,6 +582,7 @@ struct OpBond {
     // sums it fits 64 registers, so a 128^3 pass (1024 CTAs of 128 threads)
     // runs in one wave; with them, fewer registers would spill
     static constexpr int FUSED_MIN_BLOCKS = STRESS ? 2 : 8;
+    static constexpr int LOADS = STRESS ? 4 : 0;   // global loads per point (the stress sums need the registers of four)
     struct Pre {
         V F;
     };
@@ -708,15 +720,9 @@ __global__ void __launch_bounds__(NT, 1) k_plane_ct(const cplx<T>* src, cplx<T>*
     op.end(reinterpret_cast<double*>(tile), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
 }
 
-// Plane pass with both transforms (the mid segment passes), two
-// shared-memory round trips fewer than k_plane_ct: the inverse transform
-// runs along y first, and the coalesced load of thread tid (rows
+// Shapes of k_plane_load_fused: the coalesced load of a thread (rows
 // tid/N + u*NT/N of column tid%N) is the input set of its first radix stage
-// along y, so that stage runs on the loaded registers; the forward
-// transform ends along y, and its last stage stores its outputs (rows
-// i + t*SPAN of the column) straight to global memory.  Same grid, Op
-// interface and results (up to the rounding of the axis order) as
-// k_plane_ct.
+// along y.
 template <int N, int RMAX, int NT, int E>
 __host__ __device__ constexpr bool plane_fused_ok()
 {
@@ -726,82 +732,6 @@ __host__ __device__ constexpr bool plane_fused_ok()
     using AL = CtSt<N, RMAX, N, NT, NST - 1, false>;
     return A0::NB * A0::R == E && (A0::M * N) % NT == 0 && A0::TOTAL % NT == 0 && AL::NB * AL::R == E &&
            AL::TOTAL % NT == 0 && N * N == NT * E;
-}
-
-template <typename T, int N, int RMAX, int NT, int E, int S1, int S2, class Op>
-__global__ void __launch_bounds__(NT, 1) k_plane_fused(const cplx<T>* src, cplx<T>* dst, size_t fstride,
-                                                       const cplx<T>* __restrict__ twn, Op op)
-{
-    using V = cplx<T>;
-    constexpr int P = N + 1, NE = N * N;
-    constexpr int NST = ct_nst(N, RMAX);
-    static_assert(S1 != 0 && S2 != 0, "the fused plane pass runs both transforms");
-    static_assert(plane_fused_ok<N, RMAX, NT, E>(), "plane shape not supported by the fused pass");
-    using A0 = CtSt<N, RMAX, N, NT, 0, false>;          // first y stage (line = z column)
-    using AL = CtSt<N, RMAX, N, NT, NST - 1, false>;    // last y stage
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V* tile = reinterpret_cast<V*>(smem_raw);
-    V* stw = tile + N * P;
-    const int x = blockIdx.x;
-    const int f = blockIdx.y;
-    const size_t base = (size_t)f * fstride + (size_t)x * NE;
-    for (int j = threadIdx.x; j < N; j += NT) stw[j] = twn[j];
-    // the L2 prefetch of the pointwise operands goes out before the wait for
-    // the previous pass: a prefetch only moves lines into L2, the device's
-    // point of coherence, so it cannot observe a stale value, and the class
-    // table (the bulk of it) is not written during a sweep
-    if (threadIdx.x == 0) op.prefetch(base, (unsigned)NE);
-    pdl_wait();
-    op.preload();
-    V v[E];   // value u: row tid/N + u*NT/N, column tid%N
-#pragma unroll
-    for (int u = 0; u < E; ++u) v[u] = src[base + threadIdx.x + u * NT];
-    __syncthreads();   // twiddles in shared memory
-    {
-        V a[A0::NB][A0::R];
-#pragma unroll
-        for (int q = 0; q < A0::NB; ++q)
-#pragma unroll
-            for (int t = 0; t < A0::R; ++t) a[q][t] = v[q + t * (A0::M * N / NT)];
-        st_butterfly<S1, A0>(a, stw);
-        st_scatter<A0, P, 1>(tile, a);
-        __syncthreads();
-    }
-    st_range<V, S1, N, RMAX, N, P, 1, NT, false, 1, NST>(tile, stw);   // rest of y
-    ct_fft<V, S1, N, RMAX, N, 1, P, NT, E>(tile, stw);                  // z-lines
-    op.begin();
-    constexpr int EPT = NE / NT;
-    // loads in flight per batch: every FFT value is in shared memory here,
-    // so the registers hold the operands of PB points
-    constexpr int PB = (sizeof(T) == 4 && Op::LOADS <= 1) ? 16 : 4;
-#pragma unroll 1
-    for (int u0 = 0; u0 < EPT; u0 += PB) {
-        typename Op::Pre pre[PB];
-#pragma unroll
-        for (int k = 0; k < PB; ++k)
-            if (u0 + k < EPT) pre[k] = op.load(f, base + threadIdx.x + (u0 + k) * NT);
-#pragma unroll
-        for (int k = 0; k < PB; ++k)
-            if (u0 + k < EPT) {
-                const int e = threadIdx.x + (u0 + k) * NT;
-                const int y = e / N, z = e % N;
-                tile[y * P + z] = op.apply(f, x, y, z, base + e, tile[y * P + z], pre[k]);
-            }
-    }
-    pdl_trigger();
-    __syncthreads();
-    ct_fft<V, S2, N, RMAX, N, 1, P, NT, E>(tile, stw);                  // z-lines
-    st_range<V, S2, N, RMAX, N, P, 1, NT, false, 0, NST - 1>(tile, stw);
-    {
-        V a[AL::NB][AL::R];
-        st_gather<AL, P, 1>(tile, a);
-        st_butterfly<S2, AL>(a, stw);
-#pragma unroll
-        for (int q = 0; q < AL::NB; ++q)
-#pragma unroll
-            for (int t = 0; t < AL::R; ++t) dst[base + (size_t)AL::out_pos(q, t) * N + AL::line(q)] = a[q][t];
-    }
-    op.end(reinterpret_cast<double*>(tile), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
 }
 
 // Strided pass: lines of length N along y (DIM 1, outer index x) or x (DIM 0,
@@ -1198,38 +1128,6 @@ __global__ void __launch_bounds__(NT, 2) k_zline_ct(int m2, const cplx<T>* src, 
 }
 
 
-// ---------------------------------------------------------------------------
-// Plane pass of a mid segment for 128^2 complex64 planes, with the z-transform
-// pair around the pointwise step held in registers.
-//
-// The inverse transform runs y then z, the forward one z then y; both are
-// radix 16 x 8 per axis (Stockham, autosorting).  The inverse z-transform ends
-// with its radix-8 stage and the forward one starts with radix 8 (reversed
-// radix order), so one thread holds the outputs i + 16t (t < 8) of butterfly i
-// of a z-row, applies the pointwise op to them and runs the first forward
-// butterfly on the same registers: no shared-memory round trip for the
-// pointwise step, and none between the two z-transforms.  For those two
-// stages the 16 butterflies of a row go to 16 consecutive threads, so a
-// half-warp touches 16 consecutive z (128 bytes) of one row in global memory
-// (the op's loads and stores are coalesced).  The forward stage writes
-// positions 8i + t, a stride of 8 complex values; the tile's z index is
-// swizzled, z ^ ((z >> 4) & 7), which keeps every half-warp access of every
-// stage on 16 distinct 8-byte bank slots (rows are padded to ZREG_P values).
-// Every z stage works on rows that one warp owns, so the z phase needs no
-// block-wide barrier.
-//
-// Shared-memory round trips: 6 (y: 2, z: 2, z: 2 less the fused pair, y: 2
-// less the register-resident first and last stages); block barriers: 7.
-// Same grid, Op interface (forward ops: one load per point) and results, up
-// to the rounding of the operation order, as k_plane_fused.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ int plane_swz(int z) { return z ^ ((z >> 4) & 7); }
-
-// Row pitch of the k_plane_zreg tile: 136 values (272 banks = 16 mod 32), so
-// the two rows of a half-warp in the warp-owned z stages fall on opposite
-// halves of the banks; accesses along y keep one row per half-warp.
-constexpr int ZREG_P = 136;
-
 // Global loads per point of a pointwise op (Op::LOADS where declared, else 4).
 template <class Op, class = void>
 struct op_loads {
@@ -1240,182 +1138,12 @@ struct op_loads<Op, std::void_t<decltype(Op::LOADS)>> {
     static constexpr int value = Op::LOADS;
 };
 
-// Twiddles of butterfly k of a stage with twiddle step 1 (N / (R * SPAN) = 1),
-// then the radix-R DFT.
-template <int S, int R, typename V>
-__device__ __forceinline__ void bfly_k(V (&u)[R], int k, const V* __restrict__ tw)
-{
-    if (k) {
-#pragma unroll
-        for (int t = 1; t < R; ++t) u[t] = cmul(u[t], twiddle<S>(tw, t * k));
-    }
-    dftR<S, R>(u);
-}
-
-template <typename T, int S1, int S2, class Op>
-__global__ void __launch_bounds__(1024, 1) k_plane_zreg(const cplx<T>* src, cplx<T>* dst, size_t fstride,
-                                                        const cplx<T>* __restrict__ twn, Op op)
-{
-    using V = cplx<T>;
-    constexpr int N = 128, P = ZREG_P, NE = N * N;
-    static_assert(S1 != 0 && S2 != 0, "both transforms");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V* tile = reinterpret_cast<V*>(smem_raw);
-    V* stw = tile + N * P;
-    // twiddles w^(t i) of the register-resident z stage laid out [t][i]
-    // (t < 8, i < 16): its 16 consecutive threads take 16 consecutive
-    // entries, where the plain table would serve them with bank conflicts
-    V* stz = stw + N;
-    // twiddles w^(t b) of the warp-owned radix-16 z stage laid out [t][b]
-    // (t < 16, b < 8): the 8 butterflies of a row read consecutive entries
-    V* stb = stz + 128;
-    const int tid = threadIdx.x;
-    const int x = blockIdx.x;
-    const int f = blockIdx.y;
-    const size_t base = (size_t)f * fstride + (size_t)x * NE;
-    for (int j = tid; j < N; j += 1024) stw[j] = twn[j];
-    if (tid < 128) stz[tid] = twn[(tid >> 4) * (tid & 15)];
-    else if (tid < 256) stb[tid - 128] = twn[((tid - 128) >> 3) * (tid & 7)];
-    if (tid == 0) op.prefetch(base, (unsigned)NE);   // L2 prefetch: cannot observe a stale value
-    pdl_wait();
-    op.preload();
-    const int zc = tid & 127;   // column of the y-stages
-    const int hi = tid >> 7;    // 0..7
-    // inverse y, stage 0 (radix 16, span 1): the coalesced load of column zc,
-    // rows hi + 8t, is the input set of butterfly hi
-    {
-        V u[16];
-#pragma unroll
-        for (int t = 0; t < 16; ++t) u[t] = src[base + tid + t * 1024];
-        __syncthreads();   // twiddles
-        dftR<S1, 16>(u);
-#pragma unroll
-        for (int t = 0; t < 16; ++t) tile[(16 * hi + t) * P + plane_swz(zc)] = u[t];
-        __syncthreads();
-    }
-    // inverse y, stage 1 (radix 8, span 16): butterflies hi and hi + 8 of column zc
-    {
-        V u[2][8];
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-#pragma unroll
-            for (int t = 0; t < 8; ++t) u[q][t] = tile[(hi + 8 * q + 16 * t) * P + plane_swz(zc)];
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            bfly_k<S1, 8>(u[q], hi + 8 * q, stw);
-#pragma unroll
-            for (int t = 0; t < 8; ++t) tile[(hi + 8 * q + 16 * t) * P + plane_swz(zc)] = u[q][t];
-        }
-        __syncthreads();
-    }
-    // The z stages run on rows owned by one warp (rows 4w .. 4w+3 of warp
-    // w), so they synchronise with __syncwarp only: the warps drift apart
-    // there, and one warp's global loads of the pointwise step overlap the
-    // transforms and shared-memory exchanges of the others.
-    // inverse z, stage 0 (radix 16, span 1): row 4w + lane / 8, butterfly lane % 8
-    {
-        const int y = 4 * (threadIdx.x >> 5) + ((threadIdx.x & 31) >> 3), b = threadIdx.x & 7;
-        V u[16];
-#pragma unroll
-        for (int t = 0; t < 16; ++t) u[t] = tile[y * P + plane_swz(b + 8 * t)];
-        __syncwarp();
-        dftR<S1, 16>(u);
-#pragma unroll
-        for (int t = 0; t < 16; ++t) tile[y * P + plane_swz(16 * b + t)] = u[t];
-        __syncwarp();
-    }
-    // inverse z, stage 1 (radix 8, span 16) -> op -> forward z, stage 0
-    // (radix 8, span 1): butterfly i = lane % 16 of rows 4w + (lane / 16) + 2q.
-    // The op's loads depend on neither transform: those of row y0 are issued
-    // before the block reduction of begin() and those of row y0 + 2 right after
-    // the op of row y0, so their latency overlaps the barriers and the
-    // transforms.  Each row is read, transformed, passed through the op and
-    // written back in turn; per value the operations and their order are
-    // those of the two-row form.
-    const int i = threadIdx.x & 15;
-    const int y0 = 4 * (threadIdx.x >> 5) + ((threadIdx.x >> 4) & 1);   // rows y0 and y0 + 2
-    typename Op::Pre pre0[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) pre0[t] = op.load(f, base + (size_t)y0 * N + i + 16 * t);
-    op.begin();
-    {
-        typename Op::Pre pre1[8];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const int y = y0 + 2 * q;
-            V u[8];
-#pragma unroll
-            for (int t = 0; t < 8; ++t) u[t] = tile[y * P + plane_swz(i + 16 * t)];
-            __syncwarp();   // the row's reads done before its positions are rewritten
-            if (i) {
-#pragma unroll
-                for (int t = 1; t < 8; ++t) {
-                    V w = stz[t * 16 + i];
-                    if (S1 > 0) w.y = -w.y;
-                    u[t] = cmul(u[t], w);
-                }
-            }
-            dftR<S1, 8>(u);
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                const int z = i + 16 * t;
-                u[t] = op.apply(f, x, y, z, base + (size_t)y * N + z, u[t], q == 0 ? pre0[t] : pre1[t]);
-            }
-            if (q == 0) {
-#pragma unroll
-                for (int t = 0; t < 8; ++t) pre1[t] = op.load(f, base + (size_t)(y0 + 2) * N + i + 16 * t);
-            }
-            if (q == 1) pdl_trigger();
-            dftR<S2, 8>(u);
-#pragma unroll
-            for (int t = 0; t < 8; ++t) tile[y * P + plane_swz(8 * i + t)] = u[t];
-        }
-        __syncwarp();
-    }
-    // forward z, stage 1 (radix 16, span 8): row 4w + lane / 8, butterfly lane % 8
-    {
-        const int y = 4 * (threadIdx.x >> 5) + ((threadIdx.x & 31) >> 3), b = threadIdx.x & 7;
-        V u[16];
-#pragma unroll
-        for (int t = 0; t < 16; ++t) u[t] = tile[y * P + plane_swz(b + 8 * t)];
-        __syncwarp();
-        if (b) {
-#pragma unroll
-            for (int t = 1; t < 16; ++t) u[t] = cmul(u[t], twiddle<S2>(stb, t * 8 + b));
-        }
-        dftR<S2, 16>(u);
-#pragma unroll
-        for (int t = 0; t < 16; ++t) tile[y * P + plane_swz(b + 8 * t)] = u[t];
-        __syncthreads();
-    }
-    // forward y, stage 0 (radix 16, span 1): column zc, butterfly hi
-    {
-        V u[16];
-#pragma unroll
-        for (int t = 0; t < 16; ++t) u[t] = tile[(hi + 8 * t) * P + plane_swz(zc)];
-        __syncthreads();
-        dftR<S2, 16>(u);
-#pragma unroll
-        for (int t = 0; t < 16; ++t) tile[(16 * hi + t) * P + plane_swz(zc)] = u[t];
-        __syncthreads();
-    }
-    // forward y, stage 1 (radix 8, span 16): butterflies hi and hi + 8 of
-    // column zc, stored straight to global memory (consecutive z per warp)
-    {
-        V u[2][8];
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-#pragma unroll
-            for (int t = 0; t < 8; ++t) u[q][t] = tile[(hi + 8 * q + 16 * t) * P + plane_swz(zc)];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            bfly_k<S2, 8>(u[q], hi + 8 * q, stw);
-#pragma unroll
-            for (int t = 0; t < 8; ++t) dst[base + (size_t)(hi + 8 * q + 16 * t) * N + zc] = u[q][t];
-        }
-    }
-    op.end(reinterpret_cast<double*>(tile), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
-}
+// op.preload() where the op declares it
+template <class Op>
+__device__ __forceinline__ auto op_preload_if(Op& op, int) -> decltype(op.preload(), void()) { op.preload(); }
+template <class Op>
+__device__ __forceinline__ void op_preload_if(Op&, long) {}
+template <class Op>
+__device__ __forceinline__ void op_preload(Op& op) { op_preload_if(op, 0); }
 
 }  // namespace ftsp

@@ -1,0 +1,832 @@
+// Segment and bond passes of the chain sweeps with the y transform split
+// between them.
+//
+// A segment step is an inverse 3-D transform, the segment factor, a forward
+// transform and the bond factor.  With m2 = Y1 * Y2 the y transform is done
+// half in each of two passes, so that both work on small tiles:
+//
+//   real-space pass (k_split_real): the Y1 rows y0 + Y2 j (j < Y1) of one x,
+//     all z.  DFT over k1 (Y1 values, in registers), z inverse, pointwise op,
+//     z forward, DFT over j.  The twiddles w_{m2}^{y0 k1} between the halves
+//     are applied here.
+//   k-space pass (k_split_k): the Y2 consecutive rows k1 Y2 + y0 (y0 < Y2) of
+//     W columns z, all x.  DFT over y0 (Y2 values, in registers), x forward,
+//     pointwise op at (kx, ky = k1 + Y1 k2, kz), x inverse, DFT over k2.
+//
+// Between the passes a field holds, at row y0 + Y2 k1, the half-transformed
+// value (y0, k1): each tile of either pass reads and writes the same rows, so
+// a pass may run in place.
+//
+// Each 1-D transform along z (x) is two register butterflies, m = A * B (inverse along z: radix A, then B; forward in
+// reversed order, B then A), so the op sits between two radix-B butterflies
+// of the same thread and a pass is five register phases with four
+// shared-memory exchanges, whatever the length:
+//     Y1 | A | B op B | A | Y1      (real space; Y2 | A | B op B | A | Y2)
+//
+// Why split: one yz plane per block (k_plane) leaves one block of few warps
+// per SM on planes of mixed radix and does not fit at all above 112^2 in
+// complex128, where the y transform became two more passes over memory.  The
+// tiles here are 8-40 KB, so several blocks share an SM and hide each
+// other's loads and barriers, and every grid takes two passes per segment.
+// Measured on one B200, whole calls before and after (the plane and line
+// passes of passes.cuh against these): chain of 50 segments at 128^3
+// complex128 3.56 -> 2.38 ms (72.7 -> 48.5 us per segment, floor 10.3 at the
+// measured copy rate); 40 segments at 90 x 125 x 100 complex128 5.33 -> 2.50
+// ms; step at 96^3 complex64, N = 32, 8.8 -> 3.7 ms; step at 64^3 complex64,
+// N = 50, 1.44 -> 1.17 ms.  Both passes are bound by issue slots and by the
+// latency of their five dependent phases, not by memory: at 128^3 complex64
+// the real-space pass issues 0.51 and the k-space pass 0.37 instructions per
+// cycle and scheduler over 12 us of active time.
+//
+// The radices come from a plan: RtPlan reads them from the geometry (a
+// uniform switch per phase; any extents that factor into two radices),
+// CubePlan has every size at compile time (the production cubes).
+#pragma once
+
+#include "passes.cuh"
+
+#include <algorithm>
+#include <vector>
+
+namespace ftsp {
+
+constexpr int SPLIT_NT = 512;   // largest block
+constexpr int SPLIT_RADICES[] = {1, 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 25};
+
+struct SplitGeom {
+    int m1, m2, m3;
+    int ok;                  // the extents factor (see split_setup)
+    int big;                 // with radices that need RtBigPlan
+    int Y1, Y2;
+    // real-space pass: m3 = zA * zB, G row groups (y0 .. y0 + G - 1) per block
+    int zA, zB, G, rows;     // rows = G * Y1
+    int zA1, zB1;            // padded radices of the two exchanges
+    int pn, pa, pb;          // row pitches: natural order, after radix A, after radix B
+    int rt, r_threads;       // tile values, threads
+    FastDiv fzA, fzB, fm3, fY1;
+    // k-space pass: m1 = xA * xB, W columns, C = Y2 * W values per x
+    int xA, xB, W, C, pc;
+    int kt, k_threads, nzb;
+    FastDiv fC, fW, fnzb;
+    // twiddle tables: [t * zA + i] = w^(i t) (t < zB), [t * zB + i] (t < zA),
+    // the same of x, and [y0 * Y1 + k1] = w_{m2}^(y0 k1)
+    const void *tza, *tzb, *txa, *txb, *ty;
+};
+
+// ---- factors and layouts (constexpr: compile-time plans evaluate them too) ----
+constexpr bool split_radix(int r)
+{
+    for (int k : SPLIT_RADICES)
+        if (k == r) return true;
+    return false;
+}
+// n = a * b, a >= b, as even as possible, a at most amax, b at most bmax
+constexpr bool split_pair(int n, int amax, int bmax, int& a, int& b)
+{
+    for (int x = 1; x <= amax; ++x)
+        if (n % x == 0 && x * x >= n && n / x <= bmax && split_radix(x) && split_radix(n / x)) {
+            a = x;
+            b = n / x;
+            return true;
+        }
+    return false;
+}
+__host__ __device__ constexpr int split_max(int a, int b) { return a > b ? a : b; }
+constexpr int split_round32(int t) { return t < 32 ? 32 : (t + 31) / 32 * 32; }
+// Extra shared-memory cycles of one access by 64 consecutive threads, thread
+// l at value (l / o) * p + (l % o) * q: banks of 8 (complex64) or 16 bytes, 16
+// or 8 threads served at a time.
+constexpr int bank_cost(int lanes, int banks, int o, int p, int q)
+{
+    int cost = 0;
+    for (int l0 = 0; l0 < lanes && l0 < 64; l0 += banks) {
+        int n[16] = {}, worst = 1;
+        for (int l = l0; l < lanes && l < l0 + banks; ++l) {
+            const int b = ((l / o) * p + (l % o) * q) % banks;
+            n[b] += 1;
+            worst = split_max(worst, n[b]);
+        }
+        cost += worst - 1;
+    }
+    return cost;
+}
+// Exchange of radix r in a row of n values: written r values apart by the
+// (row, i < n / r) threads, read by (row, i < r): padded radix r1, row pitch.
+constexpr void split_exchange(int n, int r, int rows, int banks, int& r1, int& pitch)
+{
+    const int o = n / r;
+    int best = 1 << 30;
+    for (int pad = r; pad <= r + 1; ++pad)
+        for (int p = o * pad; p < o * pad + banks; ++p) {
+            const int c = bank_cost(rows * o, banks, o, p, pad) + bank_cost(rows * r, banks, r, p, 1);
+            if (c < best) {
+                best = c;
+                r1 = pad;
+                pitch = p;
+            }
+        }
+}
+
+constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes)
+{
+    const int banks = 128 / value_bytes;
+    g.m1 = m1; g.m2 = m2; g.m3 = m3;
+    g.ok = 0;
+    g.big = 0;
+    // the butterfly pair around the op (radix B) holds the op's operands
+    // beside its values: 10 at most, except in RtBigPlan
+    if (!split_pair(m3, 16, 10, g.zA, g.zB) || !split_pair(m1, 16, 10, g.xA, g.xB) || !split_pair(m2, 16, 16, g.Y1, g.Y2)) {
+        g.big = 1;
+        if (!split_pair(m3, 25, 16, g.zA, g.zB) || !split_pair(m1, 25, 16, g.xA, g.xB) || !split_pair(m2, 25, 16, g.Y1, g.Y2))
+            return false;
+        if (g.Y1 > 16) {   // the long half of y in the pass whose tiles are narrower
+            const int t = g.Y1;
+            g.Y1 = g.Y2;
+            g.Y2 = t;
+        }
+    }
+    // real space: as many row groups per block as leave two blocks per SM
+    g.G = 1;
+    for (int G = 2; G <= g.Y2; ++G)
+        if (g.Y2 % G == 0 && m1 * (g.Y2 / G) >= 296 && G * g.Y1 * m3 <= 1024 && G * split_max(g.Y1 * g.zA, m3) <= 256) g.G = G;
+    g.rows = g.G * g.Y1;
+    g.r_threads = split_round32(split_max(g.rows * g.zA, g.G * m3));
+    int best = 1 << 30;
+    for (int p = m3; p < m3 + banks; ++p) {   // natural order: (row, i < B) at row p + i
+        const int c = bank_cost(g.rows * g.zB, banks, g.zB, p, 1);
+        if (c < best) {
+            best = c;
+            g.pn = p;
+        }
+    }
+    split_exchange(m3, g.zA, g.rows, banks, g.zA1, g.pa);
+    split_exchange(m3, g.zB, g.rows, banks, g.zB1, g.pb);
+    g.rt = g.rows * split_max(g.pn, split_max(g.pa, g.pb));
+    g.fzA = make_fastdiv(g.zA); g.fzB = make_fastdiv(g.zB); g.fm3 = make_fastdiv(m3); g.fY1 = make_fastdiv(g.Y1);
+    // k space: 32 bytes of every row (one memory sector)
+    g.W = split_max(1, 32 / value_bytes);
+    while (g.W > 1 && (g.W / 2 >= m3 || (long long)m1 * g.Y2 * g.W * value_bytes > 72 * 1024)) g.W /= 2;
+    g.C = g.Y2 * g.W;
+    g.k_threads = split_round32(split_max(g.C * g.xA, m1 * g.W));
+    if (g.k_threads > SPLIT_NT) g.k_threads = SPLIT_NT;
+    if (g.r_threads > 256) g.r_threads = 256;
+    // both buffers of both passes within the shared memory of a block
+    if ((2LL * g.rt + 2 * m3 + g.rows) * value_bytes > 225 * 1024 || (2LL * m1 * (g.C + banks) + 2 * m1) * value_bytes > 225 * 1024)
+        return false;
+    best = 1 << 30;
+    for (int p = g.C; p < g.C + banks; ++p) {
+        const int c = bank_cost(64, banks, g.W, p, 1) + bank_cost(64, banks, g.C, p, 1) +
+                      bank_cost(64, banks, g.C, g.xA * p, 1) + bank_cost(64, banks, g.C, g.xB * p, 1);
+        if (c < best) {
+            best = c;
+            g.pc = p;
+        }
+    }
+    g.kt = m1 * g.pc;
+    g.nzb = (m3 + g.W - 1) / g.W;
+    g.fC = make_fastdiv(g.C); g.fW = make_fastdiv(g.W); g.fnzb = make_fastdiv(g.nzb);
+    g.ok = 1;
+    return true;
+}
+
+// ---- plans ----
+// RtPlan takes everything from the geometry argument, gives a thread one
+// butterfly per phase and exchanges between two buffers (one barrier each).
+struct RtPlan {
+    static constexpr bool CT = false;
+    static constexpr bool INPLACE = false;
+    static constexpr SplitGeom G = SplitGeom{};
+    static constexpr int RNT = 256, KNT = SPLIT_NT;
+    static constexpr int AMAX = 16, BMAX = 10;
+    // blocks per SM asked of the compiler, real space and k space
+    template <typename T> static constexpr int rmin = sizeof(T) == 4 ? 3 : 2;
+};
+// The same for lengths that need radix 25 (125 = 25 x 5) or two large radices
+// (192 = 16 x 12): its own kernels, so that the others keep their registers.
+struct RtBigPlan : RtPlan {
+    static constexpr int AMAX = 25, BMAX = 16;
+    template <typename T> static constexpr int rmin = 1;
+};
+// A cube of N points a side at compile time.  One buffer: a phase reads,
+// synchronises and writes.  Where the radix-B (and Y2) butterflies are a
+// multiple of the others in number, a thread takes several of them.
+constexpr int split_nt(int base, int a, int b)   // threads: a phase of `base` butterflies and two more
+{
+    const int nt = split_round32(base);
+    return a % nt == 0 && b % nt == 0 ? nt : split_round32(split_max(base, split_max(a, b)));
+}
+constexpr SplitGeom split_cube(int n, int value_bytes)
+{
+    SplitGeom g{};
+    split_setup(g, n, n, n, value_bytes);
+    g.r_threads = split_nt(split_max(g.rows * g.zB, g.G * n), g.rows * g.zA, g.rows * g.zA);
+    g.k_threads = split_nt(g.C * g.xB, g.C * g.xA, n * g.W);
+    return g;
+}
+template <int N, typename T>
+struct CubePlan {
+    static constexpr bool CT = true;
+    static constexpr bool INPLACE = true;
+    static constexpr SplitGeom G = split_cube(N, 2 * (int)sizeof(T));
+    static constexpr int RNT = G.r_threads, KNT = G.k_threads;
+    static constexpr int AMAX = 16, BMAX = 10;
+    template <typename T2> static constexpr int rmin = 1;
+};
+
+// Values of the five twiddle tables, in the order tza, tzb, txa, txb, ty
+// (2 m3 + 2 m1 + m2 values); tw(n, j) gives exp(-2 pi i j / n).
+template <class V, class Tw>
+inline std::vector<V> split_tables(const SplitGeom& g, Tw tw)
+{
+    std::vector<V> t;
+    auto put = [&](int n, int inner, int outer) {
+        for (int o = 0; o < outer; ++o)
+            for (int i = 0; i < inner; ++i) t.push_back(tw(n, (o * i) % n));
+    };
+    put(g.m3, g.zA, g.zB);
+    put(g.m3, g.zB, g.zA);
+    put(g.m1, g.xA, g.xB);
+    put(g.m1, g.xB, g.xA);
+    put(g.m2, g.Y1, g.Y2);
+    return t;
+}
+template <class V>
+inline void split_point_tables(SplitGeom& g, const V* base)
+{
+    g.tza = base;
+    g.tzb = base + g.m3;
+    g.txa = base + 2 * g.m3;
+    g.txb = base + 2 * g.m3 + g.m1;
+    g.ty = base + 2 * g.m3 + 2 * g.m1;
+}
+template <class P, class V>
+inline size_t split_real_smem(const SplitGeom& g)
+{
+    return std::max(sizeof(V) * (size_t)((P::INPLACE ? 1 : 2) * g.rt + 2 * g.m3 + g.rows), (size_t)4096);
+}
+template <class P, class V>
+inline size_t split_k_smem(const SplitGeom& g)
+{
+    return std::max(sizeof(V) * (size_t)((P::INPLACE ? 1 : 2) * g.kt + 2 * g.m1), (size_t)4096);
+}
+
+// ---- device ----
+// Composite butterflies.  Coprime factors need no twiddles: with inputs
+// n = (Q n1 + P n2) mod PQ and outputs k = k1 mod P, k2 mod Q (the prime-factor
+// algorithm), the transform is P-point DFTs over n1 and Q-point ones over n2.
+template <int S, int P, int Q, typename V>
+__device__ __forceinline__ void dft_coprime(V* u)
+{
+    constexpr int N = P * Q;
+    V a[N];
+#pragma unroll
+    for (int n2 = 0; n2 < Q; ++n2) {
+        V b[P];
+#pragma unroll
+        for (int n1 = 0; n1 < P; ++n1) b[n1] = u[(Q * n1 + P * n2) % N];
+        dftR<S, P>(b);
+#pragma unroll
+        for (int k1 = 0; k1 < P; ++k1) a[k1 * Q + n2] = b[k1];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < P; ++k1) {
+        V b[Q];
+#pragma unroll
+        for (int n2 = 0; n2 < Q; ++n2) b[n2] = a[k1 * Q + n2];
+        dftR<S, Q>(b);
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            if (k % P == k1) u[k] = b[k % Q];
+    }
+}
+
+// 9 = 3 x 3 with the twiddles w9, w9^2, w9^4
+template <int S, typename V>
+__device__ __forceinline__ void dft9(V* u)
+{
+    using R = typename RealOf<V>::type;
+    const R c1 = R(0.76604444311897803520239265055541668), s1 = R(0.64278760968653932632264340990726344);   // 40 degrees
+    const R c2 = R(0.17364817766693034885171662676931480), s2 = R(0.98480775301220805936674302458952302);   // 80 degrees
+    const R c4 = R(-0.93969262078590838405410927732473147), s4 = R(0.34202014332566873304409961468225958);  // 160 degrees
+    auto rot = [](V z, R c, R sn) { return mkc<V>(z.x * c - S * z.y * sn, z.y * c + S * z.x * sn); };
+    V a[3][3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) a[j][k] = u[j + 3 * k];
+        dft3<S>(a[j]);
+    }
+    a[1][1] = rot(a[1][1], c1, s1);
+    a[1][2] = rot(a[1][2], c2, s2);
+    a[2][1] = rot(a[2][1], c2, s2);
+    a[2][2] = rot(a[2][2], c4, s4);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        V b[3] = {a[0][k], a[1][k], a[2][k]};
+        dft3<S>(b);
+        u[k] = b[0];
+        u[k + 3] = b[1];
+        u[k + 6] = b[2];
+    }
+}
+
+// 25 = 5 x 5 with the twiddles w25^(j k)
+template <int S, typename V>
+__device__ __forceinline__ void dft25(V* u)
+{
+    using R = typename RealOf<V>::type;
+    // cos and sin of 2 pi j / 25 for the products j = 1 .. 16
+    constexpr double c[17] = {1.0, 0.96858316112863108148, 0.87630668004386363938, 0.72896862742141157547, 0.53582679497899660946,
+                              0.30901699437494742410, 0.06279051952931337608, -0.18738131458572463066, -0.42577929156507266490,
+                              -0.63742398974868967902, -0.80901699437494742410, -0.92977648588825144064, -0.99211470131447776388,
+                              -0.99211470131447776388, -0.92977648588825144064, -0.80901699437494742410, -0.63742398974868967902};
+    constexpr double sn[17] = {0.0, 0.24868988716485478824, 0.48175367410171529046, 0.68454710592868869210, 0.84432792550201508508,
+                               0.95105651629515357212, 0.99802672842827155733, 0.98228725072868865924, 0.90482705246601951990,
+                               0.77051324277578920853, 0.58778525229247312917, 0.36812455268467797320, 0.12533323356430427018,
+                               -0.12533323356430427018, -0.36812455268467797320, -0.58778525229247312917, -0.77051324277578920853};
+    V a[5][5];
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) a[j][k] = u[j + 5 * k];
+        dft5<S>(a[j]);
+#pragma unroll
+        for (int k = 1; k < 5; ++k)
+            if (j > 0) {
+                const R cc = R(c[j * k]), ss = R(sn[j * k]);
+                const V z = a[j][k];
+                a[j][k] = mkc<V>(z.x * cc - S * z.y * ss, z.y * cc + S * z.x * ss);
+            }
+    }
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        V b[5] = {a[0][k], a[1][k], a[2][k], a[3][k], a[4][k]};
+        dft5<S>(b);
+#pragma unroll
+        for (int t = 0; t < 5; ++t) u[k + 5 * t] = b[t];
+    }
+}
+
+template <int S, int R, typename V>
+__device__ __forceinline__ void dft_any(V* u)
+{
+    if constexpr (R == 6) dft_coprime<S, 2, 3>(u);
+    else if constexpr (R == 9) dft9<S>(u);
+    else if constexpr (R == 10) dft_coprime<S, 2, 5>(u);
+    else if constexpr (R == 12) dft_coprime<S, 4, 3>(u);
+    else if constexpr (R == 15) dft_coprime<S, 3, 5>(u);
+    else if constexpr (R == 25) dft25<S>(u);
+    else dftR<S, R>(u);
+}
+
+template <int R>
+struct RadixTag {
+    static constexpr int value = R;
+};
+// f(RadixTag<r>) for the radix of a phase: CTR at compile time, r (uniform
+// over the grid, at most MAX) at run time
+template <bool CT, int CTR, int MAX, class F>
+__device__ __forceinline__ void by_radix(int r, F&& f)
+{
+    if constexpr (CT) {
+        f(RadixTag<CTR>{});
+    } else {
+        switch (r) {
+        case 1: f(RadixTag<1>{}); break;
+        case 2: f(RadixTag<2>{}); break;
+        case 3: f(RadixTag<3>{}); break;
+        case 4: f(RadixTag<4>{}); break;
+        case 5: f(RadixTag<5>{}); break;
+        case 6: f(RadixTag<6>{}); break;
+        case 8: f(RadixTag<8>{}); break;
+        case 9: f(RadixTag<9>{}); break;
+        case 10: f(RadixTag<10>{}); break;
+        default:
+            if constexpr (MAX > 10) {
+                if (r == 12) f(RadixTag<12>{});
+                else if (r == 15) f(RadixTag<15>{});
+                else if (r == 16) f(RadixTag<16>{});
+            }
+            if constexpr (MAX > 16) {
+                if (r == 25) f(RadixTag<25>{});
+            }
+            break;
+        }
+    }
+}
+
+template <int S, int R, typename V>
+__device__ __forceinline__ void twiddle_table(V* u, const V* tab, int stride)
+{
+#pragma unroll
+    for (int t = 1; t < R; ++t) {
+        V w = tab[t * stride];
+        if (S > 0) w.y = -w.y;
+        u[t] = cmul(u[t], w);
+    }
+}
+
+// One phase: `items` butterflies of radix R over the block, gather(idx, u) then
+// finish(idx, u), and a barrier at the end where SYNC.  At compile time (ITEMS,
+// NT threads) a thread gathers all of its butterflies first, with the in-place
+// barrier after them.
+template <class P, int R, int ITEMS, int NT, bool INPLACE, bool SYNC, typename V, class Ga, class Fi>
+__device__ __forceinline__ void split_phase(int items, Ga gather, Fi finish)
+{
+    if constexpr (P::CT) {
+        constexpr int NB = (ITEMS + NT - 1) / NT;
+        V u[NB][R];
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            const int idx = threadIdx.x + q * NT;
+            if (ITEMS % NT == 0 || idx < ITEMS) gather(idx, u[q]);
+        }
+        if (INPLACE) __syncthreads();
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            const int idx = threadIdx.x + q * NT;
+            if (ITEMS % NT == 0 || idx < ITEMS) finish(idx, u[q]);
+        }
+    } else {
+        static_assert(P::CT || !INPLACE, "the run-time plan exchanges between two buffers");
+#pragma unroll 1
+        for (int idx = threadIdx.x; idx < items; idx += blockDim.x) {
+            V u[R];
+            gather(idx, u);
+            finish(idx, u);
+        }
+    }
+    if (SYNC) __syncthreads();
+}
+
+// geometry member: a constant of the plan, or the kernel argument's
+#define FTSP_PL(m) (P::CT ? P::G.m : g.m)
+// quotient by a geometry member with its magic-number divisor
+#define FTSP_DIV(i, m, f) (P::CT ? (int)((unsigned)(i) / (unsigned)split_max(1, P::G.m)) : (int)fdiv(i, g.f))
+
+// registers a thread is given: complex64 ops with one operand per point fit
+// 72 (7 blocks of 128 threads: 128^3 runs in one wave of 1024 blocks); wider
+// ops and complex128 take up to 128
+template <typename T, class Op>
+constexpr int split_regs()
+{
+    return sizeof(T) == 4 ? (op_loads<Op>::value == 0 ? 64 : op_loads<Op>::value == 1 ? 72 : 96) : 128;
+}
+template <class P, typename T, class Op>
+constexpr int split_min_blocks(int nt)
+{
+    return P::CT ? split_max(1, 65536 / (nt * split_regs<T, Op>())) : nt <= 256 ? P::template rmin<T> : 1;
+}
+
+// Real-space pass: grid (m1 * Y2 / G, fields).
+template <typename T, class P, int S1, int S2, class Op>
+__global__ void __launch_bounds__(P::RNT, split_min_blocks<P, T, Op>(P::RNT))
+    k_split_real(SplitGeom g, const cplx<T>* src, cplx<T>* dst, size_t fstride, Op op)
+{
+    using V = cplx<T>;
+    constexpr int NT = P::RNT;
+    constexpr bool IP = P::INPLACE;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int m2 = FTSP_PL(m2), m3 = FTSP_PL(m3), Y1 = FTSP_PL(Y1), Y2 = FTSP_PL(Y2), zA = FTSP_PL(zA), zB = FTSP_PL(zB);
+    const int rows = FTSP_PL(rows), pn = FTSP_PL(pn), pa = FTSP_PL(pa), pb = FTSP_PL(pb), zA1 = FTSP_PL(zA1), zB1 = FTSP_PL(zB1);
+    const int gpb = FTSP_PL(G), rt = FTSP_PL(rt);
+    const int nthr = P::CT ? NT : (int)blockDim.x;
+    V* b0 = reinterpret_cast<V*>(smem_raw);
+    V* b1 = IP ? b0 : b0 + rt;
+    V* ta = b1 + rt;       // radix B stage of butterfly i < A
+    V* tb = ta + m3;       // radix A stage of butterfly i < B
+    V* ty = tb + m3;       // [group][k1]
+    const int tid = threadIdx.x;
+    const int nyb = Y2 / gpb;
+    const int f = blockIdx.y;
+    const int x = blockIdx.x / nyb;
+    const int y0 = (blockIdx.x - x * nyb) * gpb;
+    const size_t base = (size_t)f * fstride + (size_t)x * m2 * m3;
+    for (int j = tid; j < m3; j += nthr) {
+        ta[j] = reinterpret_cast<const V*>(g.tza)[j];
+        tb[j] = reinterpret_cast<const V*>(g.tzb)[j];
+    }
+    for (int j = tid; j < rows; j += nthr) ty[j] = reinterpret_cast<const V*>(g.ty)[y0 * Y1 + j];
+    pdl_wait();
+    // every block has started once all have come here: the next pass may take
+    // what is idle and run its prologue (it waits for this one before it
+    // touches a field)
+    pdl_trigger();
+    op_preload(op);
+    if constexpr (S1 != 0) {
+        __syncthreads();   // twiddles
+        by_radix<P::CT, P::G.Y1, P::AMAX>(Y1, [&](auto rc) {
+            constexpr int R = decltype(rc)::value;
+            split_phase<P, R, P::G.G * P::G.m3, NT, false, true, V>(gpb * m3,
+                [&](int idx, V (&u)[R]) {
+                    const int gr = FTSP_DIV(idx, m3, fm3), z = idx - gr * m3;
+                    const V* s = src + base + (size_t)(y0 + gr) * m3 + z;
+                    const size_t st = (size_t)Y2 * m3;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) u[t] = s[t * st];
+                },
+                [&](int idx, V (&u)[R]) {
+                    const int gr = FTSP_DIV(idx, m3, fm3), z = idx - gr * m3;
+                    if (y0 + gr) twiddle_table<S1, R>(u, ty + gr * R, 1);
+                    dft_any<S1, R>(u);
+                    V* d = b0 + gr * R * pn + z;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) d[t * pn] = u[t];
+                });
+        });
+        by_radix<P::CT, P::G.zA, P::AMAX>(zA, [&](auto rc) {
+            constexpr int R = decltype(rc)::value;
+            split_phase<P, R, P::G.rows * P::G.zB, NT, IP, false, V>(rows * zB,
+                [&](int idx, V (&u)[R]) {
+                    const int r = FTSP_DIV(idx, zB, fzB), i = idx - r * zB;
+                    const V* s = b0 + r * pn + i;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) u[t] = s[t * zB];
+                },
+                [&](int idx, V (&u)[R]) {
+                    const int r = FTSP_DIV(idx, zB, fzB), i = idx - r * zB;
+                    dft_any<S1, R>(u);
+                    V* d = b1 + r * pa + i * zA1;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) d[t] = u[t];
+                });
+        });
+    }
+    op.begin();
+    __syncthreads();
+    by_radix<P::CT, P::G.zB, P::BMAX>(zB, [&](auto rc) {
+        constexpr int R = decltype(rc)::value;
+        // one operand per point: a butterfly's loads are in flight across the
+        // gather; wider ops load a few points at a time
+        constexpr int CH = op_loads<Op>::value <= 1 ? R : (R < 4 ? R : sizeof(T) == 4 ? 4 : 2);
+        auto place = [&](int idx, int& r, int& i, int& y, size_t& off) {
+            r = FTSP_DIV(idx, zA, fzA);
+            i = idx - r * zA;
+            const int gr = FTSP_DIV(r, Y1, fY1), j = r - gr * Y1;
+            y = y0 + gr + Y2 * j;
+            off = base + (size_t)y * m3 + i;
+        };
+        auto gather = [&](int idx, V (&u)[R]) {
+            const int r = FTSP_DIV(idx, zA, fzA), i = idx - r * zA;
+#pragma unroll
+            for (int t = 0; t < R; ++t) u[t] = S1 != 0 ? b1[r * pa + i + t * zA1] : mkc<V>(T(0), T(0));
+        };
+        auto loads = [&](int idx, typename Op::Pre (&pre)[CH]) {
+            int r, i, y;
+            size_t off;
+            place(idx, r, i, y, off);
+#pragma unroll
+            for (int t = 0; t < CH; ++t) pre[t] = op.load(f, off + t * zA);
+        };
+        auto finish = [&](int idx, V (&u)[R], typename Op::Pre (&pre)[CH]) {
+            int r, i, y;
+            size_t off;
+            place(idx, r, i, y, off);
+            if constexpr (S1 != 0) {
+                twiddle_table<S1, R>(u, ta + i, zA);
+                dft_any<S1, R>(u);
+            }
+#pragma unroll
+            for (int t = 0; t < R; ++t) {
+                if constexpr (CH < R) {
+                    if (t % CH == 0) {
+#pragma unroll
+                        for (int k = 0; k < CH; ++k)
+                            if (t + k < R) pre[k] = op.load(f, off + (t + k) * zA);
+                    }
+                }
+                u[t] = op.apply(f, x, y, i + t * zA, off + t * zA, u[t], pre[t % CH]);
+            }
+        };
+        auto scatter = [&](int idx, V (&u)[R]) {
+            if constexpr (S2 != 0) {
+                const int r = FTSP_DIV(idx, zA, fzA), i = idx - r * zA;
+                dft_any<S2, R>(u);
+                V* d = b0 + r * pb + i * zB1;
+#pragma unroll
+                for (int t = 0; t < R; ++t) d[t] = u[t];
+            }
+        };
+        typename Op::Pre pre[CH];
+        if constexpr (P::CT) {
+            constexpr int ITEMS = P::G.rows * P::G.zA;
+            constexpr int NB = (ITEMS + NT - 1) / NT;
+            V u[NB][R];
+            auto valid = [&](int idx) { return ITEMS % NT == 0 || idx < ITEMS; };
+            if constexpr (CH == R) {
+                if (valid(tid)) loads(tid, pre);
+            }
+#pragma unroll
+            for (int q = 0; q < NB; ++q)
+                if (valid(tid + q * NT)) gather(tid + q * NT, u[q]);
+            if (IP && S1 != 0 && S2 != 0) __syncthreads();
+#pragma unroll
+            for (int q = 0; q < NB; ++q) {
+                const int idx = tid + q * NT;
+                if (valid(idx)) {
+                    finish(idx, u[q], pre);
+                    if constexpr (CH == R) {
+                        if (q + 1 < NB && valid(idx + NT)) loads(idx + NT, pre);
+                    }
+                    scatter(idx, u[q]);
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (int idx = tid; idx < rows * zA; idx += blockDim.x) {
+                V u[R];
+                if constexpr (CH == R) loads(idx, pre);
+                gather(idx, u);
+                finish(idx, u, pre);
+                scatter(idx, u);
+            }
+        }
+    });
+    if constexpr (S2 != 0) {
+        __syncthreads();
+        by_radix<P::CT, P::G.zA, P::AMAX>(zA, [&](auto rc) {
+            constexpr int R = decltype(rc)::value;
+            split_phase<P, R, P::G.rows * P::G.zB, NT, IP, true, V>(rows * zB,
+                [&](int idx, V (&u)[R]) {
+                    const int r = FTSP_DIV(idx, zB, fzB), i = idx - r * zB;
+                    const V* s = b0 + r * pb + i;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) u[t] = s[t * zB1];
+                },
+                [&](int idx, V (&u)[R]) {
+                    const int r = FTSP_DIV(idx, zB, fzB), i = idx - r * zB;
+                    twiddle_table<S2, R>(u, tb + i, zB);
+                    dft_any<S2, R>(u);
+                    V* d = b1 + r * pn + i;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) d[t * zB] = u[t];
+                });
+        });
+        by_radix<P::CT, P::G.Y1, P::AMAX>(Y1, [&](auto rc) {
+            constexpr int R = decltype(rc)::value;
+            split_phase<P, R, P::G.G * P::G.m3, NT, false, false, V>(gpb * m3,
+                [&](int idx, V (&u)[R]) {
+                    const int gr = FTSP_DIV(idx, m3, fm3), z = idx - gr * m3;
+                    const V* s = b1 + gr * R * pn + z;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) u[t] = s[t * pn];
+                },
+                [&](int idx, V (&u)[R]) {
+                    const int gr = FTSP_DIV(idx, m3, fm3), z = idx - gr * m3;
+                    dft_any<S2, R>(u);
+                    if (y0 + gr) twiddle_table<S2, R>(u, ty + gr * R, 1);
+                    V* d = dst + base + (size_t)(y0 + gr) * m3 + z;
+                    const size_t st = (size_t)Y2 * m3;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) d[t * st] = u[t];
+                });
+        });
+    }
+    op.end(reinterpret_cast<double*>(b0), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
+}
+
+// k-space pass: grid (Y1 * nzb, fields); the input of field f is field
+// op_src_field(op, f) of src.
+template <typename T, class P, int S1, int S2, class Op>
+__global__ void __launch_bounds__(P::KNT, split_min_blocks<P, T, Op>(P::KNT))
+    k_split_k(SplitGeom g, const cplx<T>* src, cplx<T>* dst, size_t fstride, Op op)
+{
+    using V = cplx<T>;
+    constexpr int NT = P::KNT;
+    constexpr bool IP = P::INPLACE;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int m1 = FTSP_PL(m1), m2 = FTSP_PL(m2), m3 = FTSP_PL(m3), Y1 = FTSP_PL(Y1), Y2 = FTSP_PL(Y2), xA = FTSP_PL(xA), xB = FTSP_PL(xB);
+    const int W = FTSP_PL(W), C = FTSP_PL(C), pc = FTSP_PL(pc), kt = FTSP_PL(kt), nzb = FTSP_PL(nzb);
+    const int nthr = P::CT ? NT : (int)blockDim.x;
+    V* b0 = reinterpret_cast<V*>(smem_raw);
+    V* b1 = IP ? b0 : b0 + kt;
+    V* ta = b1 + kt;
+    V* tb = ta + m1;
+    const int tid = threadIdx.x;
+    const int f = blockIdx.y;
+    const int k1 = FTSP_DIV(blockIdx.x, nzb, fnzb);
+    const int z0 = (blockIdx.x - k1 * nzb) * W;
+    const size_t plane = (size_t)m2 * m3;
+    const size_t inner = (size_t)k1 * Y2 * m3 + z0;
+    const V* sp = src + (size_t)op_src_field(op, f) * fstride + inner;
+    V* dp = dst + (size_t)f * fstride + inner;
+    const size_t fbase = (size_t)f * fstride;
+    // the last tile of a row may be partial
+    const bool whole = P::CT ? P::G.m3 % split_max(1, P::G.W) == 0 : false;
+    for (int j = tid; j < m1; j += nthr) {
+        ta[j] = reinterpret_cast<const V*>(g.txa)[j];
+        tb[j] = reinterpret_cast<const V*>(g.txb)[j];
+    }
+    pdl_wait();
+    pdl_trigger();   // as in the real-space pass
+    by_radix<P::CT, P::G.Y2, P::AMAX>(Y2, [&](auto rc) {
+        constexpr int R = decltype(rc)::value;
+        split_phase<P, R, P::G.m1 * P::G.W, NT, false, true, V>(m1 * W,
+            [&](int idx, V (&u)[R]) {
+                const int x = FTSP_DIV(idx, W, fW), w = idx - x * W;
+                const bool in = whole || z0 + w < m3;
+                const V* s = sp + (size_t)x * plane + w;
+#pragma unroll
+                for (int t = 0; t < R; ++t) u[t] = in ? s[(size_t)t * m3] : mkc<V>(T(0), T(0));
+            },
+            [&](int idx, V (&u)[R]) {
+                const int x = FTSP_DIV(idx, W, fW), w = idx - x * W;
+                dft_any<S1, R>(u);
+                V* d = b0 + x * pc + w;
+#pragma unroll
+                for (int t = 0; t < R; ++t) d[t * W] = u[t];
+            });
+    });
+    by_radix<P::CT, P::G.xA, P::AMAX>(xA, [&](auto rc) {
+        constexpr int R = decltype(rc)::value;
+        split_phase<P, R, P::G.C * P::G.xB, NT, IP, false, V>(C * xB,
+            [&](int idx, V (&u)[R]) {
+                const int i = FTSP_DIV(idx, C, fC), c = idx - i * C;
+                const V* s = b0 + i * pc + c;
+#pragma unroll
+                for (int t = 0; t < R; ++t) u[t] = s[t * xB * pc];
+            },
+            [&](int idx, V (&u)[R]) {
+                const int i = FTSP_DIV(idx, C, fC), c = idx - i * C;
+                dft_any<S1, R>(u);
+                V* d = b1 + i * xA * pc + c;
+#pragma unroll
+                for (int t = 0; t < R; ++t) d[t * pc] = u[t];
+            });
+    });
+    op.begin();
+    __syncthreads();
+    by_radix<P::CT, P::G.xB, P::BMAX>(xB, [&](auto rc) {
+        constexpr int R = decltype(rc)::value;
+        split_phase<P, R, P::G.C * P::G.xA, NT, IP, true, V>(C * xA,
+            [&](int idx, V (&u)[R]) {
+                const int i = FTSP_DIV(idx, C, fC), c = idx - i * C;
+                const V* s = b1 + i * pc + c;
+#pragma unroll
+                for (int t = 0; t < R; ++t) u[t] = s[t * xA * pc];
+            },
+            [&](int idx, V (&u)[R]) {
+                const int i = FTSP_DIV(idx, C, fC), c = idx - i * C;
+                const int k2 = FTSP_DIV(c, W, fW), w = c - k2 * W;
+                const int y = k1 + Y1 * k2;
+                const size_t off = fbase + (size_t)i * plane + (size_t)y * m3 + z0 + w;
+                twiddle_table<S1, R>(u, ta + i, xA);
+                dft_any<S1, R>(u);
+                if (whole || z0 + w < m3) {
+                    typename Op::Pre pre[R];
+#pragma unroll
+                    for (int t = 0; t < R; ++t) pre[t] = op.load(f, off + (size_t)t * xA * plane);
+#pragma unroll
+                    for (int t = 0; t < R; ++t)
+                        u[t] = op.apply(f, i + t * xA, y, z0 + w, off + (size_t)t * xA * plane, u[t], pre[t]);
+                }
+                dft_any<S2, R>(u);
+                V* d = b0 + i * xB * pc + c;
+#pragma unroll
+                for (int t = 0; t < R; ++t) d[t * pc] = u[t];
+            });
+    });
+    by_radix<P::CT, P::G.xA, P::AMAX>(xA, [&](auto rc) {
+        constexpr int R = decltype(rc)::value;
+        split_phase<P, R, P::G.C * P::G.xB, NT, IP, true, V>(C * xB,
+            [&](int idx, V (&u)[R]) {
+                const int i = FTSP_DIV(idx, C, fC), c = idx - i * C;
+                const V* s = b0 + i * pc + c;
+#pragma unroll
+                for (int t = 0; t < R; ++t) u[t] = s[t * xB * pc];
+            },
+            [&](int idx, V (&u)[R]) {
+                const int i = FTSP_DIV(idx, C, fC), c = idx - i * C;
+                twiddle_table<S2, R>(u, tb + i, xB);
+                dft_any<S2, R>(u);
+                V* d = b1 + i * pc + c;
+#pragma unroll
+                for (int t = 0; t < R; ++t) d[t * xB * pc] = u[t];
+            });
+    });
+    by_radix<P::CT, P::G.Y2, P::AMAX>(Y2, [&](auto rc) {
+        constexpr int R = decltype(rc)::value;
+        split_phase<P, R, P::G.m1 * P::G.W, NT, false, false, V>(m1 * W,
+            [&](int idx, V (&u)[R]) {
+                const int x = FTSP_DIV(idx, W, fW), w = idx - x * W;
+                const V* s = b1 + x * pc + w;
+#pragma unroll
+                for (int t = 0; t < R; ++t) u[t] = s[t * W];
+            },
+            [&](int idx, V (&u)[R]) {
+                const int x = FTSP_DIV(idx, W, fW), w = idx - x * W;
+                dft_any<S2, R>(u);
+                V* d = dp + (size_t)x * plane + w;
+                if (whole || z0 + w < m3) {
+#pragma unroll
+                    for (int t = 0; t < R; ++t) d[(size_t)t * m3] = u[t];
+                }
+            });
+    });
+    op.end(reinterpret_cast<double*>(b0), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
+}
+
+#undef FTSP_PL
+#undef FTSP_DIV
+
+}  // namespace ftsp

@@ -19,7 +19,8 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 LIB = os.path.join(HERE, "libftsp.so")
 
-SOURCES = ["engine_f32.cu", "engine_f64.cu", "abi.cu"]
+SOURCES = ["engine_f32.cu", "engine_f64.cu", "split_real_f32.cu", "split_real_f64.cu", "split_k_f32.cu", "split_k_f64.cu",
+           "abi.cu"]
 HOST_SOURCES = ["host_model.cpp", "host_io.cpp", "host_run.cpp"]
 HEADERS = ["fft_core.cuh", "passes.cuh", "chain_pairs.cuh", "split_passes.cuh", "learned.cuh", "engine.cuh", "host_model.h", "host_io.h"]
 MAIN = os.path.join(HERE, "ftsp_main")

@@ -626,7 +626,7 @@ unsigned char* g_noalloc_base[NA_MAX_DEVICES] = {};
 struct NoallocTables {
     ftsp::FftPlan1 plans[3];                 // x, y, z
     double2 tw[3][NOALLOC_MAX_EXTENT];       // exp(-2 pi i j / m_d)
-    double2 split[5 * NOALLOC_MAX_EXTENT];   // twiddle tables of the split-y passes
+    double2 split[6 * NOALLOC_MAX_EXTENT];   // twiddle tables of the split-y passes
     double phi[3 * NOALLOC_MAX_EXTENT];      // separable exp(-b^2 k_d^2 / 6)
     double qsum[2];                          // sum of q_N (combine output)
 };
@@ -741,7 +741,7 @@ extern "C" int ftsp_propagate_chain_noalloc(int m1, int m2, int m3, double L1, d
         const size_t y_smem = std::max(sizeof(double2) * ((size_t)m2 * W + m2), (size_t)4096);
         const size_t z_smem = std::max(sizeof(double2) * ((size_t)B * (m3 + 1) + m3), (size_t)4096);
         if (x_threads > 256 || y_threads > 256 || z_threads > 256) throw std::runtime_error("ftsp_propagate_chain_noalloc: mesh too large for the line passes");
-        const int parts = sg.ok ? m1 * (sg.Y2 / sg.G) : plane_ok ? m1 : m1 * m2 / B;
+        const int parts = sg.ok ? split_real_blocks(sg) : plane_ok ? m1 : m1 * m2 / B;
         if ((size_t)parts > NA_PARTIALS_N) throw std::runtime_error("ftsp_propagate_chain_noalloc: too many reduction partials");
         const double2* tw1 = dtab->tw[0];
         const double2* tw2 = dtab->tw[1];
@@ -749,28 +749,12 @@ extern "C" int ftsp_propagate_chain_noalloc(int m1, int m2, int m3, double L1, d
         auto smem_attr = [&](auto kernel, size_t bytes) {
             if (bytes > 48 * 1024) FTSP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
         };
-        // dependent launch: the kernel's prologue overlaps the one before it
-        auto launch = [&](auto kernel, int grid, int threads, size_t smem, const double2* src, double2* dst, const auto& op) {
-            smem_attr(kernel, smem);
-            cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3(grid);
-            cfg.blockDim = dim3(threads);
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = stream;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            FTSP_CUDA(cudaLaunchKernelEx(&cfg, kernel, sg, src, dst, V, op));
-        };
         // real-space pass of one segment (split-y pass, plane, or y / z-line / y)
         auto seg = [&](auto s1c, auto s2c, const double2* src, double2* dst, const auto& op) {
             constexpr int S1 = decltype(s1c)::value, S2 = decltype(s2c)::value;
             using Op = std::decay_t<decltype(op)>;
             if (sg.ok) {
-                if (sg.big) launch(k_split_real<double, RtBigPlan, S1, S2, Op>, parts, sg.r_threads, split_real_smem<RtBigPlan, double2>(sg), src, dst, op);
-                else launch(k_split_real<double, RtPlan, S1, S2, Op>, parts, sg.r_threads, split_real_smem<RtPlan, double2>(sg), src, dst, op);
+                FTSP_CUDA((split_real_launch<double, S1, S2, Op>(sg, src, dst, V, 1, op, stream)));
                 return;
             }
             if (plane_ok) {
@@ -801,8 +785,7 @@ extern "C" int ftsp_propagate_chain_noalloc(int m1, int m2, int m3, double L1, d
         auto bond = [&] {
             using OB = OpBond<double, true, false>;
             if (sg.ok) {
-                if (sg.big) launch(k_split_k<double, RtBigPlan, -1, +1, OB>, sg.Y1 * sg.nzb, sg.k_threads, split_k_smem<RtBigPlan, double2>(sg), Gb, Gb, ob);
-                else launch(k_split_k<double, RtPlan, -1, +1, OB>, sg.Y1 * sg.nzb, sg.k_threads, split_k_smem<RtPlan, double2>(sg), Gb, Gb, ob);
+                FTSP_CUDA((split_k_launch<double, -1, +1, OB>(sg, Gb, Gb, V, 1, ob, stream)));
                 return;
             }
             auto kb = k_strided<double, EL, 0, -1, +1, OB>;

@@ -452,6 +452,7 @@ template <typename T>
 struct OpLoadN {
     const cplx<T>* s[16];
     size_t fs;
+    static constexpr int LOADS = 1;
     struct Pre {
         cplx<T> v;
     };
@@ -486,6 +487,7 @@ struct OpPrecond {
     T invV;
     int dc0 = -1;            // field whose k = 0 value is set to zero (psi: its mean removal), -1: none
     static constexpr int FUSED_MIN_BLOCKS = 8;
+    static constexpr int LOADS = 0;
     struct Pre {};
     __device__ __forceinline__ void begin() {}
     __device__ __forceinline__ Pre load(int, size_t) const { return Pre{}; }
@@ -550,6 +552,7 @@ struct OpLoadDensity {
     const V* rho;            // monomer density, charge density, ion charge
     size_t Vn;
     double zf;               // 0: no folded charge
+    static constexpr int LOADS = 1;
     struct Pre {
         V v;
     };
@@ -686,6 +689,7 @@ struct OpUpdate {
     bool elec;
     double* npart;           // per-CTA non-finite counts (null: not counted)
     double bad;
+    static constexpr int LOADS = 1;
     struct Pre {
         V b;
     };
@@ -719,6 +723,7 @@ struct OpUpdate {
 template <typename T>
 struct OpStore {
     cplx<T>* out;
+    static constexpr int LOADS = 0;
     struct Pre {};
     __device__ __forceinline__ void begin() {}
     __device__ __forceinline__ Pre load(int, size_t) const { return Pre{}; }
@@ -935,6 +940,7 @@ struct Engine : EngineBase {
     Buf<float> pmax;     // per-CTA propagator maxima, two slots (ping-pong by segment parity)
     SplitGeom sg{};      // split-y passes of the chain sweeps (split_passes.cuh)
     Buf<V> split_tw;     // their twiddle tables
+    Buf<V> fscr;         // half-transformed fields between the two passes of fft3
     bool use_split = false;
     Buf<float> smax;     // their propagator maxima: per species, forward [N], backward [N]; zeroed by eval
     std::vector<size_t> smax0;   // first slot of each species
@@ -1000,7 +1006,7 @@ struct Engine : EngineBase {
         plans.release();
         kx.release(); ky.release(); kz.release(); phi.release(); gam.release(); gion.release(); eta.release();
         part.release(); spart.release(); stage.release(); expo.release(); pmax.release();
-        split_tw.release(); smax.release();
+        split_tw.release(); smax.release(); fscr.release();
         pair_ix.release(); pair_wt.release(); pair_run.release();
         si_G.release(); si_inc.release(); ck.release();
         avg.acc.release();
@@ -1091,7 +1097,7 @@ struct Engine : EngineBase {
         psi.alloc(Vn); psi_bar.alloc(Vn); dpsi.alloc(Vn); dpsi_bar.alloc(Vn);
         // partials of the fused semi-implicit update (allocated here: a step
         // may run under stream capture, where nothing can be allocated)
-        if (c.scheme == FTSP_SCHEME_SI) upart.alloc(2 * (size_t)c.m1 * (nm + 1));
+        if (c.scheme == FTSP_SCHEME_SI) upart.alloc(2 * (size_t)(use_split ? c.m1 * sg.Y2 : c.m1) * (nm + 1));   // most blocks of any tiling
         eta.alloc((size_t)(nm + 1) * Vn);
         kA.alloc((size_t)2 * (nm + 1) * Vn);   // upper half: scratch of the fused evaluation's first pass
         kB.alloc((size_t)(M + 1 + J) * Vn);
@@ -1113,7 +1119,10 @@ struct Engine : EngineBase {
             slots += 2 * (size_t)s.N;
         }
         smax.alloc(std::max<size_t>(1, slots));
-        split_tw.alloc((size_t)2 * c.m1 + c.m2 + 2 * c.m3);
+        split_tw.alloc((size_t)3 * c.m1 + c.m2 + 2 * c.m3);
+        // as many fields as the widest batch of the evaluation that runs fft3;
+        // two for the learned preconditioner, the tuner and the fused evaluation
+        if (use_split) fscr.alloc(Vn * (size_t)std::max({M + 3, M + 1 + J, nm + 1}));
         spart.alloc((size_t)c.m2 * c.m3 * 12);
         if (c.restart_interval > 0) ck.alloc((size_t)(std::max(1, c.nm) + 1) * V_);
         FTSP_CUDA(cudaMalloc(&ds, sizeof(DevScal)));
@@ -1128,9 +1137,12 @@ struct Engine : EngineBase {
     }
 
     // ---- autotuner ----
-    // For every candidate geometry (FFT radix cap, strided tile width) the
-    // forward and inverse 3-D transforms of one field are timed with CUDA
-    // events (one warm-up, then the mean of three); the fastest is kept.
+    // The tiles of the split passes (row groups of the real-space pass,
+    // columns of the k-space pass) are tried on one bond pass and one mid
+    // segment pass; on a grid without split passes, the FFT radix cap and the
+    // tile width of the line passes on the forward and inverse 3-D transforms
+    // of one field.  Timed with CUDA events (one warm-up, then the mean of
+    // three); the fastest is kept.
     // Results are cached per (grid, precision, device) for the process, so a
     // set of replicas of the same grid tunes once.  Grids whose passes are
     // all compile-time kernels (32/64/128 cubes) have nothing to tune.
@@ -1142,7 +1154,7 @@ struct Engine : EngineBase {
         }
     };
     struct TuneResult {
-        int max_bits = 0, W = 0, candidates = 0;
+        int max_bits = 0, W = 0, G = 0, cube = 0, candidates = 0;
         double best_ms = 0.0, default_ms = 0.0;
         bool tuned = false, cached = false;
     };
@@ -1170,13 +1182,23 @@ struct Engine : EngineBase {
         cudaEvent_t a, b;
         FTSP_CUDA(cudaEventCreate(&a));
         FTSP_CUDA(cudaEventCreate(&b));
-        fft3<-1>(G.p, 1);
-        fft3<+1>(G.p, 1);
+        auto once = [&] {
+            if (use_split) {
+                OpBond<T, true, false> ob{};
+                set_bond(ob, 0);
+                bond_pass<-1, +1, true, false>(G.p, H.p, ob);
+                OpProp<T, FWD_MID> op{};
+                op.E = E.p;
+                op.qstore = qF.p;
+                seg_pass<+1, -1, FWD_MID>(H.p, G.p, op);
+            } else {
+                fft3<-1>(G.p, 1);
+                fft3<+1>(G.p, 1);
+            }
+        };
+        once();
         FTSP_CUDA(cudaEventRecord(a, stream));
-        for (int r = 0; r < reps; ++r) {
-            fft3<-1>(G.p, 1);
-            fft3<+1>(G.p, 1);
-        }
+        for (int r = 0; r < reps; ++r) once();
         FTSP_CUDA(cudaEventRecord(b, stream));
         FTSP_CUDA(cudaEventSynchronize(b));
         float ms = 0.0f;
@@ -1184,6 +1206,18 @@ struct Engine : EngineBase {
         cudaEventDestroy(a);
         cudaEventDestroy(b);
         return (double)ms / reps;
+    }
+
+    // other tiles for the split passes (cube: side of a compile-time plan, which
+    // brings its own tiles); false: they do not fit
+    bool retile(int groups, int W, int cube)
+    {
+        SplitGeom g = sg;
+        if (!split_tiles(g, (int)sizeof(V), groups, W)) return false;
+        g.cube = cube;
+        sg = g;
+        geo_W = W;
+        return true;
     }
 
     void autotune()
@@ -1194,7 +1228,8 @@ struct Engine : EngineBase {
         if (it != tune_cache().end()) {
             tune = it->second;
             tune.cached = true;
-            setup_geometry(tune.max_bits, tune.W);
+            if (use_split) retile(tune.G, tune.W, tune.cube);
+            else setup_geometry(tune.max_bits, tune.W);
             return;
         }
         TuneResult r{};
@@ -1206,6 +1241,28 @@ struct Engine : EngineBase {
             return;
         }
         FTSP_CUDA(cudaMemsetAsync(G.p, 0, sizeof(V) * V_, stream));
+        if (use_split) {
+            FTSP_CUDA(cudaMemsetAsync(E.p, 0, sizeof(V) * V_, stream));
+            r.max_bits = geo_max_bits;
+            r.W = sg.W; r.G = sg.G; r.cube = sg.cube;
+            r.best_ms = r.default_ms = time_fft(3);
+            const int G0 = sg.G;
+            for (int g : {G0, G0 > 1 ? 1 : 2})
+                for (int bytes : {32, 64, 128}) {
+                    if (sg.Y2 % g || !retile(g, std::max(1, bytes / (int)sizeof(V)), 0)) continue;
+                    const double t = time_fft(3);
+                    ++r.candidates;
+                    if (t < r.best_ms) {
+                        r.best_ms = t;
+                        r.W = sg.W; r.G = g; r.cube = 0;
+                    }
+                }
+            retile(r.G, r.W, r.cube);
+            r.tuned = true;
+            tune_cache()[key] = r;
+            tune = r;
+            return;
+        }
         std::vector<int> bits = F32 ? std::vector<int>{2, 3, 4} : std::vector<int>{2, 3};
         std::vector<int> Ws;
         for (int w = w_max(); w >= 1 && Ws.size() < 3; --w)
@@ -1423,13 +1480,13 @@ struct Engine : EngineBase {
     {
         const size_t Vn = V_;
         const int nf = c.nm + 1;
-        if (plane_ok) {
+        if (si_fused()) {
             // yz forward; x forward, P(k) / V, x inverse in one pencil pass; yz inverse
             cudaEvent_t ev = prof_begin();
             OpLoadN<T> self{};
             for (int f = 0; f < nf; ++f) self.s[f] = si_inc.p + (size_t)f * Vn;
             self.fs = Vn;
-            plane<0, -1>(nullptr, si_inc.p, nf, self);
+            yz_forward(si_inc.p, nf, self);
             OpPrecond<T> op{};
             op.GA = si_G.p;
             op.GL = lr.on_use ? lr.GL.p : nullptr;
@@ -1438,8 +1495,8 @@ struct Engine : EngineBase {
             for (int a = 0; a < c.nm; ++a) op.st.s[a] = c.dt * c.lambda[a];
             op.st.s[c.nm] = c.dt * c.lpsi;
             op.invV = (T)(1.0 / (double)Vn);
-            strided<0, -1, +1>(si_inc.p, si_inc.p, nf, op);
-            plane<+1, 0>(si_inc.p, nullptr, nf, OpStore<T>{si_inc.p});
+            x_factor(si_inc.p, si_inc.p, nf, op);
+            yz_inverse(si_inc.p, nf, OpStore<T>{si_inc.p});
             // three passes reading and writing every field, plus the G table
             prof_end(ev, "field_fft", (double)nf * (6.0 * sizeof(V) + sizeof(T)) * (double)Vn);
             return;
@@ -1480,7 +1537,8 @@ struct Engine : EngineBase {
     {
         const size_t Vn = V_;
         const int nm = c.nm, nf = nm + 1;
-        const size_t nparts = (size_t)c.m1 * nf;
+        const int fparts = yz_blocks();
+        const size_t nparts = (size_t)fparts * nf;
         cudaEvent_t ev = prof_begin();
         if (corr) {
             OpIncrement<T, true> op{};
@@ -1488,14 +1546,14 @@ struct Engine : EngineBase {
             for (int a = 0; a < nm; ++a) op.cs.s[a] = -0.5 * c.dt * c.lambda[a];
             op.cs.s[nm] = -0.5 * c.dt * c.lpsi;
             op.invV = 1.0 / (double)Vn; op.Vn = Vn; op.nm = nm; op.elec = c.elec; op.dpart = upart.p;
-            plane<0, -1>(nullptr, si_inc.p, nf, op);
+            yz_forward(si_inc.p, nf, op);
         } else {
             OpIncrement<T, false> op{};
             op.u0 = drift.p; op.e = eta.p; op.dp = dpsi.p; op.d = ds;
             for (int a = 0; a < nm; ++a) op.cs.s[a] = -c.dt * c.lambda[a];
             op.cs.s[nm] = -c.dt * c.lpsi;
             op.invV = 1.0 / (double)Vn; op.Vn = Vn; op.nm = nm; op.elec = c.elec;
-            plane<0, -1>(nullptr, si_inc.p, nf, op);
+            yz_forward(si_inc.p, nf, op);
         }
         OpPrecond<T> pr{};
         pr.GA = si_G.p;
@@ -1506,7 +1564,7 @@ struct Engine : EngineBase {
         pr.st.s[nm] = c.dt * c.lpsi;
         pr.invV = (T)(1.0 / (double)Vn);
         pr.dc0 = c.elec ? nm : -1;
-        strided<0, -1, +1>(si_inc.p, si_inc.p, nf, pr);
+        x_factor(si_inc.p, si_inc.p, nf, pr);
         OpUpdate<T> up{};
         up.w0 = corr ? omega.p : omega.p;
         up.p0 = psi.p;
@@ -1514,7 +1572,7 @@ struct Engine : EngineBase {
         up.p1 = corr ? psi.p : psi_bar.p;
         up.Vn = Vn; up.nm = nm; up.elec = c.elec;
         up.npart = corr ? upart.p + nparts : nullptr;
-        plane<+1, 0>(si_inc.p, nullptr, nf, up);
+        yz_inverse(si_inc.p, nf, up);
         // loads: drifts, noise (real), psi drift read and written; three
         // passes over the increments; the fields read and written
         const double units = corr ? (2.0 * nm + 0.5 * nf + 3.0 + nf) + 2.5 * nf + 3.0 * nf
@@ -1522,7 +1580,7 @@ struct Engine : EngineBase {
         prof_end(ev, "field_fft", units * sizeof(V) * (double)Vn);
         if (corr) {
             for (int f = 0; f < nf; ++f) {
-                k_combine<true><<<1, COMBINE_THREADS, 0, stream>>>(upart.p + (size_t)f * c.m1, c.m1, 1, ds->dmax + f);
+                k_combine<true><<<1, COMBINE_THREADS, 0, stream>>>(upart.p + (size_t)f * fparts, fparts, 1, ds->dmax + f);
                 ++launches;
             }
             k_combine<false><<<1, COMBINE_THREADS, 0, stream>>>(upart.p + nparts, (int)nparts, 1, ds->corr + 2);
@@ -2184,7 +2242,10 @@ struct Engine : EngineBase {
     }
     // the density evaluation with its k-space factors inside x-pencil passes:
     // one interaction mode, one monomer type, every ion smeared like the beads
-    bool eval_fused_ok() const { return plane_ok && c.nm == 1 && c.M == 1 && ion_common && x_fused(c.m1); }
+    bool eval_fused_ok() const
+    {
+        return c.nm == 1 && c.M == 1 && ion_common && (use_split || (plane_ok && x_fused(c.m1)));
+    }
 
     template <int DIM, int S1, int S2, class Op>
     void strided(const V* src, V* dst, int nf, const Op& op)
@@ -2255,6 +2316,13 @@ struct Engine : EngineBase {
         for (int f = 0; f < nf; ++f) self.s[f] = dst + (size_t)f * V_;
         self.fs = V_;
         cudaEvent_t ev = prof_begin();
+        if (use_split) {
+            // either sign runs the real-space pass first: natural order in and out
+            split_real<0, S>(nullptr, fscr.p, nf, in);
+            split_k<S, 0>(fscr.p, nullptr, nf, OpStore<T>{dst});
+            prof_end(ev, "field_fft", 4.0 * nf * sizeof(V) * (double)V_);
+            return;
+        }
         if (plane_ok) {
             plane<0, S>(nullptr, dst, nf, in);
         } else {
@@ -2267,57 +2335,44 @@ struct Engine : EngineBase {
     }
 
     // ---- split-y passes (split_passes.cuh) ----
-    template <class P, int S1, int S2, class Op>
-    void split_real_plan(const V* src, V* dst, int nf, const Op& op)
-    {
-        auto k = k_split_real<T, P, S1, S2, Op>;
-        const SplitGeom& p = P::CT ? P::G : sg;
-        const size_t smem = split_real_smem<P, V>(p);
-        set_smem(k, smem);
-        launch_pass(k, dim3(p.m1 * (p.Y2 / p.G), nf), p.r_threads, smem, sg, src, dst, (size_t)V_, op);
-        ++launches;
-    }
-    template <class P, int S1, int S2, class Op>
-    void split_k_plan(const V* src, V* dst, int nf, const Op& op)
-    {
-        auto k = k_split_k<T, P, S1, S2, Op>;
-        const SplitGeom& p = P::CT ? P::G : sg;
-        const size_t smem = split_k_smem<P, V>(p);
-        set_smem(k, smem);
-        launch_pass(k, dim3(p.Y1 * p.nzb, nf), p.k_threads, smem, sg, src, dst, (size_t)V_, op);
-        ++launches;
-    }
-    int cube() const { return c.m1 == c.m2 && c.m2 == c.m3 ? c.m1 : 0; }
     template <int S1, int S2, class Op>
     void split_real(const V* src, V* dst, int nf, const Op& op)
     {
-        // the passes at the ends of a sweep (one transform) run once: the
-        // run-time plan serves them
-        if constexpr (S1 != 0 && S2 != 0) switch (cube()) {
-            case 32: return split_real_plan<CubePlan<32, T>, S1, S2>(src, dst, nf, op);
-            case 48: return split_real_plan<CubePlan<48, T>, S1, S2>(src, dst, nf, op);
-            case 64: return split_real_plan<CubePlan<64, T>, S1, S2>(src, dst, nf, op);
-            case 96: return split_real_plan<CubePlan<96, T>, S1, S2>(src, dst, nf, op);
-            case 128: return split_real_plan<CubePlan<128, T>, S1, S2>(src, dst, nf, op);
-            default: break;
-        }
-        if (sg.big) return split_real_plan<RtBigPlan, S1, S2>(src, dst, nf, op);
-        split_real_plan<RtPlan, S1, S2>(src, dst, nf, op);
+        FTSP_CUDA((split_real_launch<T, S1, S2, Op>(sg, src, dst, (size_t)V_, nf, op, stream)));
+        ++launches;
     }
     template <int S1, int S2, class Op>
     void split_k(const V* src, V* dst, int nf, const Op& op)
     {
-        switch (cube()) {
-            case 32: return split_k_plan<CubePlan<32, T>, S1, S2>(src, dst, nf, op);
-            case 48: return split_k_plan<CubePlan<48, T>, S1, S2>(src, dst, nf, op);
-            case 64: return split_k_plan<CubePlan<64, T>, S1, S2>(src, dst, nf, op);
-            case 96: return split_k_plan<CubePlan<96, T>, S1, S2>(src, dst, nf, op);
-            case 128: return split_k_plan<CubePlan<128, T>, S1, S2>(src, dst, nf, op);
-            default: break;
-        }
-        if (sg.big) return split_k_plan<RtBigPlan, S1, S2>(src, dst, nf, op);
-        split_k_plan<RtPlan, S1, S2>(src, dst, nf, op);
+        FTSP_CUDA((split_k_launch<T, S1, S2, Op>(sg, src, dst, (size_t)V_, nf, op, stream)));
+        ++launches;
     }
+    // The three passes of a forward transform, a k-space factor and an inverse
+    // transform: field loads and yz forward, x forward - factor - x inverse,
+    // yz inverse and field stores (with the split passes, "yz" stands for the
+    // real-space pass and the fields between hold half-transformed rows).
+    template <class Op>
+    void yz_forward(V* dst, int nf, const Op& op)
+    {
+        if (use_split) split_real<0, -1>(nullptr, dst, nf, op);
+        else plane<0, -1>(nullptr, dst, nf, op);
+    }
+    template <class Op>
+    void x_factor(const V* src, V* dst, int nf, const Op& op)
+    {
+        if (use_split) split_k<-1, +1>(src, dst, nf, op);
+        else strided<0, -1, +1>(src, dst, nf, op);
+    }
+    template <class Op>
+    void yz_inverse(const V* src, int nf, const Op& op)
+    {
+        if (use_split) split_real<+1, 0>(src, nullptr, nf, op);
+        else plane<+1, 0>(src, nullptr, nf, op);
+    }
+    // the semi-implicit update in those passes
+    bool si_fused() const { return use_split || plane_ok; }
+    // blocks of one field of a yz pass
+    int yz_blocks() const { return use_split ? split_real_blocks(sg) : c.m1; }
 
     // Real-space pass of one segment: [inverse S1] op [forward S2] with the
     // propagator op.  Plane pass when the plane fits, else y / z-line / y.
@@ -2370,7 +2425,7 @@ struct Engine : EngineBase {
 
     int seg_pass_ctas() const
     {
-        if (use_split) return sg.m1 * (sg.Y2 / sg.G);
+        if (use_split) return split_real_blocks(sg);
         if (plane_ok) return c.m1;
         return c.m1 * c.m2 / gz.B;
     }
@@ -2763,7 +2818,7 @@ struct Engine : EngineBase {
             in.s[0] = om;
             in.s[1] = ps;
             in.fs = Vn;
-            plane<0, -1>(nullptr, kAx, 2, in);
+            yz_forward(kAx, 2, in);
             const double invV = 1.0 / (double)Vn;
             OpKScale<T> op{};
             op.kst = kA.p;
@@ -2779,8 +2834,8 @@ struct Engine : EngineBase {
             op.c[0] = make_double2(c.gamma[0].x * c.O[0] * invV, c.gamma[0].y * c.O[0] * invV);
             op.c[1] = make_double2(elec ? invV : 0.0, 0.0);
             op.c[2] = make_double2(elec ? invV / (4.0 * PI * c.lB) : 0.0, 0.0);
-            strided<0, -1, +1>(kAx, kB.p, 3, op);
-            plane<+1, 0>(kB.p, nullptr, 3, OpStore<T>{kB.p});
+            x_factor(kAx, kB.p, 3, op);
+            yz_inverse(kB.p, 3, OpStore<T>{kB.p});
             // plane: 2 in, 2 out; pencil: 3 in, 2 + 3 out; plane: 3 in, 3 out
             prof_end(ev, "field_fft", 18.0 * sizeof(V) * (double)Vn);
         }
@@ -2945,7 +3000,7 @@ struct Engine : EngineBase {
             ld.Vn = Vn;
             for (size_t k = 0; k < fold_type.size(); ++k)
                 if (fold_type[k] >= 0) ld.zf += fold_z[k];   // one type: at most one species folds
-            plane<0, -1>(nullptr, kC.p, 3, ld);
+            yz_forward(kC.p, 3, ld);
             const double invV = 1.0 / (double)Vn;
             OpKScale<T> op{};
             op.kst = dB.p;
@@ -2960,8 +3015,8 @@ struct Engine : EngineBase {
                 op.src[f] = f;
                 op.c[f] = make_double2(invV, 0.0);
             }
-            strided<0, -1, +1>(kC.p, kC.p, 3, op);
-            plane<+1, 0>(kC.p, nullptr, 3, OpStore<T>{kC.p});
+            x_factor(kC.p, kC.p, 3, op);
+            yz_inverse(kC.p, 3, OpStore<T>{kC.p});
             // plane: 3 in, 3 out; pencil: 3 in, 3 + 3 out; plane: 3 in, 3 out
             prof_end(ev, "field_fft", 21.0 * sizeof(V) * (double)Vn);
         }
@@ -3187,7 +3242,7 @@ struct Engine : EngineBase {
         T* e = eta.p;
         DevScal* d = ds;
         const double invV = 1.0 / (double)Vn;
-        if (c.scheme == FTSP_SCHEME_SI && plane_ok) {
+        if (c.scheme == FTSP_SCHEME_SI && si_fused()) {
             si_update_fused(false, lr.on_collect || lr.on_use);
             return;
         }
@@ -3290,7 +3345,7 @@ struct Engine : EngineBase {
         const T* e = eta.p;
         DevScal* d = ds;
         const double invV = 1.0 / (double)Vn;
-        if (c.scheme == FTSP_SCHEME_SI && plane_ok) {
+        if (c.scheme == FTSP_SCHEME_SI && si_fused()) {
             si_update_fused(true, false);
             return;
         }

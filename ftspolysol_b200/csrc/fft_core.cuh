@@ -45,11 +45,48 @@ __device__ __forceinline__ V mkc(typename RealOf<V>::type x, typename RealOf<V>:
 }
 template <typename V> __device__ __forceinline__ V cadd(V a, V b) { return mkc<V>(a.x + b.x, a.y + b.y); }
 template <typename V> __device__ __forceinline__ V csub(V a, V b) { return mkc<V>(a.x - b.x, a.y - b.y); }
+// The sums of the butterflies: vadd, vsub, vfma (a s + b, s real).
+template <typename V> __device__ __forceinline__ V vadd(V a, V b) { return cadd(a, b); }
+template <typename V> __device__ __forceinline__ V vsub(V a, V b) { return csub(a, b); }
+template <typename V> __device__ __forceinline__ V vfma(V a, typename RealOf<V>::type s, V b)
+{
+    return mkc<V>(fma(a.x, s, b.x), fma(a.y, s, b.y));
+}
+// complex64: both components in one packed instruction (same rounding per
+// component); the transforms are bound by issue slots
+template <> __device__ __forceinline__ float2 vadd(float2 a, float2 b)
+{
+    float2 r;
+    asm("{.reg .b64 p, q, s;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tadd.rn.f32x2 s, p, q;\n\tmov.b64 {%0, %1}, s;}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+template <> __device__ __forceinline__ float2 vsub(float2 a, float2 b)
+{
+    float2 r;
+    asm("{.reg .b64 p, q, s;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tsub.rn.f32x2 s, p, q;\n\tmov.b64 {%0, %1}, s;}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+template <> __device__ __forceinline__ float2 vfma(float2 a, float s, float2 b)
+{
+    float2 r;
+    asm("{.reg .b64 p, q, k, t;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tmov.b64 k, {%6, %6};\n\t"
+        "fma.rn.f32x2 t, p, k, q;\n\tmov.b64 {%0, %1}, t;}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(s));
+    return r;
+}
 template <typename V> __device__ __forceinline__ V cmul(V a, V b)
 {
     return mkc<V>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 template <typename V> __device__ __forceinline__ V cscale(V a, typename RealOf<V>::type s) { return mkc<V>(s * a.x, s * a.y); }
+// z (c + S i sn)
+template <int S, typename V>
+__device__ __forceinline__ V crot(V z, typename RealOf<V>::type c, typename RealOf<V>::type sn)
+{
+    return mkc<V>(z.x * c - S * z.y * sn, z.y * c + S * z.x * sn);
+}
 // multiply by S*i
 template <int S, typename V> __device__ __forceinline__ V mul_si(V z)
 {
@@ -60,31 +97,31 @@ template <int S, typename V> __device__ __forceinline__ V mul_si(V z)
 template <int S, typename V> __device__ __forceinline__ void dft2(V* u)
 {
     const V a = u[0], b = u[1];
-    u[0] = cadd(a, b);
-    u[1] = csub(a, b);
+    u[0] = vadd(a, b);
+    u[1] = vsub(a, b);
 }
 
 template <int S, typename V> __device__ __forceinline__ void dft3(V* u)
 {
     using R = typename RealOf<V>::type;
     const R h = R(0.86602540378443864676372317075293618);   // sin(2 pi / 3)
-    const V a = cadd(u[1], u[2]);
-    const V b = csub(u[1], u[2]);
+    const V a = vadd(u[1], u[2]);
+    const V b = vsub(u[1], u[2]);
     const V c = mkc<V>(u[0].x - R(0.5) * a.x, u[0].y - R(0.5) * a.y);
     const V sb = mul_si<S>(cscale(b, h));
-    u[0] = cadd(u[0], a);
-    u[1] = cadd(c, sb);
-    u[2] = csub(c, sb);
+    u[0] = vadd(u[0], a);
+    u[1] = vadd(c, sb);
+    u[2] = vsub(c, sb);
 }
 
 template <int S, typename V> __device__ __forceinline__ void dft4(V* u)
 {
-    const V a0 = cadd(u[0], u[2]), a1 = csub(u[0], u[2]);
-    const V b0 = cadd(u[1], u[3]), b1 = mul_si<S>(csub(u[1], u[3]));
-    u[0] = cadd(a0, b0);
-    u[2] = csub(a0, b0);
-    u[1] = cadd(a1, b1);
-    u[3] = csub(a1, b1);
+    const V a0 = vadd(u[0], u[2]), a1 = vsub(u[0], u[2]);
+    const V b0 = vadd(u[1], u[3]), b1 = mul_si<S>(vsub(u[1], u[3]));
+    u[0] = vadd(a0, b0);
+    u[2] = vsub(a0, b0);
+    u[1] = vadd(a1, b1);
+    u[3] = vsub(a1, b1);
 }
 
 template <int S, typename V> __device__ __forceinline__ void dft5(V* u)
@@ -94,17 +131,17 @@ template <int S, typename V> __device__ __forceinline__ void dft5(V* u)
     const R c2 = R(-0.80901699437494742410229341718281906); // cos(4 pi/5)
     const R s1 = R(0.95105651629515357211643933337938214);  // sin(2 pi/5)
     const R s2 = R(0.58778525229247312916870595463907277);  // sin(4 pi/5)
-    const V a1 = cadd(u[1], u[4]), b1 = csub(u[1], u[4]);
-    const V a2 = cadd(u[2], u[3]), b2 = csub(u[2], u[3]);
+    const V a1 = vadd(u[1], u[4]), b1 = vsub(u[1], u[4]);
+    const V a2 = vadd(u[2], u[3]), b2 = vsub(u[2], u[3]);
     const V r1 = mkc<V>(u[0].x + c1 * a1.x + c2 * a2.x, u[0].y + c1 * a1.y + c2 * a2.y);
     const V r2 = mkc<V>(u[0].x + c2 * a1.x + c1 * a2.x, u[0].y + c2 * a1.y + c1 * a2.y);
     const V i1 = mul_si<S>(mkc<V>(s1 * b1.x + s2 * b2.x, s1 * b1.y + s2 * b2.y));
     const V i2 = mul_si<S>(mkc<V>(s2 * b1.x - s1 * b2.x, s2 * b1.y - s1 * b2.y));
-    u[0] = cadd(u[0], cadd(a1, a2));
-    u[1] = cadd(r1, i1);
-    u[4] = csub(r1, i1);
-    u[2] = cadd(r2, i2);
-    u[3] = csub(r2, i2);
+    u[0] = vadd(u[0], vadd(a1, a2));
+    u[1] = vadd(r1, i1);
+    u[4] = vsub(r1, i1);
+    u[2] = vadd(r2, i2);
+    u[3] = vsub(r2, i2);
 }
 
 template <int S, typename V> __device__ __forceinline__ void dft8(V* u)
@@ -115,15 +152,17 @@ template <int S, typename V> __device__ __forceinline__ void dft8(V* u)
     V o[4] = {u[1], u[3], u[5], u[7]};
     dft4<S>(e);
     dft4<S>(o);
-    // o[t] *= exp(S*2*pi*i*t/8)
+    // o[t] *= exp(S*2*pi*i*t/8); the 1/sqrt2 of odd t goes into the sums
     const V o1 = o[1], o3 = o[3];
-    o[1] = mkc<V>(r * (o1.x - S * o1.y), r * (o1.y + S * o1.x));   // (1 + S i)/sqrt2
+    o[1] = mkc<V>(o1.x - S * o1.y, o1.y + S * o1.x);     // (1 + S i)
     o[2] = mul_si<S>(o[2]);
-    o[3] = mkc<V>(r * (-o3.x - S * o3.y), r * (-o3.y + S * o3.x)); // (-1 + S i)/sqrt2
+    o[3] = mkc<V>(-o3.x - S * o3.y, -o3.y + S * o3.x);   // (-1 + S i)
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-        u[t] = cadd(e[t], o[t]);
-        u[t + 4] = csub(e[t], o[t]);
+    for (int t = 0; t < 4; t += 2) {
+        u[t] = vadd(e[t], o[t]);
+        u[t + 4] = vsub(e[t], o[t]);
+        u[t + 1] = vfma(o[t + 1], r, e[t + 1]);
+        u[t + 5] = vfma(o[t + 1], -r, e[t + 1]);
     }
 }
 
@@ -145,7 +184,7 @@ template <int S, typename V> __device__ __forceinline__ void dft16(V* u)
         dft4<S>(a[j]);
     }
     // a[j][k] *= exp(S*2*pi*i*j*k/16) for j, k in 1..3
-    auto rot = [](V z, R c, R sn) { return mkc<V>(z.x * c - S * z.y * sn, z.y * c + S * z.x * sn); };
+    auto rot = [](V z, R c, R sn) { return crot<S>(z, c, sn); };
     a[1][1] = rot(a[1][1], c1, s1);
     a[1][2] = rot(a[1][2], r2, r2);
     a[1][3] = rot(a[1][3], s1, c1);

@@ -600,11 +600,20 @@ struct OpBond {
         if (!FWD && STRESS) p.F = Fread[g];
         return p;
     }
+    // For kernels that stage the x factors themselves (x_table, in shared
+    // memory): column() gives the factor of a thread's column, once, and
+    // apply_x() is apply() with the x factor and the column factor given.
+    __device__ __forceinline__ const T* x_table() const { return phix; }
+    __device__ __forceinline__ T column(int y, int z) const { return __ldg(phiy + y) * __ldg(phiz + z); }
     __device__ __forceinline__ V apply(int, int x, int y, int z, size_t g, V v, const Pre& pre)
     {
         // read-only loads: they do not alias the Fstore writes, so the y and z
         // factors (fixed for a thread's column) are loaded once
-        const T phi = __ldg(phix + x) * __ldg(phiy + y) * __ldg(phiz + z);
+        return apply_x(x, y, z, g, v, pre, __ldg(phix + x), column(y, z));
+    }
+    __device__ __forceinline__ V apply_x(int x, int y, int z, size_t g, V v, const Pre& pre, T px, T pyz)
+    {
+        const T phi = px * pyz;
         if (FWD) {
             if (Fstore) Fstore[g] = v;
         } else if (STRESS) {
@@ -1137,6 +1146,12 @@ template <class Op>
 struct op_loads<Op, std::void_t<decltype(Op::LOADS)>> {
     static constexpr int value = Op::LOADS;
 };
+
+// ops with x_table(), column() and apply_x()
+template <class Op, class = void>
+struct op_has_xtab : std::false_type {};
+template <class Op>
+struct op_has_xtab<Op, std::void_t<decltype(&Op::x_table)>> : std::true_type {};
 
 // op.preload() where the op declares it
 template <class Op>

@@ -1,0 +1,7 @@
+// k-space bond passes of the chain sweeps, complex64 (split_passes.cuh).
+#define FTSP_SPLIT_INSTANCES
+#include "split_passes.cuh"
+
+namespace ftsp {
+FTSP_SPLIT_K_ALL(template, float)
+}  // namespace ftsp

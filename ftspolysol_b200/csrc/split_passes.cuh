@@ -57,6 +57,7 @@ struct SplitGeom {
     int m1, m2, m3;
     int ok;                  // the extents factor (see split_setup)
     int big;                 // with radices that need RtBigPlan
+    int cube;                // side of the CubePlan to run, 0: a run-time plan
     int Y1, Y2;
     // real-space pass: m3 = zA * zB, G row groups (y0 .. y0 + G - 1) per block
     int zA, zB, G, rows;     // rows = G * Y1
@@ -71,6 +72,7 @@ struct SplitGeom {
     // twiddle tables: [t * zA + i] = w^(i t) (t < zB), [t * zB + i] (t < zA),
     // the same of x, and [y0 * Y1 + k1] = w_{m2}^(y0 k1)
     const void *tza, *tzb, *txa, *txb, *ty;
+    const void* tx;          // w_{m1}^j
 };
 
 // ---- factors and layouts (constexpr: compile-time plans evaluate them too) ----
@@ -127,9 +129,52 @@ constexpr void split_exchange(int n, int r, int rows, int banks, int& r1, int& p
         }
 }
 
-constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes)
+// Tiles of G row groups (real space) and W columns (k space): pitches, sizes,
+// threads.
+constexpr bool split_tiles(SplitGeom& g, int value_bytes, int G, int W)
 {
     const int banks = 128 / value_bytes;
+    const int m1 = g.m1, m3 = g.m3;
+    g.G = G;
+    g.rows = g.G * g.Y1;
+    g.r_threads = split_round32(split_max(g.rows * g.zA, g.G * m3));
+    if (g.r_threads > 256) g.r_threads = 256;
+    int best = 1 << 30;
+    for (int p = m3; p < m3 + banks; ++p) {   // natural order: (row, i < B) at row p + i
+        const int c = bank_cost(g.rows * g.zB, banks, g.zB, p, 1);
+        if (c < best) {
+            best = c;
+            g.pn = p;
+        }
+    }
+    split_exchange(m3, g.zA, g.rows, banks, g.zA1, g.pa);
+    split_exchange(m3, g.zB, g.rows, banks, g.zB1, g.pb);
+    g.rt = g.rows * split_max(g.pn, split_max(g.pa, g.pb));
+    g.fzA = make_fastdiv(g.zA); g.fzB = make_fastdiv(g.zB); g.fm3 = make_fastdiv(m3); g.fY1 = make_fastdiv(g.Y1);
+    g.W = W;
+    g.C = g.Y2 * g.W;
+    g.k_threads = split_round32(split_max(g.C * g.xA, m1 * g.W));
+    if (g.k_threads > SPLIT_NT) g.k_threads = SPLIT_NT;
+    // both buffers of both passes within the shared memory of a block
+    if ((2LL * g.rt + 2 * m3 + g.rows) * value_bytes > 225 * 1024 || (2LL * m1 * (g.C + banks) + 2 * m1) * value_bytes > 225 * 1024)
+        return false;
+    best = 1 << 30;
+    for (int p = g.C; p < g.C + banks; ++p) {
+        const int c = bank_cost(64, banks, g.W, p, 1) + bank_cost(64, banks, g.C, p, 1) +
+                      bank_cost(64, banks, g.C, g.xA * p, 1) + bank_cost(64, banks, g.C, g.xB * p, 1);
+        if (c < best) {
+            best = c;
+            g.pc = p;
+        }
+    }
+    g.kt = m1 * g.pc;
+    g.nzb = (m3 + g.W - 1) / g.W;
+    g.fC = make_fastdiv(g.C); g.fW = make_fastdiv(g.W); g.fnzb = make_fastdiv(g.nzb);
+    return true;
+}
+
+constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes)
+{
     g.m1 = m1; g.m2 = m2; g.m3 = m3;
     g.ok = 0;
     g.big = 0;
@@ -146,47 +191,15 @@ constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes
         }
     }
     // real space: as many row groups per block as leave two blocks per SM
-    g.G = 1;
-    for (int G = 2; G <= g.Y2; ++G)
-        if (g.Y2 % G == 0 && m1 * (g.Y2 / G) >= 296 && G * g.Y1 * m3 <= 1024 && G * split_max(g.Y1 * g.zA, m3) <= 256) g.G = G;
-    g.rows = g.G * g.Y1;
-    g.r_threads = split_round32(split_max(g.rows * g.zA, g.G * m3));
-    int best = 1 << 30;
-    for (int p = m3; p < m3 + banks; ++p) {   // natural order: (row, i < B) at row p + i
-        const int c = bank_cost(g.rows * g.zB, banks, g.zB, p, 1);
-        if (c < best) {
-            best = c;
-            g.pn = p;
-        }
-    }
-    split_exchange(m3, g.zA, g.rows, banks, g.zA1, g.pa);
-    split_exchange(m3, g.zB, g.rows, banks, g.zB1, g.pb);
-    g.rt = g.rows * split_max(g.pn, split_max(g.pa, g.pb));
-    g.fzA = make_fastdiv(g.zA); g.fzB = make_fastdiv(g.zB); g.fm3 = make_fastdiv(m3); g.fY1 = make_fastdiv(g.Y1);
+    int G = 1;
+    for (int t = 2; t <= g.Y2; ++t)
+        if (g.Y2 % t == 0 && m1 * (g.Y2 / t) >= 296 && t * g.Y1 * m3 <= 1024 && t * split_max(g.Y1 * g.zA, m3) <= 256) G = t;
     // k space: 32 bytes of every row (one memory sector)
-    g.W = split_max(1, 32 / value_bytes);
-    while (g.W > 1 && (g.W / 2 >= m3 || (long long)m1 * g.Y2 * g.W * value_bytes > 72 * 1024)) g.W /= 2;
-    g.C = g.Y2 * g.W;
-    g.k_threads = split_round32(split_max(g.C * g.xA, m1 * g.W));
-    if (g.k_threads > SPLIT_NT) g.k_threads = SPLIT_NT;
-    if (g.r_threads > 256) g.r_threads = 256;
-    // both buffers of both passes within the shared memory of a block
-    if ((2LL * g.rt + 2 * m3 + g.rows) * value_bytes > 225 * 1024 || (2LL * m1 * (g.C + banks) + 2 * m1) * value_bytes > 225 * 1024)
-        return false;
-    best = 1 << 30;
-    for (int p = g.C; p < g.C + banks; ++p) {
-        const int c = bank_cost(64, banks, g.W, p, 1) + bank_cost(64, banks, g.C, p, 1) +
-                      bank_cost(64, banks, g.C, g.xA * p, 1) + bank_cost(64, banks, g.C, g.xB * p, 1);
-        if (c < best) {
-            best = c;
-            g.pc = p;
-        }
-    }
-    g.kt = m1 * g.pc;
-    g.nzb = (m3 + g.W - 1) / g.W;
-    g.fC = make_fastdiv(g.C); g.fW = make_fastdiv(g.W); g.fnzb = make_fastdiv(g.nzb);
-    g.ok = 1;
-    return true;
+    int W = split_max(1, 32 / value_bytes);
+    while (W > 1 && (W / 2 >= m3 || (long long)m1 * g.Y2 * W * value_bytes > 72 * 1024)) W /= 2;
+    g.cube = m1 == m2 && m2 == m3 && (m1 == 32 || m1 == 48 || m1 == 64 || m1 == 96 || m1 == 128) ? m1 : 0;
+    g.ok = split_tiles(g, value_bytes, G, W) ? 1 : 0;
+    return g.ok != 0;
 }
 
 // ---- plans ----
@@ -233,8 +246,8 @@ struct CubePlan {
     template <typename T2> static constexpr int rmin = 1;
 };
 
-// Values of the five twiddle tables, in the order tza, tzb, txa, txb, ty
-// (2 m3 + 2 m1 + m2 values); tw(n, j) gives exp(-2 pi i j / n).
+// Values of the twiddle tables, in the order tza, tzb, txa, txb, ty, tx
+// (2 m3 + 3 m1 + m2 values); tw(n, j) gives exp(-2 pi i j / n).
 template <class V, class Tw>
 inline std::vector<V> split_tables(const SplitGeom& g, Tw tw)
 {
@@ -248,6 +261,8 @@ inline std::vector<V> split_tables(const SplitGeom& g, Tw tw)
     put(g.m1, g.xA, g.xB);
     put(g.m1, g.xB, g.xA);
     put(g.m2, g.Y1, g.Y2);
+    put(g.m1, g.m1, 2);
+    t.erase(t.end() - 2 * g.m1, t.end() - g.m1);   // the row of first powers
     return t;
 }
 template <class V>
@@ -258,6 +273,7 @@ inline void split_point_tables(SplitGeom& g, const V* base)
     g.txa = base + 2 * g.m3;
     g.txb = base + 2 * g.m3 + g.m1;
     g.ty = base + 2 * g.m3 + 2 * g.m1;
+    g.tx = base + 2 * g.m3 + 2 * g.m1 + g.m2;
 }
 template <class P, class V>
 inline size_t split_real_smem(const SplitGeom& g)
@@ -367,6 +383,47 @@ __device__ __forceinline__ void dft25(V* u)
     }
 }
 
+// cos(2 pi m / 32)
+__host__ __device__ constexpr double cos32(int m)
+{
+    constexpr double c[9] = {1.0, 0.98078528040323044913, 0.92387953251128675613, 0.83146961230254523708, 0.70710678118654752440,
+                             0.55557023301960222474, 0.38268343236508977173, 0.19509032201612826785, 0.0};
+    m &= 31;
+    if (m > 16) m = 32 - m;
+    return m <= 8 ? c[m] : -c[16 - m];
+}
+// 32 = 4 x 8: DFT8 over the stride-4 sub-sequences, twiddles w32^(j k), DFT4
+template <int S, typename V>
+__device__ __forceinline__ void dft32(V* u)
+{
+    using R = typename RealOf<V>::type;
+    V a[4][8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) a[j][k] = u[j + 4 * k];
+        dft8<S>(a[j]);
+#pragma unroll
+        for (int k = 1; k < 8; ++k) {
+            if (j == 0) continue;
+            if (j * k == 8) {
+                a[j][k] = mul_si<S>(a[j][k]);
+            } else {
+                const R c = R(cos32(j * k)), sn = R(cos32(j * k + 24));   // sin(t) = cos(t - 90 degrees)
+                const V z = a[j][k];
+                a[j][k] = mkc<V>(z.x * c - S * z.y * sn, z.y * c + S * z.x * sn);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        V b[4] = {a[0][k], a[1][k], a[2][k], a[3][k]};
+        dft4<S>(b);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) u[k + 8 * t] = b[t];
+    }
+}
+
 template <int S, int R, typename V>
 __device__ __forceinline__ void dft_any(V* u)
 {
@@ -376,6 +433,7 @@ __device__ __forceinline__ void dft_any(V* u)
     else if constexpr (R == 12) dft_coprime<S, 4, 3>(u);
     else if constexpr (R == 15) dft_coprime<S, 3, 5>(u);
     else if constexpr (R == 25) dft25<S>(u);
+    else if constexpr (R == 32) dft32<S>(u);
     else dftR<S, R>(u);
 }
 
@@ -686,7 +744,8 @@ __global__ void __launch_bounds__(P::RNT, split_min_blocks<P, T, Op>(P::RNT))
 }
 
 // k-space pass: grid (Y1 * nzb, fields); the input of field f is field
-// op_src_field(op, f) of src.
+// op_src_field(op, f) of src.  Without the second transform (S2 = 0) the op
+// stores, in natural order.
 template <typename T, class P, int S1, int S2, class Op>
 __global__ void __launch_bounds__(P::KNT, split_min_blocks<P, T, Op>(P::KNT))
     k_split_k(SplitGeom g, const cplx<T>* src, cplx<T>* dst, size_t fstride, Op op)
@@ -780,53 +839,301 @@ __global__ void __launch_bounds__(P::KNT, split_min_blocks<P, T, Op>(P::KNT))
                     for (int t = 0; t < R; ++t)
                         u[t] = op.apply(f, i + t * xA, y, z0 + w, off + (size_t)t * xA * plane, u[t], pre[t]);
                 }
-                dft_any<S2, R>(u);
-                V* d = b0 + i * xB * pc + c;
+                if constexpr (S2 != 0) {
+                    dft_any<S2, R>(u);
+                    V* d = b0 + i * xB * pc + c;
 #pragma unroll
-                for (int t = 0; t < R; ++t) d[t * pc] = u[t];
-            });
-    });
-    by_radix<P::CT, P::G.xA, P::AMAX>(xA, [&](auto rc) {
-        constexpr int R = decltype(rc)::value;
-        split_phase<P, R, P::G.C * P::G.xB, NT, IP, true, V>(C * xB,
-            [&](int idx, V (&u)[R]) {
-                const int i = FTSP_DIV(idx, C, fC), c = idx - i * C;
-                const V* s = b0 + i * pc + c;
-#pragma unroll
-                for (int t = 0; t < R; ++t) u[t] = s[t * xB * pc];
-            },
-            [&](int idx, V (&u)[R]) {
-                const int i = FTSP_DIV(idx, C, fC), c = idx - i * C;
-                twiddle_table<S2, R>(u, tb + i, xB);
-                dft_any<S2, R>(u);
-                V* d = b1 + i * pc + c;
-#pragma unroll
-                for (int t = 0; t < R; ++t) d[t * xB * pc] = u[t];
-            });
-    });
-    by_radix<P::CT, P::G.Y2, P::AMAX>(Y2, [&](auto rc) {
-        constexpr int R = decltype(rc)::value;
-        split_phase<P, R, P::G.m1 * P::G.W, NT, false, false, V>(m1 * W,
-            [&](int idx, V (&u)[R]) {
-                const int x = FTSP_DIV(idx, W, fW), w = idx - x * W;
-                const V* s = b1 + x * pc + w;
-#pragma unroll
-                for (int t = 0; t < R; ++t) u[t] = s[t * W];
-            },
-            [&](int idx, V (&u)[R]) {
-                const int x = FTSP_DIV(idx, W, fW), w = idx - x * W;
-                dft_any<S2, R>(u);
-                V* d = dp + (size_t)x * plane + w;
-                if (whole || z0 + w < m3) {
-#pragma unroll
-                    for (int t = 0; t < R; ++t) d[(size_t)t * m3] = u[t];
+                    for (int t = 0; t < R; ++t) d[t * pc] = u[t];
                 }
             });
     });
+    if constexpr (S2 != 0) {
+        by_radix<P::CT, P::G.xA, P::AMAX>(xA, [&](auto rc) {
+            constexpr int R = decltype(rc)::value;
+            split_phase<P, R, P::G.C * P::G.xB, NT, IP, true, V>(C * xB,
+                [&](int idx, V (&u)[R]) {
+                    const int i = FTSP_DIV(idx, C, fC), c = idx - i * C;
+                    const V* s = b0 + i * pc + c;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) u[t] = s[t * xB * pc];
+                },
+                [&](int idx, V (&u)[R]) {
+                    const int i = FTSP_DIV(idx, C, fC), c = idx - i * C;
+                    twiddle_table<S2, R>(u, tb + i, xB);
+                    dft_any<S2, R>(u);
+                    V* d = b1 + i * pc + c;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) d[t * xB * pc] = u[t];
+                });
+        });
+        by_radix<P::CT, P::G.Y2, P::AMAX>(Y2, [&](auto rc) {
+            constexpr int R = decltype(rc)::value;
+            split_phase<P, R, P::G.m1 * P::G.W, NT, false, false, V>(m1 * W,
+                [&](int idx, V (&u)[R]) {
+                    const int x = FTSP_DIV(idx, W, fW), w = idx - x * W;
+                    const V* s = b1 + x * pc + w;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) u[t] = s[t * W];
+                },
+                [&](int idx, V (&u)[R]) {
+                    const int x = FTSP_DIV(idx, W, fW), w = idx - x * W;
+                    dft_any<S2, R>(u);
+                    V* d = dp + (size_t)x * plane + w;
+                    if (whole || z0 + w < m3) {
+#pragma unroll
+                        for (int t = 0; t < R; ++t) d[(size_t)t * m3] = u[t];
+                    }
+                });
+        });
+    }
     op.end(reinterpret_cast<double*>(b0), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
 }
 
 #undef FTSP_PL
 #undef FTSP_DIV
+
+// The k-space pass of a cube with m1 = XP * XQ in two exchanges instead of
+// four: a thread first holds the Y2 rows of XP points x = i + XQ p of one
+// column (DFT over the rows, DFT over p, twiddle), then the XQ points of one
+// (p, row, column) for the second x stage, the op and its inverse; it writes
+// those back where it read them, so the pass has two barriers and the XP - 1
+// twiddles of a thread stay in registers.  About 32 values per thread.
+template <int N, typename T>
+struct CubeK {
+    static constexpr SplitGeom G = split_cube(N, 2 * (int)sizeof(T));
+    static constexpr int BANKS = 128 / (2 * (int)sizeof(T));
+    static constexpr int XP = N % 3 == 0 ? 3 : 4, XQ = N / XP;
+    static constexpr int Y1 = G.Y1, Y2 = G.Y2;
+    static constexpr int W = (N >= 96 ? 64 : 32) / (2 * (int)sizeof(T));   // columns per tile
+    static constexpr int C = Y2 * W;
+    static constexpr int PITCH = C + ((W - C) % BANKS + BANKS) % BANKS;    // threads (i, w) on different banks
+    static constexpr int NZB = N / W;
+    static constexpr int NT = split_round32(split_max(XQ * W, XP * C));
+    static constexpr size_t SMEM = 2 * sizeof(T) * (size_t)N * PITCH + sizeof(T) * (size_t)N;   // tile, x factors
+    static_assert(N % W == 0 && XP * XQ == N, "tile shape");
+};
+
+template <typename T, int N, int S1, int S2, class Op>
+__global__ void __launch_bounds__(CubeK<N, T>::NT, split_max(1, 65536 / (CubeK<N, T>::NT * (sizeof(T) == 4 ? 128 : 255))))
+    k_cube_k(const cplx<T>* __restrict__ tx, const cplx<T>* src, cplx<T>* dst, size_t fstride, Op op)
+{
+    using V = cplx<T>;
+    using P = CubeK<N, T>;
+    constexpr int XP = P::XP, XQ = P::XQ, Y1 = P::Y1, Y2 = P::Y2, W = P::W, C = P::C, PITCH = P::PITCH;
+    static_assert(S1 != 0 && S2 != 0, "both transforms");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    V* tile = reinterpret_cast<V*>(smem_raw);
+    const int tid = threadIdx.x;
+    const int f = blockIdx.y;
+    const int k1 = blockIdx.x / P::NZB;
+    const int z0 = (blockIdx.x % P::NZB) * W;
+    constexpr size_t plane = (size_t)N * N;
+    const size_t inner = (size_t)k1 * Y2 * N + z0;
+    const size_t fbase = (size_t)f * fstride;
+    const V* sp = src + (size_t)op_src_field(op, f) * fstride + inner;
+    V* dp = dst + fbase + inner;
+    const int i = tid / W, w = tid % W;
+    const bool one = XQ * W == P::NT || tid < XQ * W;
+    // the op's x factors: 32 loads per thread from global memory throttled the
+    // load queue (2.5 of 9.5 cycles per instruction at 128^3 complex64)
+    constexpr bool XTAB = op_has_xtab<Op>::value;
+    T* xtab = reinterpret_cast<T*>(tile + N * PITCH);
+    if constexpr (XTAB)
+        for (int j = tid; j < N; j += P::NT) xtab[j] = op.x_table()[j];
+    V tw[XP];
+    if (one) {
+#pragma unroll
+        for (int p = 1; p < XP; ++p) tw[p] = tx[i * p];
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (one) {
+        V u[XP][Y2];
+        const V* s = sp + (size_t)i * plane + w;
+#pragma unroll
+        for (int p = 0; p < XP; ++p)
+#pragma unroll
+            for (int y = 0; y < Y2; ++y) u[p][y] = s[(size_t)(p * XQ) * plane + y * N];
+#pragma unroll
+        for (int p = 0; p < XP; ++p) dft_any<S1, Y2>(u[p]);
+        V* d = tile + i * PITCH + w;
+#pragma unroll
+        for (int y = 0; y < Y2; ++y) {
+            V b[XP];
+#pragma unroll
+            for (int p = 0; p < XP; ++p) b[p] = u[p][y];
+            dft_any<S1, XP>(b);
+#pragma unroll
+            for (int p = 0; p < XP; ++p) {
+                if (p > 0) b[p] = cmul(b[p], S1 > 0 ? mkc<V>(tw[p].x, -tw[p].y) : tw[p]);
+                d[p * XQ * PITCH + y * W] = b[p];
+            }
+        }
+    }
+    op.begin();
+    __syncthreads();
+    if (XP * C == P::NT || tid < XP * C) {
+        const int p = tid / C, c = tid % C;
+        const int y = k1 + Y1 * (c / W), z = z0 + c % W;
+        const size_t off = fbase + (size_t)p * plane + (size_t)y * N + z;
+        V* d = tile + p * XQ * PITCH + c;
+        V u[XQ];
+#pragma unroll
+        for (int q = 0; q < XQ; ++q) u[q] = d[q * PITCH];
+        dft_any<S1, XQ>(u);
+        constexpr int CH = op_loads<Op>::value == 0 ? XQ : XQ < 4 ? XQ : 4;   // operands in flight
+        typename Op::Pre pre[CH];
+        T col = T(0);
+        if constexpr (XTAB) col = op.column(y, z);
+#pragma unroll
+        for (int q = 0; q < XQ; ++q) {
+            if (q % CH == 0) {
+#pragma unroll
+                for (int k = 0; k < CH; ++k)
+                    if (q + k < XQ) pre[k] = op.load(f, off + (size_t)(XP * (q + k)) * plane);
+            }
+            if constexpr (XTAB)
+                u[q] = op.apply_x(p + XP * q, y, z, off + (size_t)(XP * q) * plane, u[q], pre[q % CH], xtab[p + XP * q], col);
+            else
+                u[q] = op.apply(f, p + XP * q, y, z, off + (size_t)(XP * q) * plane, u[q], pre[q % CH]);
+        }
+        dft_any<S2, XQ>(u);
+#pragma unroll
+        for (int q = 0; q < XQ; ++q) d[q * PITCH] = u[q];
+    }
+    __syncthreads();
+    if (one) {
+        V u[XP][Y2];
+        const V* s = tile + i * PITCH + w;
+#pragma unroll
+        for (int y = 0; y < Y2; ++y) {
+            V b[XP];
+#pragma unroll
+            for (int p = 0; p < XP; ++p) {
+                b[p] = s[p * XQ * PITCH + y * W];
+                if (p > 0) b[p] = cmul(b[p], S2 > 0 ? mkc<V>(tw[p].x, -tw[p].y) : tw[p]);
+            }
+            dft_any<S2, XP>(b);
+#pragma unroll
+            for (int p = 0; p < XP; ++p) u[p][y] = b[p];
+        }
+        V* d = dp + (size_t)i * plane + w;
+#pragma unroll
+        for (int p = 0; p < XP; ++p) {
+            dft_any<S2, Y2>(u[p]);
+#pragma unroll
+            for (int y = 0; y < Y2; ++y) d[(size_t)(p * XQ) * plane + y * N] = u[p][y];
+        }
+    }
+    op.end(reinterpret_cast<double*>(tile), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
+}
+
+// ---- launches ----
+// Launched as dependents of the kernel before them (programmatic dependent
+// launch): the prologue overlaps its tail.
+template <class... Params, class... Args>
+inline cudaError_t split_launch(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args)
+{
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <class P, typename T, int S1, int S2, class Op>
+cudaError_t split_real_plan(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst, size_t fstride, int nf, const Op& op,
+                            cudaStream_t stream)
+{
+    const SplitGeom& p = P::CT ? P::G : g;
+    return split_launch(k_split_real<T, P, S1, S2, Op>, dim3(p.m1 * (p.Y2 / p.G), nf), p.r_threads,
+                        split_real_smem<P, cplx<T>>(p), stream, g, src, dst, fstride, op);
+}
+template <class P, typename T, int S1, int S2, class Op>
+cudaError_t split_k_plan(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst, size_t fstride, int nf, const Op& op,
+                         cudaStream_t stream)
+{
+    const SplitGeom& p = P::CT ? P::G : g;
+    return split_launch(k_split_k<T, P, S1, S2, Op>, dim3(p.Y1 * p.nzb, nf), p.k_threads, split_k_smem<P, cplx<T>>(p),
+                        stream, g, src, dst, fstride, op);
+}
+// blocks of one field of the real-space pass
+inline int split_real_blocks(const SplitGeom& g) { return g.m1 * (g.Y2 / g.G); }
+
+// The production cubes run their compile-time plans (where g says so), the
+// passes at the ends of a sweep (one transform, run once) the run-time one.
+template <typename T, int S1, int S2, class Op>
+cudaError_t split_real_launch(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst, size_t fstride, int nf, const Op& op,
+                              cudaStream_t stream)
+{
+    if constexpr (S1 != 0 && S2 != 0) switch (g.cube) {
+        case 32: return split_real_plan<CubePlan<32, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+        case 48: return split_real_plan<CubePlan<48, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+        case 64: return split_real_plan<CubePlan<64, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+        case 96: return split_real_plan<CubePlan<96, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+        case 128: return split_real_plan<CubePlan<128, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+        default: break;
+    }
+    if (g.big) return split_real_plan<RtBigPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+    return split_real_plan<RtPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+}
+template <int N, typename T, int S1, int S2, class Op>
+cudaError_t cube_k(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst, size_t fstride, int nf, const Op& op, cudaStream_t stream)
+{
+    using P = CubeK<N, T>;
+    return split_launch(k_cube_k<T, N, S1, S2, Op>, dim3(P::Y1 * P::NZB, nf), P::NT, P::SMEM, stream,
+                        reinterpret_cast<const cplx<T>*>(g.tx), src, dst, fstride, op);
+}
+template <typename T, int S1, int S2, class Op>
+cudaError_t split_k_launch(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst, size_t fstride, int nf, const Op& op,
+                           cudaStream_t stream)
+{
+    if constexpr (S1 != 0 && S2 != 0) switch (g.cube) {
+        case 32: return split_k_plan<CubePlan<32, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+        case 48: return split_k_plan<CubePlan<48, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+        case 64: return split_k_plan<CubePlan<64, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+        case 96: return cube_k<96, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+        case 128: return cube_k<128, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+        default: break;
+    }
+    if (g.big) return split_k_plan<RtBigPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+    return split_k_plan<RtPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+}
+
+// The sweeps' passes are compiled in split_real_*.cu and split_k_*.cu.
+#define FTSP_SPLIT_REAL(PRE, T, S1, S2, KIND)                                                                             \
+    PRE cudaError_t split_real_launch<T, S1, S2, OpProp<T, KIND>>(const SplitGeom&, const cplx<T>*, cplx<T>*, size_t, int, \
+                                                                  const OpProp<T, KIND>&, cudaStream_t);
+#define FTSP_SPLIT_REAL_ALL(PRE, T)                                                                                  \
+    FTSP_SPLIT_REAL(PRE, T, 0, -1, FWD_START)                                                                        \
+    FTSP_SPLIT_REAL(PRE, T, 1, -1, FWD_MID)                                                                          \
+    FTSP_SPLIT_REAL(PRE, T, 1, 0, FWD_LAST)                                                                          \
+    FTSP_SPLIT_REAL(PRE, T, 0, 0, FWD_SINGLE)                                                                        \
+    FTSP_SPLIT_REAL(PRE, T, 0, 1, BWD_START)                                                                         \
+    FTSP_SPLIT_REAL(PRE, T, -1, 1, BWD_MID)                                                                          \
+    FTSP_SPLIT_REAL(PRE, T, -1, 0, BWD_LAST)                                                                         \
+    FTSP_SPLIT_REAL(PRE, T, 0, 0, BWD_SINGLE)
+#define FTSP_SPLIT_K(PRE, T, S1, S2, F, ST)                                                                              \
+    PRE cudaError_t split_k_launch<T, S1, S2, OpBond<T, F, ST>>(const SplitGeom&, const cplx<T>*, cplx<T>*, size_t, int, \
+                                                                const OpBond<T, F, ST>&, cudaStream_t);
+#define FTSP_SPLIT_K_ALL(PRE, T)                                                                                     \
+    FTSP_SPLIT_K(PRE, T, -1, 1, true, false)                                                                         \
+    FTSP_SPLIT_K(PRE, T, 1, -1, false, true)                                                                         \
+    FTSP_SPLIT_K(PRE, T, 1, -1, false, false)
+#ifndef FTSP_SPLIT_INSTANCES
+FTSP_SPLIT_REAL_ALL(extern template, float)
+FTSP_SPLIT_REAL_ALL(extern template, double)
+FTSP_SPLIT_K_ALL(extern template, float)
+FTSP_SPLIT_K_ALL(extern template, double)
+#endif
 
 }  // namespace ftsp

@@ -21,6 +21,7 @@
 #include <mutex>
 #include <tuple>
 #include <stdexcept>
+#include <thread>
 #include <string>
 #include <vector>
 
@@ -486,7 +487,6 @@ struct OpPrecond {
     SigTab st;               // dt lambda_f per field
     T invV;
     int dc0 = -1;            // field whose k = 0 value is set to zero (psi: its mean removal), -1: none
-    static constexpr int FUSED_MIN_BLOCKS = 8;
     static constexpr int LOADS = 0;
     struct Pre {};
     __device__ __forceinline__ void begin() {}
@@ -513,7 +513,6 @@ template <typename T>
 struct OpKScale {
     using V = cplx<T>;
     static constexpr int NSRC = 4;
-    static constexpr int FUSED_MIN_BLOCKS = 8;
     V* kst;
     const T* gm;             // Gamma per axis: x, then y, then z
     const double* kx;
@@ -913,8 +912,6 @@ struct Engine : EngineBase {
     static constexpr bool F32 = sizeof(T) == 4;
     static constexpr int EP = F32 ? 32 : 16;   // elements per thread, runtime-plan plane pass
     static constexpr int EL = F32 ? 16 : 8;    // elements per thread, runtime-plan line passes
-    static constexpr int RMAX = F32 ? 16 : 8;  // largest radix of the compile-time transforms
-    static constexpr int WCT = F32 ? 16 : 8;   // z-columns per tile of the compile-time strided passes (128-byte rows)
     Buf<FftPlan1> plans;                       // device-memory plans: x, y, z
 
     // device buffers
@@ -956,8 +953,6 @@ struct Engine : EngineBase {
     };
     std::vector<SymTables> sym;
     bool chain_sym = true;       // use the pair kernels for mirror-symmetric species
-    bool fused_strided = true;   // bond passes with register-resident middle stages (k_strided_fused)
-    bool fused_plane = true;     // field loads with a register-resident first stage (k_plane_load_fused)
     // every ion smeared like the beads (and at most 3 ion species): the ion
     // potentials are psi_s itself, and the ion charge is one combined field
     // sum_j z_j (n_j/V)/Q_j exp(-i z_j psi_s), transformed once (see eval)
@@ -979,6 +974,8 @@ struct Engine : EngineBase {
         FTSP_CUDA(cudaSetDevice(c.device));
         V_ = c.V;
         setup_geometry();
+        ion_common = c.elec && !c.ions.empty() && c.ions.size() <= 3;
+        for (auto& ion : c.ions) ion_common = ion_common && ion.smear == c.a;
         allocate();
         build_tables();
         plan_charge_fold();
@@ -1109,7 +1106,7 @@ struct Engine : EngineBase {
         for (auto& s : c.sp) Nmax = std::max(Nmax, s.N);
         qF.alloc(Vn * Nmax);
         if (c.stress_on()) Fst.alloc(Vn * Nmax);
-        G.alloc(Vn); H.alloc(Vn);
+        G.alloc(std::max<size_t>(Vn, 2)); H.alloc(Vn);   // G: also one FP64 value of copy_out at least
         part.alloc((size_t)std::max(RED_BLOCKS, std::max(c.m1, c.m1 * c.m2)) * 32);
         expo.alloc((size_t)2 * Nmax);
         pmax.alloc((size_t)2 * std::max(c.m1, c.m1 * c.m2));
@@ -1120,9 +1117,9 @@ struct Engine : EngineBase {
         }
         smax.alloc(std::max<size_t>(1, slots));
         split_tw.alloc((size_t)3 * c.m1 + c.m2 + 2 * c.m3);
-        // as many fields as the widest batch of the evaluation that runs fft3;
-        // two for the learned preconditioner, the tuner and the fused evaluation
-        if (use_split) fscr.alloc(Vn * (size_t)std::max({M + 3, M + 1 + J, nm + 1}));
+        // as many fields as the widest batch of the evaluation that runs fft3
+        // (the learned preconditioner, the other user, allocates its own)
+        if (use_split && !eval_fused_ok()) fscr.alloc(Vn * (size_t)std::max({M + 3, M + 1 + J, nm + 1}));
         spart.alloc((size_t)c.m2 * c.m3 * 12);
         if (c.restart_interval > 0) ck.alloc((size_t)(std::max(1, c.nm) + 1) * V_);
         FTSP_CUDA(cudaMalloc(&ds, sizeof(DevScal)));
@@ -1170,12 +1167,7 @@ struct Engine : EngineBase {
     }
     TuneResult tune{};
 
-    bool all_compile_time() const
-    {
-        const bool plane = plane_ok && c.m2 == c.m3 && (c.m3 == 32 || c.m3 == 64 || c.m3 == 128) &&
-                           (F32 || c.m3 != 128);
-        return plane && strided_is_ct(c.m1);
-    }
+    bool all_compile_time() const { return use_split && (sg.cube == 32 || sg.cube == 64 || sg.cube == 128); }
 
     double time_fft(int reps)
     {
@@ -1347,8 +1339,6 @@ struct Engine : EngineBase {
         }
         if (gi.empty()) gi = sep(0.0);
         upload(gion, gi);
-        ion_common = c.elec && !c.ions.empty() && c.ions.size() <= 3;
-        for (auto& ion : c.ions) ion_common = ion_common && ion.smear == c.a;
         if (c.scheme == FTSP_SCHEME_SI) build_si_tables();
     }
 
@@ -1730,6 +1720,7 @@ struct Engine : EngineBase {
         lr.nb = lr.batch / mlp::GRAD_THREADS;
         const size_t Vn = V_;
         lr.A.alloc(nf * Vn); lr.B.alloc(nf * Vn); lr.Pw.alloc(Vn); lr.Pp.alloc(Vn);
+        if (use_split && !fscr.p) fscr.alloc(std::max(nf, 2) * Vn);   // transforms of du and of the spectral powers
         lr.GL.alloc(nf * Vn); lr.dw.alloc(nf * Vn); lr.du.alloc(nf * Vn); lr.fk.alloc(2 * Vn);
         lr.w.alloc(lr.np); lr.m1.alloc(lr.np); lr.m2.alloc(lr.np);
         lr.partial.alloc((size_t)lr.nb * lr.np); lr.lpart.alloc(2 * (size_t)lr.nb); lr.loss.alloc(2);
@@ -2113,12 +2104,7 @@ struct Engine : EngineBase {
         prof_end(ev, "field_reduce", bpe * (double)n);
     }
 
-    // Batched in-place (or out-of-place from per-field sources) 3-D FFT of nf
-    // contiguous fields of dst.  src[f] (optional) gives the input of field f.
-    // ---- pass launchers: compile-time kernels for the production lengths
-    // (32, 64, 128), runtime-plan kernels for every other 2/3/5-smooth grid ----
-    template <int N> static constexpr bool plane_ct_ok() { return F32 ? (N == 32 || N == 64 || N == 128) : (N == 32 || N == 64); }
-
+    // ---- pass launchers ----
     // Launches a pass kernel with programmatic dependent launch (the kernel
     // waits for its predecessor with griddepcontrol.wait).
     bool use_pdl = true;
@@ -2142,44 +2128,10 @@ struct Engine : EngineBase {
         FTSP_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
     }
 
-    template <int N, int S1, int S2, class Op>
-    void plane_ct(const V* src, V* dst, int nf, const Op& op)
-    {
-        constexpr int E = F32 ? (N >= 128 ? 16 : 16) : (N >= 64 ? 16 : 8);
-        constexpr int NT = N * N / E;
-        const size_t smem = std::max(sizeof(V) * (size_t)(N * (N + 1) + N), (size_t)4096);
-        // field loads (one value per point) only: wider operators keep their batched loads
-        if constexpr (S1 == 0 && S2 != 0 && sizeof(typename Op::Pre) == sizeof(V) && plane_fused_ok<N, RMAX, NT, E>()) {
-            if (fused_plane) {
-                auto k = k_plane_load_fused<T, N, RMAX, NT, E, S2, Op>;
-                set_smem(k, smem);
-                launch_pass(k, dim3(c.m1, nf), NT, smem, dst, (size_t)V_, (const V*)tw3.p, op);
-                ++launches;
-                return;
-            }
-        }
-        auto k = k_plane_ct<T, N, RMAX, NT, E, S1, S2, Op>;
-        set_smem(k, smem);
-        launch_pass(k, dim3(c.m1, nf), NT, smem, src, dst, (size_t)V_, (const V*)tw3.p, op);
-        ++launches;
-    }
-
+    // The plane, strided and z-line passes (run-time plans): grids that the
+    // split-y passes do not take.
     template <int S1, int S2, class Op>
     void plane(const V* src, V* dst, int nf, const Op& op)
-    {
-        if (c.m2 == c.m3) {
-            if constexpr (plane_ct_ok<128>())
-                if (c.m3 == 128) return plane_ct<128, S1, S2>(src, dst, nf, op);
-            if constexpr (plane_ct_ok<64>())
-                if (c.m3 == 64) return plane_ct<64, S1, S2>(src, dst, nf, op);
-            if constexpr (plane_ct_ok<32>())
-                if (c.m3 == 32) return plane_ct<32, S1, S2>(src, dst, nf, op);
-        }
-        plane_rt<S1, S2>(src, dst, nf, op);
-    }
-    // the run-time plan (the only one that the sweeps of a grid without split passes use)
-    template <int S1, int S2, class Op>
-    void plane_rt(const V* src, V* dst, int nf, const Op& op)
     {
         auto kp = k_plane<T, EP, S1, S2, Op>;
         set_smem(kp, plane_smem);
@@ -2187,84 +2139,15 @@ struct Engine : EngineBase {
         ++launches;
     }
 
-    template <int DIM, int N, int S1, int S2, class Op>
-    void strided_ct(const V* src, V* dst, int nf, const Op& op)
-    {
-        constexpr int E = F32 ? 16 : 8;
-        constexpr int NT = N * WCT / E;
-        const size_t smem = std::max(sizeof(V) * (size_t)(N * WCT + N), (size_t)4096);
-        const int outer = DIM == 1 ? c.m1 : c.m2;
-        // field loads (one value per point) only: wider operators keep their batched loads
-        if constexpr (S1 == 0 && S2 != 0 && sizeof(typename Op::Pre) == sizeof(V) && strided_fused_ok<N, WCT, RMAX, NT, E>()) {
-            if (fused_strided) {
-                auto k = k_strided_load_fused<T, N, WCT, DIM, RMAX, NT, E, S2, Op>;
-                set_smem(k, smem);
-                launch_pass(k, dim3(outer * (c.m3 / WCT), nf), NT, smem, c.m2, c.m3, dst, (size_t)V_,
-                            (const V*)(DIM == 1 ? tw2.p : tw1.p), op);
-                ++launches;
-                return;
-            }
-        }
-        if constexpr (S1 != 0 && S2 != 0 && strided_fused_ok<N, WCT, RMAX, NT, E>()) {
-            if (fused_strided) {
-                auto k = k_strided_fused<T, N, WCT, DIM, RMAX, NT, E, S1, S2, Op>;
-                set_smem(k, smem);
-                launch_pass(k, dim3(outer * (c.m3 / WCT), nf), NT, smem, c.m2, c.m3, src, dst, (size_t)V_,
-                            (const V*)(DIM == 1 ? tw2.p : tw1.p), op);
-                ++launches;
-                return;
-            }
-        }
-        if constexpr (op_has_src<Op>::value) {
-            throw std::runtime_error("pencil op with a source map needs the fused pencil pass");
-        } else {
-            auto k = k_strided_ct<T, N, WCT, DIM, RMAX, NT, E, S1, S2, Op>;
-            set_smem(k, smem);
-            launch_pass(k, dim3(outer * (c.m3 / WCT), nf), NT, smem, c.m2, c.m3, src, dst, (size_t)V_,
-                        (const V*)(DIM == 1 ? tw2.p : tw1.p), op);
-            ++launches;
-        }
-    }
-
-    bool strided_is_ct(int n) const { return c.m3 % WCT == 0 && (n == 32 || n == 64 || n == 128); }
-
-    // the x pass of length n runs k_strided_fused (both transforms in one pass)
-    template <int N>
-    static constexpr bool x_fused_ct()
-    {
-        constexpr int E = F32 ? 16 : 8;
-        return strided_fused_ok<N, WCT, RMAX, N * WCT / E, E>();
-    }
-    bool x_fused(int n) const
-    {
-        if (!fused_strided || !strided_is_ct(n)) return false;
-        return n == 128 ? x_fused_ct<128>() : n == 64 ? x_fused_ct<64>() : x_fused_ct<32>();
-    }
-    // the density evaluation with its k-space factors inside x-pencil passes:
+    // the density evaluation with its k-space factors inside the split passes:
     // one interaction mode, one monomer type, every ion smeared like the beads
-    bool eval_fused_ok() const
-    {
-        return c.nm == 1 && c.M == 1 && ion_common && (use_split || (plane_ok && x_fused(c.m1)));
-    }
+    bool eval_fused_ok() const { return use_split && c.nm == 1 && c.M == 1 && ion_common; }
 
     template <int DIM, int S1, int S2, class Op>
     void strided(const V* src, V* dst, int nf, const Op& op)
     {
-        const int n = DIM == 1 ? c.m2 : c.m1;
-        if constexpr (DIM == 0 || !F32) {
-            if (strided_is_ct(n)) {
-                if (n == 128) return strided_ct<DIM, 128, S1, S2>(src, dst, nf, op);
-                if (n == 64) return strided_ct<DIM, 64, S1, S2>(src, dst, nf, op);
-                return strided_ct<DIM, 32, S1, S2>(src, dst, nf, op);
-            }
-        }
-        strided_rt<DIM, S1, S2>(src, dst, nf, op);
-    }
-    template <int DIM, int S1, int S2, class Op>
-    void strided_rt(const V* src, V* dst, int nf, const Op& op)
-    {
         if constexpr (op_has_src<Op>::value) {
-            throw std::runtime_error("pencil op with a source map needs the fused pencil pass");
+            throw std::runtime_error("an op with a source map needs the split passes");
         } else {
             const LineGeom& g = DIM == 1 ? gy : gx;
             auto k = k_strided<T, EL, DIM, S1, S2, Op>;
@@ -2279,22 +2162,6 @@ struct Engine : EngineBase {
 
     template <int S1, int S2, class Op>
     void zline(const V* src, V* dst, int nf, const Op& op)
-    {
-        if constexpr (!F32) {
-            if (c.m3 == 128 && (c.m1 * c.m2) % 16 == 0) {
-                constexpr int N = 128, BR = 16, E = 8, NT = BR * N / E;
-                auto k = k_zline_ct<T, N, BR, RMAX, NT, E, S1, S2, Op>;
-                const size_t smem = sizeof(V) * (size_t)(BR * (N + 1) + N);
-                set_smem(k, smem);
-                k<<<dim3(c.m1 * c.m2 / BR, nf), NT, smem, stream>>>(c.m2, src, dst, V_, tw3.p, op);
-                ++launches;
-                return;
-            }
-        }
-        zline_rt<S1, S2>(src, dst, nf, op);
-    }
-    template <int S1, int S2, class Op>
-    void zline_rt(const V* src, V* dst, int nf, const Op& op)
     {
         auto k = k_zline<T, EL, S1, S2, Op>;
         set_smem(k, z_smem);
@@ -2415,11 +2282,11 @@ struct Engine : EngineBase {
             return;
         }
         if (plane_ok) {
-            plane_rt<S1, S2>(src, dst, 1, op);
+            plane<S1, S2>(src, dst, 1, op);
             return;
         }
         if (S1 != 0) strided<1, 0, S1>(nullptr, const_cast<V*>(src), 1, OpLoadOne{src});   // y-lines, in place
-        zline_rt<S1, S2>(src, dst, 1, op);
+        zline<S1, S2>(src, dst, 1, op);
         if (S2 != 0) strided<1, 0, S2>(nullptr, dst, 1, OpLoadOne{dst});                    // y-lines, in place
     }
 
@@ -2432,7 +2299,7 @@ struct Engine : EngineBase {
     // blocks that write connectivity-stress partials: the pair kernel's (x_ctas)
     // and, with the split passes, the backward bond pass's
     int stress_parts() const { return std::max(x_ctas(), use_split ? sg.Y1 * sg.nzb : 0); }
-    int x_ctas() const { return c.m2 * (c.m3 / (strided_is_ct(c.m1) ? WCT : gx.W)); }
+    int x_ctas() const { return c.m2 * (c.m3 / gx.W); }
 
     template <int S1, int S2, bool FWD, bool STRESS>
     void bond_pass(const V* src, V* dst, const OpBond<T, FWD, STRESS>& op)
@@ -2441,7 +2308,7 @@ struct Engine : EngineBase {
         if (use_split) {
             split_k<S1, S2>(src, dst, 1, op);
         } else {
-            strided_rt<0, S1, S2>(src, dst, 1, op);
+            strided<0, S1, S2>(src, dst, 1, op);
         }
         // G in, H out, plus the stored/read forward spectrum when the stress is on
         const bool extra = FWD ? op.Fstore != nullptr : STRESS;
@@ -3531,6 +3398,42 @@ struct Engine : EngineBase {
         }, ds->kobs + 14, 2.0 * sizeof(V));
     }
 
+    // Number of wave vectors k != 0 of the grid and sum k_a k_b / k^2 over
+    // them: constants of the grid, summed once per handle (every measure()
+    // and every step launched without a graph read them).  Over the
+    // non-negative half of each axis: a component and its opposite share k^2,
+    // so a diagonal term counts every pair twice and an off-diagonal one
+    // keeps only the wave numbers without an opposite (the Nyquist ones).
+    long long mode_count = -1;
+    double mode_sum[6] = {0, 0, 0, 0, 0, 0};
+    void mode_sums()
+    {
+        const int n[3] = {c.m1, c.m2, c.m3};
+        std::vector<double> k[3], all[3], odd[3];   // wave number, its multiplicity, its unpaired part
+        for (int d = 0; d < 3; ++d)
+            for (int i = 0; i <= n[d] / 2; ++i) {
+                const bool pair = i > 0 && 2 * i != n[d];
+                k[d].push_back(wave_number(i, n[d], c.L[d]));
+                all[d].push_back(pair ? 2.0 : 1.0);
+                odd[d].push_back(pair ? 0.0 : k[d].back());
+            }
+        for (double& v : mode_sum) v = 0.0;
+        for (size_t x = 0; x < k[0].size(); ++x)
+            for (size_t y = 0; y < k[1].size(); ++y)
+                for (size_t z = 0; z < k[2].size(); ++z) {
+                    const double k2 = k[0][x] * k[0][x] + k[1][y] * k[1][y] + k[2][z] * k[2][z];
+                    if (!(k2 > 0.0)) continue;
+                    const double inv = 1.0 / k2, w = all[0][x] * all[1][y] * all[2][z];
+                    mode_sum[0] += w * k[0][x] * k[0][x] * inv;
+                    mode_sum[1] += w * k[1][y] * k[1][y] * inv;
+                    mode_sum[2] += w * k[2][z] * k[2][z] * inv;
+                    mode_sum[3] += odd[0][x] * odd[1][y] * all[2][z] * inv;
+                    mode_sum[4] += odd[0][x] * all[1][y] * odd[2][z] * inv;
+                    mode_sum[5] += all[0][x] * odd[1][y] * odd[2][z] * inv;
+                }
+        mode_count = (long long)V_ - 1;
+    }
+
     void finalize_record(bool with_stress)
     {
         if (with_stress) {
@@ -3558,24 +3461,9 @@ struct Engine : EngineBase {
         for (auto& s : c.sp) chains += s.nc;
         const double ideal = (chains + ion_total) / c.volume;
         // mode term of stress::build_kernels (stress.cu:106-149)
-        double sum[6] = {0, 0, 0, 0, 0, 0};
-        long long modes = 0;
-        if (c.elec) {
-            std::vector<double> hx(c.m1), hy(c.m2), hz(c.m3);
-            for (int i = 0; i < c.m1; ++i) hx[i] = wave_number(i, c.m1, c.L[0]);
-            for (int i = 0; i < c.m2; ++i) hy[i] = wave_number(i, c.m2, c.L[1]);
-            for (int i = 0; i < c.m3; ++i) hz[i] = wave_number(i, c.m3, c.L[2]);
-            for (int x = 0; x < c.m1; ++x)
-                for (int y = 0; y < c.m2; ++y)
-                    for (int z = 0; z < c.m3; ++z) {
-                        const double k2 = hx[x] * hx[x] + hy[y] * hy[y] + hz[z] * hz[z];
-                        if (k2 > 0.0) {
-                            ++modes;
-                            const double v[6] = {hx[x] * hx[x], hy[y] * hy[y], hz[z] * hz[z], hx[x] * hy[y], hx[x] * hz[z], hy[y] * hz[z]};
-                            for (int cc = 0; cc < 6; ++cc) sum[cc] += v[cc] / k2;
-                        }
-                    }
-        }
+        if (c.elec && mode_count < 0) mode_sums();
+        const long long modes = c.elec ? mode_count : 0;
+        const double* sum = mode_sum;
         for (int cc = 0; cc < 6; ++cc) {
             const double delta = cc < 3 ? 1.0 : 0.0;
             const double mode_term = c.elec ? ((1.0 / 3.0) * (double)modes * delta - sum[cc]) / c.volume : 0.0;
@@ -3754,6 +3642,50 @@ struct Engine : EngineBase {
         }
     }
 
+    // n device values to host memory as FP64 pairs: converted on the device
+    // (complex64: through the sweeps' scratch field, half a field at a time)
+    // and copied straight to the caller.  Above 16 MiB the caller's pages are
+    // touched by a few threads first: memory of that size comes fresh from
+    // the system, and its first touch costs more than the copy.  Measured,
+    // complex64 into fresh memory: 128^3 18 ms (copy, then a host loop) -> 6,
+    // 96^3 3.3 -> 2.0, 64^3 1.0 -> 0.65; a pinned staging buffer was no
+    // faster and took 2-7 ms to allocate.
+    void copy_out(const V* p, size_t n, double* out)
+    {
+        const size_t bytes = n * sizeof(double2);
+        if (bytes >= ((size_t)16 << 20)) {
+            const size_t pages = bytes / 4096;
+            auto touch = [out](size_t a, size_t b) {
+                for (size_t i = a; i < b; ++i) *reinterpret_cast<volatile double*>(out + i * 512) = 0.0;
+            };
+            const size_t nt = std::min(8u, std::max(1u, std::thread::hardware_concurrency()));
+            std::vector<std::thread> pool;
+            size_t done = 0;
+            try {
+                for (size_t t = 0; t + 1 < nt; ++t) {
+                    pool.emplace_back(touch, done, pages * (t + 1) / nt);
+                    done = pages * (t + 1) / nt;
+                }
+            } catch (...) {   // no more threads: the rest here
+            }
+            touch(done, pages);
+            for (auto& t : pool) t.join();
+        }
+        if constexpr (!F32) {
+            FTSP_CUDA(cudaMemcpyAsync(out, p, bytes, cudaMemcpyDeviceToHost, stream));
+        } else {
+            double2* d = reinterpret_cast<double2*>(G.p);
+            const size_t chunk = std::max<size_t>(1, V_ / 2);
+            for (size_t i0 = 0; i0 < n; i0 += chunk) {
+                const size_t m = std::min(chunk, n - i0);
+                const V* src = p + i0;
+                foreach(m, [=] __device__(size_t i) { d[i] = to_d(src[i]); });
+                FTSP_CUDA(cudaMemcpyAsync(out + 2 * i0, d, sizeof(double2) * m, cudaMemcpyDeviceToHost, stream));
+            }
+        }
+        FTSP_CUDA(cudaStreamSynchronize(stream));
+    }
+
     long long get_field(const std::string& name, double* out) override
     {
         install_pending_fields();
@@ -3837,13 +3769,15 @@ struct Engine : EngineBase {
             return (long long)(2 * nr);
         }
         else return -1;
-        if (out && n) {
+        if (out && n && name != "qF") {
+            copy_out(p, n, out);
+        } else if (out && n) {
             std::vector<V> tmp(n);
             FTSP_CUDA(cudaMemcpyAsync(tmp.data(), p, sizeof(V) * n, cudaMemcpyDeviceToHost, stream));
             std::vector<int> ex((size_t)Nmax, 0);
-            if (name == "qF") FTSP_CUDA(cudaMemcpyAsync(ex.data(), expo.p, sizeof(int) * Nmax, cudaMemcpyDeviceToHost, stream));
+            FTSP_CUDA(cudaMemcpyAsync(ex.data(), expo.p, sizeof(int) * Nmax, cudaMemcpyDeviceToHost, stream));
             // a mirror-symmetric species stores u = q / E (u = 1 at s = 0): q = u E
-            const int su = name == "qF" ? qF_holds_u : -1;
+            const int su = qF_holds_u;
             std::vector<V> et;
             if (su >= 0) {
                 et.resize(E.n);
@@ -3852,7 +3786,7 @@ struct Engine : EngineBase {
             FTSP_CUDA(cudaStreamSynchronize(stream));
             for (size_t i = 0; i < n; ++i) {
                 // qF is stored renormalised by 2^-aF[s]; return the true propagator
-                const int e2 = name == "qF" ? ex[i / Vn] : 0;
+                const int e2 = ex[i / Vn];
                 double qx = (double)tmp[i].x, qy = (double)tmp[i].y;
                 const size_t seg = i / Vn;
                 if (su >= 0 && seg < (size_t)c.sp[su].N) {

@@ -379,14 +379,6 @@ __device__ __forceinline__ int reduce_exponent(const float* pm, int n) { return 
 //             propagation continues with qB[s] = u * E.
 enum PropKind { FWD_START = 0, FWD_MID = 1, FWD_LAST = 2, FWD_SINGLE = 3, BWD_START = 4, BWD_MID = 5, BWD_LAST = 6, BWD_SINGLE = 7 };
 
-// Bulk prefetch of a contiguous global range into L2 (the TMA unit's
-// non-blocking prefetch: no shared memory, no barrier, nothing to wait on).
-// Address 16-byte aligned, size a multiple of 16.
-__device__ __forceinline__ void l2_prefetch_bulk(const void* p, unsigned bytes)
-{
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
 template <typename T, int KIND>
 struct OpProp {
     using V = cplx<T>;
@@ -474,19 +466,6 @@ struct OpProp {
             if (rho_charge) p.c = rho_charge[g];
         }
         return p;
-    }
-    // the operands of the pointwise step of one plane (elements g0 .. g0+n),
-    // requested at kernel start so that the loads after the inverse transform
-    // find them in L2
-    __device__ __forceinline__ void prefetch(size_t g0, unsigned n) const
-    {
-        const unsigned bytes = n * (unsigned)sizeof(V);
-        if (NEED_E) l2_prefetch_bulk(E + g0, bytes);
-        if (!FWD) {
-            l2_prefetch_bulk(qread + g0, bytes);
-            l2_prefetch_bulk(rho_type + g0, bytes);
-            if (rho_charge) l2_prefetch_bulk(rho_charge + g0, bytes);
-        }
     }
     __device__ __forceinline__ void track(V q)
     {
@@ -578,10 +557,6 @@ struct OpBond {
     const int* eB;
     int s, N;                // bond s -> s+1 of a species with N segments
     double acc[12];
-    // resident CTAs per SM asked of the fused bond pass: without the stress
-    // sums it fits 64 registers, so a 128^3 pass (1024 CTAs of 128 threads)
-    // runs in one wave; with them, fewer registers would spill
-    static constexpr int FUSED_MIN_BLOCKS = STRESS ? 2 : 8;
     static constexpr int LOADS = STRESS ? 4 : 0;   // global loads per point (the stress sums need the registers of four)
     struct Pre {
         V F;
@@ -656,191 +631,7 @@ struct OpBond {
 namespace ftsp {
 
 
-// ---------------------------------------------------------------------------
-// Compile-time specialisations of the three passes for production grids.
-// Same structure and Op interface as the runtime-plan kernels above; all
-// sizes are template constants.
-// ---------------------------------------------------------------------------
-
-// Plane pass for an m2 = m3 = N plane, NT threads, E elements per thread.
-template <typename T, int N, int RMAX, int NT, int E, int S1, int S2, class Op>
-__global__ void __launch_bounds__(NT, 1) k_plane_ct(const cplx<T>* src, cplx<T>* dst, size_t fstride,
-                                                    const cplx<T>* __restrict__ twn, Op op)
-{
-    using V = cplx<T>;
-    constexpr int P = N + 1, NE = N * N;
-    static_assert(NE <= NT * E, "plane does not fit the thread block");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V* tile = reinterpret_cast<V*>(smem_raw);
-    V* stw = tile + N * P;
-    const int x = blockIdx.x;
-    const int f = blockIdx.y;
-    const size_t base = (size_t)f * fstride + (size_t)x * NE;
-    if (S1 != 0 || S2 != 0)
-        for (int j = threadIdx.x; j < N; j += NT) stw[j] = twn[j];
-    pdl_wait();
-    constexpr int EPT = (NE + NT - 1) / NT;   // elements per thread
-    if (S1 != 0) {
-        V v[EPT];   // every load of the thread in flight before the first smem store
-#pragma unroll
-        for (int u = 0; u < EPT; ++u) {
-            const int e = threadIdx.x + u * NT;
-            if (NE % NT == 0 || e < NE) v[u] = src[base + e];
-        }
-#pragma unroll
-        for (int u = 0; u < EPT; ++u) {
-            const int e = threadIdx.x + u * NT;
-            if (NE % NT == 0 || e < NE) tile[(e / N) * P + e % N] = v[u];
-        }
-        __syncthreads();
-        ct_fft<V, S1, N, RMAX, N, 1, P, NT, E>(tile, stw);   // z-lines
-        ct_fft<V, S1, N, RMAX, N, P, 1, NT, E>(tile, stw);   // y-lines
-    } else {
-        __syncthreads();
-    }
-    op.begin();
-    constexpr int PB = (sizeof(T) == 4 && NT < 1024) ? 8 : 4;
-#pragma unroll 1
-    for (int u0 = 0; u0 < EPT; u0 += PB) {
-        typename Op::Pre pre[PB];
-#pragma unroll
-        for (int k = 0; k < PB; ++k) {
-            const int e = threadIdx.x + (u0 + k) * NT;
-            if (u0 + k < EPT && (NE % NT == 0 || e < NE)) pre[k] = op.load(f, base + e);
-        }
-#pragma unroll
-        for (int k = 0; k < PB; ++k) {
-            const int e = threadIdx.x + (u0 + k) * NT;
-            if (u0 + k < EPT && (NE % NT == 0 || e < NE)) {
-                const int y = e / N, z = e % N;
-                V v = S1 != 0 ? tile[y * P + z] : mkc<V>(T(0), T(0));
-                v = op.apply(f, x, y, z, base + e, v, pre[k]);
-                if (S2 != 0) tile[y * P + z] = v;
-            }
-        }
-    }
-    pdl_trigger();
-    if (S2 != 0) {
-        __syncthreads();
-        ct_fft<V, S2, N, RMAX, N, 1, P, NT, E>(tile, stw);
-        ct_fft<V, S2, N, RMAX, N, P, 1, NT, E>(tile, stw);
-        for (int e = threadIdx.x; e < NE; e += NT) dst[base + e] = tile[(e / N) * P + e % N];
-    }
-    op.end(reinterpret_cast<double*>(tile), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
-}
-
-// Shapes of k_plane_load_fused: the coalesced load of a thread (rows
-// tid/N + u*NT/N of column tid%N) is the input set of its first radix stage
-// along y.
-template <int N, int RMAX, int NT, int E>
-__host__ __device__ constexpr bool plane_fused_ok()
-{
-    constexpr int NST = ct_nst(N, RMAX);
-    if (NST < 2 || NT % N != 0) return false;
-    using A0 = CtSt<N, RMAX, N, NT, 0, false>;
-    using AL = CtSt<N, RMAX, N, NT, NST - 1, false>;
-    return A0::NB * A0::R == E && (A0::M * N) % NT == 0 && A0::TOTAL % NT == 0 && AL::NB * AL::R == E &&
-           AL::TOTAL % NT == 0 && N * N == NT * E;
-}
-
-// Strided pass: lines of length N along y (DIM 1, outer index x) or x (DIM 0,
-// outer index y), W contiguous z-columns per tile; grid (outer * M3/W, nf).
-template <typename T, int N, int W, int DIM, int RMAX, int NT, int E, int S1, int S2, class Op>
-__global__ void __launch_bounds__(NT, 2) k_strided_ct(int m2, int m3, const cplx<T>* src, cplx<T>* dst,
-                                                      size_t fstride, const cplx<T>* __restrict__ twn, Op op)
-{
-    using V = cplx<T>;
-    constexpr int NE = N * W;
-    static_assert(NE <= NT * E, "tile does not fit the thread block");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V* tile = reinterpret_cast<V*>(smem_raw);
-    V* stw = tile + NE;
-    const int nzb = m3 / W;
-    const int outer = blockIdx.x / nzb;
-    const int z0 = (blockIdx.x - outer * nzb) * W;
-    const int f = blockIdx.y;
-    const size_t plane = (size_t)m2 * m3;
-    const size_t lstride = DIM == 1 ? (size_t)m3 : plane;
-    const size_t base = (size_t)f * fstride + (DIM == 1 ? (size_t)outer * plane : (size_t)outer * m3) + z0;
-    if (S1 != 0 || S2 != 0)
-        for (int j = threadIdx.x; j < N; j += NT) stw[j] = twn[j];
-    pdl_wait();
-    constexpr int EPT = (NE + NT - 1) / NT;
-    if (S1 != 0) {
-        V v[EPT];
-#pragma unroll
-        for (int u = 0; u < EPT; ++u) {
-            const int e = threadIdx.x + u * NT;
-            if (NE % NT == 0 || e < NE) v[u] = src[base + (e / W) * lstride + e % W];
-        }
-#pragma unroll
-        for (int u = 0; u < EPT; ++u) {
-            const int e = threadIdx.x + u * NT;
-            if (NE % NT == 0 || e < NE) tile[e] = v[u];
-        }
-        __syncthreads();
-        ct_fft<V, S1, N, RMAX, W, W, 1, NT, E>(tile, stw);
-    } else {
-        __syncthreads();
-    }
-    op.begin();
-    constexpr int PB = (sizeof(T) == 4 && NT < 1024) ? 8 : 4;
-#pragma unroll 1
-    for (int u0 = 0; u0 < EPT; u0 += PB) {
-        typename Op::Pre pre[PB];
-#pragma unroll
-        for (int k = 0; k < PB; ++k) {
-            const int e = threadIdx.x + (u0 + k) * NT;
-            if (u0 + k < EPT && (NE % NT == 0 || e < NE)) pre[k] = op.load(f, base + (e / W) * lstride + e % W);
-        }
-#pragma unroll
-        for (int k = 0; k < PB; ++k) {
-            const int e = threadIdx.x + (u0 + k) * NT;
-            if (u0 + k < EPT && (NE % NT == 0 || e < NE)) {
-                const int j = e / W, w = e % W;
-                const int x = DIM == 1 ? outer : j;
-                const int y = DIM == 1 ? j : outer;
-                const size_t off = base + j * lstride + w;
-                V v = S1 != 0 ? tile[e] : mkc<V>(T(0), T(0));
-                v = op.apply(f, x, y, z0 + w, off, v, pre[k]);
-                if (S2 != 0) tile[e] = v;
-            }
-        }
-    }
-    pdl_trigger();
-    if (S2 != 0) {
-        __syncthreads();
-        ct_fft<V, S2, N, RMAX, W, W, 1, NT, E>(tile, stw);
-        for (int e = threadIdx.x; e < NE; e += NT) dst[base + (e / W) * lstride + e % W] = tile[e];
-    }
-    op.end(reinterpret_cast<double*>(tile), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
-}
-
-// Strided pass with both transforms (the bond pass), shared-memory round
-// trips cut to the stages that need them.  The coalesced load of thread
-// tid (positions tid/W + u*NT/W of column tid%W) is the input set of its
-// first-stage butterflies, so stage 0 runs on the loaded registers; the
-// second transform runs in reversed radix order, so the last stage of the
-// first transform, the pointwise op and the first stage of the second stay
-// in registers; the last stage stores its outputs (positions i + t*SPAN of
-// the column) straight to global memory.  For N = 128 (radix 16 x 8) that is
-// two shared-memory round trips instead of six.  Same grid, Op interface and
-// results (up to the rounding of the second transform's radix order) as
-// k_strided_ct.
-template <int N, int W, int RMAX, int NT, int E>
-__host__ __device__ constexpr bool strided_fused_ok()
-{
-    constexpr int NST = ct_nst(N, RMAX);
-    if (NST < 2 || NT % W != 0) return false;
-    using A0 = CtSt<N, RMAX, W, NT, 0, false>;
-    using AL = CtSt<N, RMAX, W, NT, NST - 1, false>;
-    using BL = CtSt<N, RMAX, W, NT, NST - 1, true>;
-    return A0::NB * A0::R == E && (A0::M * W) % NT == 0 && A0::TOTAL % NT == 0 && BL::NB * BL::R == E &&
-           (BL::SPAN * W) % NT == 0 && BL::TOTAL % NT == 0 && AL::NB * AL::R == E && AL::TOTAL % NT == 0 &&
-           N * W == NT * E;
-}
-
-// Source field of output field f of a pencil pass: Op::NSRC entries of
+// Source field of output field f of a k-space pass: Op::NSRC entries of
 // Op::src where the op declares them (an output computed from another
 // field's transform), else f.  The entries are read with constant indices.
 template <class Op, class = void>
@@ -860,282 +651,6 @@ __device__ __forceinline__ int op_src_field(const Op& op, int f)
         return f;
     }
 }
-
-template <typename T, int N, int W, int DIM, int RMAX, int NT, int E, int S1, int S2, class Op>
-__global__ void __launch_bounds__(NT, Op::FUSED_MIN_BLOCKS) k_strided_fused(int m2, int m3, const cplx<T>* src, cplx<T>* dst,
-                                                         size_t fstride, const cplx<T>* __restrict__ twn, Op op)
-{
-    using V = cplx<T>;
-    constexpr int NE = N * W;
-    constexpr int NST = ct_nst(N, RMAX);
-    static_assert(S1 != 0 && S2 != 0, "the fused pass runs both transforms");
-    static_assert(strided_fused_ok<N, W, RMAX, NT, E>(), "tile shape not supported by the fused pass");
-    using A0 = CtSt<N, RMAX, W, NT, 0, false>;          // first stage, first transform
-    using AL = CtSt<N, RMAX, W, NT, NST - 1, false>;    // last stage, first transform
-    using B0 = CtSt<N, RMAX, W, NT, 0, true>;           // first stage, second transform (radix of AL)
-    using BL = CtSt<N, RMAX, W, NT, NST - 1, true>;     // last stage, second transform
-    static_assert(B0::R == AL::R && B0::NB == AL::NB && B0::M == AL::SPAN, "stage mismatch");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V* tile = reinterpret_cast<V*>(smem_raw);
-    V* stw = tile + NE;
-    const int nzb = m3 / W;
-    const int outer = blockIdx.x / nzb;
-    const int z0 = (blockIdx.x - outer * nzb) * W;
-    const int f = blockIdx.y;
-    const size_t plane = (size_t)m2 * m3;
-    const size_t lstride = DIM == 1 ? (size_t)m3 : plane;
-    const size_t inner = (DIM == 1 ? (size_t)outer * plane : (size_t)outer * m3) + z0;
-    const size_t base = (size_t)f * fstride + inner;
-    const size_t sbase = (size_t)op_src_field(op, f) * fstride + inner;
-    for (int j = threadIdx.x; j < N; j += NT) stw[j] = twn[j];
-    pdl_wait();
-    // load: value u of the thread is position tid/W + u*NT/W of column tid%W
-    V v[E];
-#pragma unroll
-    for (int u = 0; u < E; ++u) {
-        const int e = threadIdx.x + u * NT;
-        v[u] = src[sbase + (e / W) * lstride + e % W];
-    }
-    __syncthreads();   // twiddles in shared memory
-    {
-        V a[A0::NB][A0::R];
-#pragma unroll
-        for (int q = 0; q < A0::NB; ++q)
-#pragma unroll
-            for (int t = 0; t < A0::R; ++t) a[q][t] = v[q + t * (A0::M * W / NT)];
-        st_butterfly<S1, A0>(a, stw);
-        st_scatter<A0, W, 1>(tile, a);
-        __syncthreads();
-    }
-    st_range<V, S1, N, RMAX, W, W, 1, NT, false, 1, NST - 1>(tile, stw);
-    op.begin();
-    {
-        V a[AL::NB][AL::R];
-        st_gather<AL, W, 1>(tile, a);
-        typename Op::Pre pre[AL::NB][AL::R];
-#pragma unroll
-        for (int q = 0; q < AL::NB; ++q)
-#pragma unroll
-            for (int t = 0; t < AL::R; ++t)
-                pre[q][t] = op.load(f, base + (size_t)AL::out_pos(q, t) * lstride + AL::line(q));
-        __syncthreads();   // every gather done before the tile is rewritten
-        st_butterfly<S1, AL>(a, stw);
-#pragma unroll
-        for (int q = 0; q < AL::NB; ++q)
-#pragma unroll
-            for (int t = 0; t < AL::R; ++t) {
-                const int j = AL::out_pos(q, t), w = AL::line(q);
-                const int x = DIM == 1 ? outer : j;
-                const int y = DIM == 1 ? j : outer;
-                a[q][t] = op.apply(f, x, y, z0 + w, base + (size_t)j * lstride + w, a[q][t], pre[q][t]);
-            }
-        pdl_trigger();
-        st_butterfly<S2, B0>(a, stw);
-        st_scatter<B0, W, 1>(tile, a);
-        __syncthreads();
-    }
-    st_range<V, S2, N, RMAX, W, W, 1, NT, true, 1, NST - 1>(tile, stw);
-    {
-        V a[BL::NB][BL::R];
-        st_gather<BL, W, 1>(tile, a);
-        st_butterfly<S2, BL>(a, stw);
-#pragma unroll
-        for (int q = 0; q < BL::NB; ++q)
-#pragma unroll
-            for (int t = 0; t < BL::R; ++t)
-                dst[base + (size_t)BL::out_pos(q, t) * lstride + BL::line(q)] = a[q][t];
-    }
-    op.end(reinterpret_cast<double*>(tile), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
-}
-
-// Strided pass with one transform after the op (S1 = 0: the field loads of
-// the batched 3-D transforms).  The op's values for the loaded positions
-// (tid/W + u*NT/W of column tid%W) are the first-stage inputs, so stage 0
-// runs on registers, and the last stage stores straight to global memory.
-template <typename T, int N, int W, int DIM, int RMAX, int NT, int E, int S2, class Op>
-__global__ void __launch_bounds__(NT, 2) k_strided_load_fused(int m2, int m3, cplx<T>* dst, size_t fstride,
-                                                              const cplx<T>* __restrict__ twn, Op op)
-{
-    using V = cplx<T>;
-    constexpr int NE = N * W;
-    constexpr int NST = ct_nst(N, RMAX);
-    static_assert(S2 != 0, "one transform");
-    static_assert(strided_fused_ok<N, W, RMAX, NT, E>(), "tile shape not supported by the fused pass");
-    using A0 = CtSt<N, RMAX, W, NT, 0, false>;
-    using AL = CtSt<N, RMAX, W, NT, NST - 1, false>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V* tile = reinterpret_cast<V*>(smem_raw);
-    V* stw = tile + NE;
-    const int nzb = m3 / W;
-    const int outer = blockIdx.x / nzb;
-    const int z0 = (blockIdx.x - outer * nzb) * W;
-    const int f = blockIdx.y;
-    const size_t plane = (size_t)m2 * m3;
-    const size_t lstride = DIM == 1 ? (size_t)m3 : plane;
-    const size_t base = (size_t)f * fstride + (DIM == 1 ? (size_t)outer * plane : (size_t)outer * m3) + z0;
-    for (int j = threadIdx.x; j < N; j += NT) stw[j] = twn[j];
-    pdl_wait();
-    op.begin();
-    V v[E];
-    {
-        typename Op::Pre pre[E];
-#pragma unroll
-        for (int u = 0; u < E; ++u) {
-            const int e = threadIdx.x + u * NT;
-            pre[u] = op.load(f, base + (e / W) * lstride + e % W);
-        }
-#pragma unroll
-        for (int u = 0; u < E; ++u) {
-            const int e = threadIdx.x + u * NT;
-            const int j = e / W, w = e % W;
-            const int x = DIM == 1 ? outer : j;
-            const int y = DIM == 1 ? j : outer;
-            v[u] = op.apply(f, x, y, z0 + w, base + j * lstride + w, mkc<V>(T(0), T(0)), pre[u]);
-        }
-    }
-    pdl_trigger();
-    __syncthreads();   // twiddles in shared memory
-    {
-        V a[A0::NB][A0::R];
-#pragma unroll
-        for (int q = 0; q < A0::NB; ++q)
-#pragma unroll
-            for (int t = 0; t < A0::R; ++t) a[q][t] = v[q + t * (A0::M * W / NT)];
-        st_butterfly<S2, A0>(a, stw);
-        st_scatter<A0, W, 1>(tile, a);
-        __syncthreads();
-    }
-    st_range<V, S2, N, RMAX, W, W, 1, NT, false, 1, NST - 1>(tile, stw);
-    {
-        V a[AL::NB][AL::R];
-        st_gather<AL, W, 1>(tile, a);
-        st_butterfly<S2, AL>(a, stw);
-#pragma unroll
-        for (int q = 0; q < AL::NB; ++q)
-#pragma unroll
-            for (int t = 0; t < AL::R; ++t)
-                dst[base + (size_t)AL::out_pos(q, t) * lstride + AL::line(q)] = a[q][t];
-    }
-    op.end(reinterpret_cast<double*>(tile), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
-}
-
-// Plane pass with one transform after the op (S1 = 0): the op's values for
-// the loaded positions (rows tid/N + u*NT/N of column tid%N) are the inputs
-// of the first radix stage along y, which runs on registers; then the rest
-// of y, then z, then the plane is stored from shared memory.
-template <typename T, int N, int RMAX, int NT, int E, int S2, class Op>
-__global__ void __launch_bounds__(NT, 1) k_plane_load_fused(cplx<T>* dst, size_t fstride,
-                                                            const cplx<T>* __restrict__ twn, Op op)
-{
-    using V = cplx<T>;
-    constexpr int P = N + 1, NE = N * N;
-    constexpr int NST = ct_nst(N, RMAX);
-    static_assert(S2 != 0, "one transform");
-    static_assert(plane_fused_ok<N, RMAX, NT, E>(), "plane shape not supported by the fused pass");
-    using A0 = CtSt<N, RMAX, N, NT, 0, false>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V* tile = reinterpret_cast<V*>(smem_raw);
-    V* stw = tile + N * P;
-    const int x = blockIdx.x;
-    const int f = blockIdx.y;
-    const size_t base = (size_t)f * fstride + (size_t)x * NE;
-    for (int j = threadIdx.x; j < N; j += NT) stw[j] = twn[j];
-    pdl_wait();
-    op.begin();
-    V v[E];
-    {
-        typename Op::Pre pre[E];
-#pragma unroll
-        for (int u = 0; u < E; ++u) pre[u] = op.load(f, base + threadIdx.x + u * NT);
-#pragma unroll
-        for (int u = 0; u < E; ++u) {
-            const int e = threadIdx.x + u * NT;
-            v[u] = op.apply(f, x, e / N, e % N, base + e, mkc<V>(T(0), T(0)), pre[u]);
-        }
-    }
-    pdl_trigger();
-    __syncthreads();   // twiddles in shared memory
-    {
-        V a[A0::NB][A0::R];
-#pragma unroll
-        for (int q = 0; q < A0::NB; ++q)
-#pragma unroll
-            for (int t = 0; t < A0::R; ++t) a[q][t] = v[q + t * (A0::M * N / NT)];
-        st_butterfly<S2, A0>(a, stw);
-        st_scatter<A0, P, 1>(tile, a);
-        __syncthreads();
-    }
-    st_range<V, S2, N, RMAX, N, P, 1, NT, false, 1, NST>(tile, stw);   // rest of y
-    ct_fft<V, S2, N, RMAX, N, 1, P, NT, E>(tile, stw);                  // z-lines
-    for (int e = threadIdx.x; e < NE; e += NT) dst[base + e] = tile[(e / N) * P + e % N];
-    op.end(reinterpret_cast<double*>(tile), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
-}
-
-// z-line pass: BR rows of length N per CTA; grid (m1*m2/BR, nf).
-template <typename T, int N, int BR, int RMAX, int NT, int E, int S1, int S2, class Op>
-__global__ void __launch_bounds__(NT, 2) k_zline_ct(int m2, const cplx<T>* src, cplx<T>* dst, size_t fstride,
-                                                    const cplx<T>* __restrict__ twn, Op op)
-{
-    using V = cplx<T>;
-    constexpr int P = N + 1, NE = BR * N;
-    static_assert(NE <= NT * E, "tile does not fit the thread block");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V* tile = reinterpret_cast<V*>(smem_raw);
-    V* stw = tile + BR * P;
-    const int f = blockIdx.y;
-    const int row0 = blockIdx.x * BR;
-    const size_t base = (size_t)f * fstride + (size_t)row0 * N;
-    if (S1 != 0 || S2 != 0)
-        for (int j = threadIdx.x; j < N; j += NT) stw[j] = twn[j];
-    constexpr int EPT = (NE + NT - 1) / NT;
-    if (S1 != 0) {
-        V v[EPT];
-#pragma unroll
-        for (int u = 0; u < EPT; ++u) {
-            const int e = threadIdx.x + u * NT;
-            if (NE % NT == 0 || e < NE) v[u] = src[base + e];
-        }
-#pragma unroll
-        for (int u = 0; u < EPT; ++u) {
-            const int e = threadIdx.x + u * NT;
-            if (NE % NT == 0 || e < NE) tile[(e / N) * P + e % N] = v[u];
-        }
-        __syncthreads();
-        ct_fft<V, S1, N, RMAX, BR, 1, P, NT, E>(tile, stw);
-    } else {
-        __syncthreads();
-    }
-    op.begin();
-    constexpr int PB = (sizeof(T) == 4 && NT < 1024) ? 8 : 4;
-#pragma unroll 1
-    for (int u0 = 0; u0 < EPT; u0 += PB) {
-        typename Op::Pre pre[PB];
-#pragma unroll
-        for (int k = 0; k < PB; ++k) {
-            const int e = threadIdx.x + (u0 + k) * NT;
-            if (u0 + k < EPT && (NE % NT == 0 || e < NE)) pre[k] = op.load(f, base + e);
-        }
-#pragma unroll
-        for (int k = 0; k < PB; ++k) {
-            const int e = threadIdx.x + (u0 + k) * NT;
-            if (u0 + k < EPT && (NE % NT == 0 || e < NE)) {
-                const int b = e / N, z = e % N;
-                const int row = row0 + b;
-                const int x = row / m2, y = row - x * m2;
-                V v = S1 != 0 ? tile[b * P + z] : mkc<V>(T(0), T(0));
-                v = op.apply(f, x, y, z, base + e, v, pre[k]);
-                if (S2 != 0) tile[b * P + z] = v;
-            }
-        }
-    }
-    if (S2 != 0) {
-        __syncthreads();
-        ct_fft<V, S2, N, RMAX, BR, 1, P, NT, E>(tile, stw);
-        for (int e = threadIdx.x; e < NE; e += NT) dst[base + e] = tile[(e / N) * P + e % N];
-    }
-    op.end(reinterpret_cast<double*>(tile), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
-}
-
 
 // Global loads per point of a pointwise op (Op::LOADS where declared, else 4).
 template <class Op, class = void>

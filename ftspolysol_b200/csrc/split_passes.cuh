@@ -51,7 +51,7 @@
 namespace ftsp {
 
 constexpr int SPLIT_NT = 512;   // largest block
-constexpr int SPLIT_RADICES[] = {1, 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 25};
+constexpr int SPLIT_RADICES[] = {1, 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 24, 25, 32};
 
 struct SplitGeom {
     int m1, m2, m3;
@@ -154,7 +154,7 @@ constexpr bool split_tiles(SplitGeom& g, int value_bytes, int G, int W)
     g.W = W;
     g.C = g.Y2 * g.W;
     g.k_threads = split_round32(split_max(g.C * g.xA, m1 * g.W));
-    if (g.k_threads > SPLIT_NT) g.k_threads = SPLIT_NT;
+    if (g.k_threads > (g.big ? 256 : SPLIT_NT)) g.k_threads = g.big ? 256 : SPLIT_NT;
     // both buffers of both passes within the shared memory of a block
     if ((2LL * g.rt + 2 * m3 + g.rows) * value_bytes > 225 * 1024 || (2LL * m1 * (g.C + banks) + 2 * m1) * value_bytes > 225 * 1024)
         return false;
@@ -182,7 +182,7 @@ constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes
     // beside its values: 10 at most, except in RtBigPlan
     if (!split_pair(m3, 16, 10, g.zA, g.zB) || !split_pair(m1, 16, 10, g.xA, g.xB) || !split_pair(m2, 16, 16, g.Y1, g.Y2)) {
         g.big = 1;
-        if (!split_pair(m3, 25, 16, g.zA, g.zB) || !split_pair(m1, 25, 16, g.xA, g.xB) || !split_pair(m2, 25, 16, g.Y1, g.Y2))
+        if (!split_pair(m3, 32, 16, g.zA, g.zB) || !split_pair(m1, 32, 16, g.xA, g.xB) || !split_pair(m2, 32, 16, g.Y1, g.Y2))
             return false;
         if (g.Y1 > 16) {   // the long half of y in the pass whose tiles are narrower
             const int t = g.Y1;
@@ -214,10 +214,12 @@ struct RtPlan {
     // blocks per SM asked of the compiler, real space and k space
     template <typename T> static constexpr int rmin = sizeof(T) == 4 ? 3 : 2;
 };
-// The same for lengths that need radix 25 (125 = 25 x 5) or two large radices
-// (192 = 16 x 12): its own kernels, so that the others keep their registers.
+// The same for lengths that need a radix of 18 to 32 (125 = 25 x 5, 320 = 20 x
+// 16) or two large radices (192 = 16 x 12): its own kernels, so that the others
+// keep their registers.
 struct RtBigPlan : RtPlan {
-    static constexpr int AMAX = 25, BMAX = 16;
+    static constexpr int KNT = 256;
+    static constexpr int AMAX = 32, BMAX = 16;
     template <typename T> static constexpr int rmin = 1;
 };
 // A cube of N points a side at compile time.  One buffer: a phase reads,
@@ -287,35 +289,6 @@ inline size_t split_k_smem(const SplitGeom& g)
 }
 
 // ---- device ----
-// Composite butterflies.  Coprime factors need no twiddles: with inputs
-// n = (Q n1 + P n2) mod PQ and outputs k = k1 mod P, k2 mod Q (the prime-factor
-// algorithm), the transform is P-point DFTs over n1 and Q-point ones over n2.
-template <int S, int P, int Q, typename V>
-__device__ __forceinline__ void dft_coprime(V* u)
-{
-    constexpr int N = P * Q;
-    V a[N];
-#pragma unroll
-    for (int n2 = 0; n2 < Q; ++n2) {
-        V b[P];
-#pragma unroll
-        for (int n1 = 0; n1 < P; ++n1) b[n1] = u[(Q * n1 + P * n2) % N];
-        dftR<S, P>(b);
-#pragma unroll
-        for (int k1 = 0; k1 < P; ++k1) a[k1 * Q + n2] = b[k1];
-    }
-#pragma unroll
-    for (int k1 = 0; k1 < P; ++k1) {
-        V b[Q];
-#pragma unroll
-        for (int n2 = 0; n2 < Q; ++n2) b[n2] = a[k1 * Q + n2];
-        dftR<S, Q>(b);
-#pragma unroll
-        for (int k = 0; k < N; ++k)
-            if (k % P == k1) u[k] = b[k % Q];
-    }
-}
-
 // 9 = 3 x 3 with the twiddles w9, w9^2, w9^4
 template <int S, typename V>
 __device__ __forceinline__ void dft9(V* u)
@@ -343,6 +316,42 @@ __device__ __forceinline__ void dft9(V* u)
         u[k] = b[0];
         u[k + 3] = b[1];
         u[k + 6] = b[2];
+    }
+}
+
+template <int S, int R, typename V>
+__device__ __forceinline__ void dft_factor(V* u)
+{
+    if constexpr (R == 9) dft9<S>(u);
+    else dftR<S, R>(u);
+}
+
+// Composite butterflies.  Coprime factors need no twiddles: with inputs
+// n = (Q n1 + P n2) mod PQ and outputs k = k1 mod P, k2 mod Q (the prime-factor
+// algorithm), the transform is P-point DFTs over n1 and Q-point ones over n2.
+template <int S, int P, int Q, typename V>
+__device__ __forceinline__ void dft_coprime(V* u)
+{
+    constexpr int N = P * Q;
+    V a[N];
+#pragma unroll
+    for (int n2 = 0; n2 < Q; ++n2) {
+        V b[P];
+#pragma unroll
+        for (int n1 = 0; n1 < P; ++n1) b[n1] = u[(Q * n1 + P * n2) % N];
+        dft_factor<S, P>(b);
+#pragma unroll
+        for (int k1 = 0; k1 < P; ++k1) a[k1 * Q + n2] = b[k1];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < P; ++k1) {
+        V b[Q];
+#pragma unroll
+        for (int n2 = 0; n2 < Q; ++n2) b[n2] = a[k1 * Q + n2];
+        dft_factor<S, Q>(b);
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            if (k % P == k1) u[k] = b[k % Q];
     }
 }
 
@@ -432,6 +441,9 @@ __device__ __forceinline__ void dft_any(V* u)
     else if constexpr (R == 10) dft_coprime<S, 2, 5>(u);
     else if constexpr (R == 12) dft_coprime<S, 4, 3>(u);
     else if constexpr (R == 15) dft_coprime<S, 3, 5>(u);
+    else if constexpr (R == 18) dft_coprime<S, 2, 9>(u);
+    else if constexpr (R == 20) dft_coprime<S, 4, 5>(u);
+    else if constexpr (R == 24) dft_coprime<S, 8, 3>(u);
     else if constexpr (R == 25) dft25<S>(u);
     else if constexpr (R == 32) dft32<S>(u);
     else dftR<S, R>(u);
@@ -466,7 +478,11 @@ __device__ __forceinline__ void by_radix(int r, F&& f)
                 else if (r == 16) f(RadixTag<16>{});
             }
             if constexpr (MAX > 16) {
-                if (r == 25) f(RadixTag<25>{});
+                if (r == 18) f(RadixTag<18>{});
+                else if (r == 20) f(RadixTag<20>{});
+                else if (r == 24) f(RadixTag<24>{});
+                else if (r == 25) f(RadixTag<25>{});
+                else if (r == 32) f(RadixTag<32>{});
             }
             break;
         }

@@ -20,7 +20,7 @@ pytestmark = pytest.mark.gpu
 
 CHAINS = [(2, 3, 5), (1, 4, 1), (8, 9, 10), (12, 15, 16), (18, 20, 27), (25, 30, 45), (81, 6, 75), (90, 40, 36),
           (125, 6, 8), (8, 125, 6), (6, 8, 125), (25, 125, 20), (150, 10, 12), (12, 144, 10), (10, 12, 160), (192, 6, 5),
-          (4, 256, 9), (5, 6, 225), (200, 9, 4), (162, 4, 6), (32, 32, 32), (48, 48, 48), (64, 64, 64), (96, 96, 96), (128, 128, 128)]
+          (4, 256, 9), (5, 6, 225), (200, 9, 4), (162, 4, 6), (6, 200, 5), (320, 8, 3), (4, 10, 384), (16, 12, 512), (243, 4, 6), (32, 32, 32), (48, 48, 48), (64, 64, 64), (96, 96, 96), (128, 128, 128)]
 
 
 def reference_chain(w, L, N, b):

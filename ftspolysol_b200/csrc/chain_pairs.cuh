@@ -278,8 +278,7 @@ __global__ void __launch_bounds__(256) k_pair_density_vec(size_t n, PairTable tb
 
 // partial[cta][c] += factor sum_k k_a k_b Phi(k) sum_pairs scale t(k), the
 // six components (xx, yy, zz, xy, xz, yz) in the layout of the backward
-// bond pass, so the same fixed-order combine reads them.  Launched with as
-// many CTAs as that pass has.
+// bond pass, so the same fixed-order combine reads them.
 template <typename T>
 __global__ void __launch_bounds__(256) k_pair_stress(int m1, int m2, int m3, PairTable tb,
                                                      const cplx<T>* __restrict__ F, const T* __restrict__ phi,
@@ -300,7 +299,9 @@ __global__ void __launch_bounds__(256) k_pair_stress(int m1, int m2, int m3, Pai
 #pragma unroll
     for (int c = 0; c < 12; ++c) acc[c] = 0.0;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    // the lower index of every pair has x <= m1 / 2
+    const size_t half = (size_t)(m1 / 2 + 1) * m2 * m3;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < half; i += stride) {
         const int z = (int)(i % m3);
         const size_t rest = i / m3;
         const int y = (int)(rest % m2), x = (int)(rest / m2);
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(256) k_pair_stress(int m1, int m2, int m3, Pai
             const double p0 = (double)(ph[x] * ph[m1 + y] * ph[m1 + m2 + z]);
             const double p1 = (double)(ph[nx] * ph[m1 + ny] * ph[m1 + m2 + nz]);
             double tx = 0.0, ty = 0.0;
-#pragma unroll 2
+#pragma unroll 4
             for (int j = R.j0; j < R.j1; ++j) {
                 const int2 pr = sp[j];
                 const V* Fb = F + (size_t)pr.x * n;

@@ -487,14 +487,21 @@ struct OpPrecond {
     SigTab st;               // dt lambda_f per field
     T invV;
     int dc0 = -1;            // field whose k = 0 value is set to zero (psi: its mean removal), -1: none
-    static constexpr int LOADS = 0;
-    struct Pre {};
-    __device__ __forceinline__ void begin() {}
-    __device__ __forceinline__ Pre load(int, size_t) const { return Pre{}; }
-    __device__ __forceinline__ cplx<T> apply(int f, int x, int y, int z, size_t g, cplx<T> v, const Pre&) const
+    double dts;              // read once per thread (begin)
+    bool learned;
+    static constexpr int LOADS = 1;
+    struct Pre {
+        T G;
+    };
+    __device__ __forceinline__ void begin()
     {
-        const T G = (GL && d->lr_use) ? GL[g] : GA[g];
-        const cplx<T> k = cscale(v, (T)(1.0 / (1.0 + (pick(st.s, f) * d->dt_scale) * (double)G)));
+        dts = d->dt_scale;
+        learned = GL && d->lr_use;
+    }
+    __device__ __forceinline__ Pre load(int, size_t g) const { return Pre{learned ? GL[g] : GA[g]}; }
+    __device__ __forceinline__ cplx<T> apply(int f, int x, int y, int z, size_t g, cplx<T> v, const Pre& p) const
+    {
+        const cplx<T> k = cscale(v, (T)(1.0 / (1.0 + (pick(st.s, f) * dts) * (double)p.G)));
         if (dw) dw[g] = k;
         if (f == dc0 && (x | y | z) == 0) return mkc<cplx<T>>(T(0), T(0));
         return cscale(k, invV);
@@ -526,6 +533,33 @@ struct OpKScale {
     struct Pre {};
     __device__ __forceinline__ void begin() {}
     __device__ __forceinline__ Pre load(int, size_t) const { return Pre{}; }
+    // x factors staged by the kernel, the factors of a column read once (see OpBond)
+    struct XVal {
+        double k2;
+        T g;
+    };
+    struct Column {
+        double k2, cx, cy;
+        T g;
+        bool lap;
+    };
+    __device__ __forceinline__ XVal x_value(int x) const
+    {
+        const double ax = __ldg(kx + x);
+        return XVal{ax * ax, __ldg(gm + x)};
+    }
+    __device__ __forceinline__ Column column(int f, int y, int z) const
+    {
+        const double ay = __ldg(ky + y), az = __ldg(kz + z);
+        const double2 cf = pick(c, f);
+        return Column{ay * ay + az * az, cf.x, cf.y, __ldg(gm + m1 + y) * __ldg(gm + m1 + m2 + z), pick(lap, f) != 0};
+    }
+    __device__ __forceinline__ V apply_x(int f, int, int, int, size_t g, V v, const Pre&, XVal x, const Column& col) const
+    {
+        if (f < nst) kst[g] = v;
+        const double fac = col.lap ? x.k2 + col.k2 : (double)(x.g * col.g);
+        return from_d<V>(dscale(dmul(to_d(v), make_double2(col.cx, col.cy)), fac));
+    }
     __device__ __forceinline__ V apply(int f, int x, int y, int z, size_t g, V v, const Pre&) const
     {
         if (f < nst) kst[g] = v;
@@ -593,6 +627,8 @@ struct OpIncrement {
     bool elec;
     double* dpart;           // corrector: per-CTA drift maxima
     double dmax;
+    double dts, me;          // step scalars, read once per thread (begin)
+    double2 md;
     // the raw operands of a point; the loads carry no side effect, so a
     // kernel keeps a whole batch of them in flight, and apply() does the
     // arithmetic and the write-backs
@@ -600,7 +636,13 @@ struct OpIncrement {
         V a, b;              // modes: u, u_bar; psi: psi drift, psi drift at the predictor
         T e;
     };
-    __device__ __forceinline__ void begin() { dmax = 0.0; }
+    __device__ __forceinline__ void begin()
+    {
+        dmax = 0.0;
+        dts = d->dt_scale;
+        me = CORR ? 0.0 : -(d->mean_eta * invV);
+        md = dscale(d->mean_dpsi, -invV);
+    }
     __device__ __forceinline__ Pre load(int f, size_t g) const
     {
         const size_t i = g - (size_t)f * Vn;
@@ -628,7 +670,7 @@ struct OpIncrement {
                 if (!isfinite(m)) m = INFINITY;
                 dmax = fmax(dmax, m);
             }
-            V v = cscale(s, (T)(pick(cs.s, f) * d->dt_scale));
+            V v = cscale(s, (T)(pick(cs.s, f) * dts));
             v.x += p.e;
             return v;
         }
@@ -640,19 +682,19 @@ struct OpIncrement {
         // and the caller read them
         V s;
         if (!CORR) {
-            ep = (T)((double)ep + (-(d->mean_eta * invV)));
+            ep = (T)((double)ep + me);
             e[(size_t)nm * Vn + i] = ep;
-            s = cadd(p.a, from_d<V>(dscale(d->mean_dpsi, -invV)));
+            s = cadd(p.a, from_d<V>(md));
             dp[i] = s;
         } else {
-            const V dbv = cadd(p.b, from_d<V>(dscale(d->mean_dpsi, -invV)));
+            const V dbv = cadd(p.b, from_d<V>(md));
             db[i] = dbv;
             s = cadd(p.a, dbv);
             double m = (double)s.x * s.x + (double)s.y * s.y;
             if (!isfinite(m)) m = INFINITY;
             dmax = fmax(dmax, m);
         }
-        V v = cscale(s, (T)(pick(cs.s, nm) * d->dt_scale));
+        V v = cscale(s, (T)(pick(cs.s, nm) * dts));
         v.x += ep;
         return v;
     }
@@ -2296,10 +2338,15 @@ struct Engine : EngineBase {
         if (plane_ok) return c.m1;
         return c.m1 * c.m2 / gz.B;
     }
-    // blocks that write connectivity-stress partials: the pair kernel's (x_ctas)
-    // and, with the split passes, the backward bond pass's
-    int stress_parts() const { return std::max(x_ctas(), use_split ? sg.Y1 * sg.nzb : 0); }
-    int x_ctas() const { return c.m2 * (c.m3 / gx.W); }
+    // blocks that write connectivity-stress partials: the pair kernel's and the
+    // backward bond pass's
+    int stress_parts() const { return std::max(pair_blocks(), use_split ? sg.Y1 * sg.nzb : c.m2 * (c.m3 / gx.W)); }
+    // blocks of the pair-stress kernel: a thread per pair {k, -k} up to eight
+    // blocks per SM (128^3 complex64: 1024-1184 blocks 221 us, 512 blocks 424)
+    int pair_blocks() const
+    {
+        return (int)std::max<size_t>(1, std::min<size_t>({(V_ / 2 + 255) / 256, (size_t)RED_BLOCKS, (size_t)c.m2 * c.m3}));
+    }
 
     template <int S1, int S2, bool FWD, bool STRESS>
     void bond_pass(const V* src, V* dst, const OpBond<T, FWD, STRESS>& op)
@@ -2480,7 +2527,7 @@ struct Engine : EngineBase {
                 }
                 FTSP_CUDA(cudaEventRecord(ev_fork, stream));
                 FTSP_CUDA(cudaStreamWaitEvent(aux, ev_fork, 0));
-                k_pair_stress<T><<<x_ctas(), threads, sm, aux>>>(
+                k_pair_stress<T><<<pair_blocks(), threads, sm, aux>>>(
                     c.m1, c.m2, c.m3, t.stress, (const V*)Fst.p, (const T*)phi.p, (const double*)kx.p,
                     (const double*)ky.p, (const double*)kz.p, (const int*)expo.p, s.N, factor,
                     reinterpret_cast<double2*>(spart.p));
@@ -2488,7 +2535,7 @@ struct Engine : EngineBase {
                 aux_pending = true;
             } else {
                 cudaEvent_t ev = prof_begin();
-                launch_pass(k_pair_stress<T>, dim3(x_ctas()), threads, sm, c.m1, c.m2, c.m3, t.stress,
+                launch_pass(k_pair_stress<T>, dim3(pair_blocks()), threads, sm, c.m1, c.m2, c.m3, t.stress,
                             (const V*)Fst.p, (const T*)phi.p, (const double*)kx.p, (const double*)ky.p,
                             (const double*)kz.p, (const int*)expo.p, s.N, factor, reinterpret_cast<double2*>(spart.p));
                 prof_end(ev, "pair_stress", (double)(s.N - 1) * sizeof(V) * (double)Vn);
@@ -3644,7 +3691,7 @@ struct Engine : EngineBase {
 
     // n device values to host memory as FP64 pairs: converted on the device
     // (complex64: through the sweeps' scratch field, half a field at a time)
-    // and copied straight to the caller.  Above 16 MiB the caller's pages are
+    // and copied straight to the caller.  Above 4 MiB the caller's pages are
     // touched by a few threads first: memory of that size comes fresh from
     // the system, and its first touch costs more than the copy.  Measured,
     // complex64 into fresh memory: 128^3 18 ms (copy, then a host loop) -> 6,
@@ -3653,7 +3700,7 @@ struct Engine : EngineBase {
     void copy_out(const V* p, size_t n, double* out)
     {
         const size_t bytes = n * sizeof(double2);
-        if (bytes >= ((size_t)16 << 20)) {
+        if (bytes >= ((size_t)4 << 20)) {
             const size_t pages = bytes / 4096;
             auto touch = [out](size_t a, size_t b) {
                 for (size_t i = a; i < b; ++i) *reinterpret_cast<volatile double*>(out + i * 512) = 0.0;

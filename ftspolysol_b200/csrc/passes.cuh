@@ -575,18 +575,20 @@ struct OpBond {
         if (!FWD && STRESS) p.F = Fread[g];
         return p;
     }
-    // For kernels that stage the x factors themselves (x_table, in shared
+    // For kernels that stage the x factors themselves (x_value, in shared
     // memory): column() gives the factor of a thread's column, once, and
     // apply_x() is apply() with the x factor and the column factor given.
-    __device__ __forceinline__ const T* x_table() const { return phix; }
-    __device__ __forceinline__ T column(int y, int z) const { return __ldg(phiy + y) * __ldg(phiz + z); }
-    __device__ __forceinline__ V apply(int, int x, int y, int z, size_t g, V v, const Pre& pre)
+    using XVal = T;
+    using Column = T;
+    __device__ __forceinline__ T x_value(int x) const { return phix[x]; }
+    __device__ __forceinline__ T column(int, int y, int z) const { return __ldg(phiy + y) * __ldg(phiz + z); }
+    __device__ __forceinline__ V apply(int f, int x, int y, int z, size_t g, V v, const Pre& pre)
     {
         // read-only loads: they do not alias the Fstore writes, so the y and z
         // factors (fixed for a thread's column) are loaded once
-        return apply_x(x, y, z, g, v, pre, __ldg(phix + x), column(y, z));
+        return apply_x(f, x, y, z, g, v, pre, __ldg(phix + x), column(f, y, z));
     }
-    __device__ __forceinline__ V apply_x(int x, int y, int z, size_t g, V v, const Pre& pre, T px, T pyz)
+    __device__ __forceinline__ V apply_x(int, int x, int y, int z, size_t g, V v, const Pre& pre, T px, T pyz)
     {
         const T phi = px * pyz;
         if (FWD) {
@@ -662,11 +664,21 @@ struct op_loads<Op, std::void_t<decltype(Op::LOADS)>> {
     static constexpr int value = Op::LOADS;
 };
 
-// ops with x_table(), column() and apply_x()
+// ops with x_value(), column() and apply_x()
 template <class Op, class = void>
 struct op_has_xtab : std::false_type {};
 template <class Op>
-struct op_has_xtab<Op, std::void_t<decltype(&Op::x_table)>> : std::true_type {};
+struct op_has_xtab<Op, std::void_t<typename Op::XVal>> : std::true_type {};
+template <class Op, bool = op_has_xtab<Op>::value>
+struct op_xval {
+    using type = char;
+    using column = char;
+};
+template <class Op>
+struct op_xval<Op, true> {
+    using type = typename Op::XVal;
+    using column = typename Op::Column;
+};
 
 // op.preload() where the op declares it
 template <class Op>

@@ -56,7 +56,7 @@ constexpr int SPLIT_RADICES[] = {1, 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20,
 struct SplitGeom {
     int m1, m2, m3;
     int ok;                  // the extents factor (see split_setup)
-    int big;                 // with radices that need RtBigPlan
+    int big_r, big_k;        // passes with radices that need RtBigPlan
     int cube;                // side of the CubePlan to run, 0: a run-time plan
     int Y1, Y2;
     // real-space pass: m3 = zA * zB, G row groups (y0 .. y0 + G - 1) per block
@@ -154,7 +154,7 @@ constexpr bool split_tiles(SplitGeom& g, int value_bytes, int G, int W)
     g.W = W;
     g.C = g.Y2 * g.W;
     g.k_threads = split_round32(split_max(g.C * g.xA, m1 * g.W));
-    if (g.k_threads > (g.big ? 256 : SPLIT_NT)) g.k_threads = g.big ? 256 : SPLIT_NT;
+    if (g.k_threads > SPLIT_NT) g.k_threads = SPLIT_NT;
     // both buffers of both passes within the shared memory of a block
     if ((2LL * g.rt + 2 * m3 + g.rows) * value_bytes > 225 * 1024 || (2LL * m1 * (g.C + banks) + 2 * m1) * value_bytes > 225 * 1024)
         return false;
@@ -177,11 +177,9 @@ constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes
 {
     g.m1 = m1; g.m2 = m2; g.m3 = m3;
     g.ok = 0;
-    g.big = 0;
     // the butterfly pair around the op (radix B) holds the op's operands
     // beside its values: 10 at most, except in RtBigPlan
     if (!split_pair(m3, 16, 10, g.zA, g.zB) || !split_pair(m1, 16, 10, g.xA, g.xB) || !split_pair(m2, 16, 16, g.Y1, g.Y2)) {
-        g.big = 1;
         if (!split_pair(m3, 32, 16, g.zA, g.zB) || !split_pair(m1, 32, 16, g.xA, g.xB) || !split_pair(m2, 32, 16, g.Y1, g.Y2))
             return false;
         if (g.Y1 > 16) {   // the long half of y in the pass whose tiles are narrower
@@ -197,6 +195,8 @@ constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes
     // k space: 32 bytes of every row (one memory sector)
     int W = split_max(1, 32 / value_bytes);
     while (W > 1 && (W / 2 >= m3 || (long long)m1 * g.Y2 * W * value_bytes > 72 * 1024)) W /= 2;
+    g.big_r = g.zA > 16 || g.zB > 10 || g.Y1 > 16;
+    g.big_k = g.xA > 16 || g.xB > 10 || g.Y2 > 16;
     g.cube = m1 == m2 && m2 == m3 && (m1 == 32 || m1 == 48 || m1 == 64 || m1 == 96 || m1 == 128) ? m1 : 0;
     g.ok = split_tiles(g, value_bytes, G, W) ? 1 : 0;
     return g.ok != 0;
@@ -218,7 +218,6 @@ struct RtPlan {
 // 16) or two large radices (192 = 16 x 12): its own kernels, so that the others
 // keep their registers.
 struct RtBigPlan : RtPlan {
-    static constexpr int KNT = 256;
     static constexpr int AMAX = 32, BMAX = 16;
     template <typename T> static constexpr int rmin = 1;
 };
@@ -538,18 +537,25 @@ __device__ __forceinline__ void split_phase(int items, Ga gather, Fi finish)
 // quotient by a geometry member with its magic-number divisor
 #define FTSP_DIV(i, m, f) (P::CT ? (int)((unsigned)(i) / (unsigned)split_max(1, P::G.m)) : (int)fdiv(i, g.f))
 
-// registers a thread is given: complex64 ops with one operand per point fit
-// 72 (7 blocks of 128 threads: 128^3 runs in one wave of 1024 blocks); wider
-// ops and complex128 take up to 128
+// registers a thread is given: at 128^3 complex64 ops with one operand per
+// point fit 72 (7 blocks of 128 threads: 1024 blocks in one wave; 20.4 us per
+// segment with its bond pass, 21.0 with 128 registers), and 64^3 steps are
+// faster with it too (22.4 against 24.1 ms per 20 steps); on the mixed-radix
+// cubes and at 32^3, 128 registers keep more loads in flight (96^3 17.4 -> 16.5
+// us per segment with its share of the pair densities, 48^3 6.2 -> 5.8, 32^3
+// 5.1 -> 4.9)
 template <typename T, class Op>
-constexpr int split_regs()
+constexpr int split_regs(int n)
 {
-    return sizeof(T) == 4 ? (op_loads<Op>::value == 0 ? 64 : op_loads<Op>::value == 1 ? 72 : 96) : 128;
+    return sizeof(T) == 4 && (n == 128 || n == 64) ? (op_loads<Op>::value == 0 ? 64 : op_loads<Op>::value == 1 ? 72 : 96) : 128;
 }
 template <class P, typename T, class Op>
 constexpr int split_min_blocks(int nt)
 {
-    return P::CT ? split_max(1, 65536 / (nt * split_regs<T, Op>())) : nt <= 256 ? P::template rmin<T> : 1;
+    // small complex128 cubes never fill an SM: no cap (32^3: 4.9 us per segment
+    // in the step graph, 5.4 capped at 128)
+    if (P::CT && sizeof(T) == 8 && P::G.m1 <= 64) return 1;
+    return P::CT ? split_max(1, 65536 / (nt * split_regs<T, Op>(P::G.m1))) : nt <= 256 ? P::template rmin<T> : 1;
 }
 
 // Real-space pass: grid (m1 * Y2 / G, fields).
@@ -920,12 +926,12 @@ struct CubeK {
     static constexpr int BANKS = 128 / (2 * (int)sizeof(T));
     static constexpr int XP = N % 3 == 0 ? 3 : 4, XQ = N / XP;
     static constexpr int Y1 = G.Y1, Y2 = G.Y2;
-    static constexpr int W = (N >= 96 ? 64 : 32) / (2 * (int)sizeof(T));   // columns per tile
+    static constexpr int W = 64 / (2 * (int)sizeof(T));   // columns per tile
     static constexpr int C = Y2 * W;
     static constexpr int PITCH = C + ((W - C) % BANKS + BANKS) % BANKS;    // threads (i, w) on different banks
     static constexpr int NZB = N / W;
     static constexpr int NT = split_round32(split_max(XQ * W, XP * C));
-    static constexpr size_t SMEM = 2 * sizeof(T) * (size_t)N * PITCH + sizeof(T) * (size_t)N;   // tile, x factors
+    static constexpr size_t SMEM = 2 * sizeof(T) * (size_t)N * PITCH + 16 * (size_t)N;   // tile, x factors
     static_assert(N % W == 0 && XP * XQ == N, "tile shape");
 };
 
@@ -953,9 +959,9 @@ __global__ void __launch_bounds__(CubeK<N, T>::NT, split_max(1, 65536 / (CubeK<N
     // the op's x factors: 32 loads per thread from global memory throttled the
     // load queue (2.5 of 9.5 cycles per instruction at 128^3 complex64)
     constexpr bool XTAB = op_has_xtab<Op>::value;
-    T* xtab = reinterpret_cast<T*>(tile + N * PITCH);
+    typename op_xval<Op>::type* xtab = reinterpret_cast<typename op_xval<Op>::type*>(tile + N * PITCH);
     if constexpr (XTAB)
-        for (int j = tid; j < N; j += P::NT) xtab[j] = op.x_table()[j];
+        for (int j = tid; j < N; j += P::NT) xtab[j] = op.x_value(j);
     V tw[XP];
     if (one) {
 #pragma unroll
@@ -999,8 +1005,8 @@ __global__ void __launch_bounds__(CubeK<N, T>::NT, split_max(1, 65536 / (CubeK<N
         dft_any<S1, XQ>(u);
         constexpr int CH = op_loads<Op>::value == 0 ? XQ : XQ < 4 ? XQ : 4;   // operands in flight
         typename Op::Pre pre[CH];
-        T col = T(0);
-        if constexpr (XTAB) col = op.column(y, z);
+        typename op_xval<Op>::column col{};
+        if constexpr (XTAB) col = op.column(f, y, z);
 #pragma unroll
         for (int q = 0; q < XQ; ++q) {
             if (q % CH == 0) {
@@ -1009,7 +1015,7 @@ __global__ void __launch_bounds__(CubeK<N, T>::NT, split_max(1, 65536 / (CubeK<N
                     if (q + k < XQ) pre[k] = op.load(f, off + (size_t)(XP * (q + k)) * plane);
             }
             if constexpr (XTAB)
-                u[q] = op.apply_x(p + XP * q, y, z, off + (size_t)(XP * q) * plane, u[q], pre[q % CH], xtab[p + XP * q], col);
+                u[q] = op.apply_x(f, p + XP * q, y, z, off + (size_t)(XP * q) * plane, u[q], pre[q % CH], xtab[p + XP * q], col);
             else
                 u[q] = op.apply(f, p + XP * q, y, z, off + (size_t)(XP * q) * plane, u[q], pre[q % CH]);
         }
@@ -1085,8 +1091,9 @@ cudaError_t split_k_plan(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst, s
 // blocks of one field of the real-space pass
 inline int split_real_blocks(const SplitGeom& g) { return g.m1 * (g.Y2 / g.G); }
 
-// The production cubes run their compile-time plans (where g says so), the
-// passes at the ends of a sweep (one transform, run once) the run-time one.
+// The production cubes run their compile-time plans (where g says so); passes
+// with one transform (the ends of a sweep, the field transforms) only at 96 and
+// 128, where they are not a matter of launch latency.
 template <typename T, int S1, int S2, class Op>
 cudaError_t split_real_launch(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst, size_t fstride, int nf, const Op& op,
                               cudaStream_t stream)
@@ -1099,7 +1106,12 @@ cudaError_t split_real_launch(const SplitGeom& g, const cplx<T>* src, cplx<T>* d
         case 128: return split_real_plan<CubePlan<128, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
         default: break;
     }
-    if (g.big) return split_real_plan<RtBigPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+    else switch (g.cube) {
+        case 96: return split_real_plan<CubePlan<96, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+        case 128: return split_real_plan<CubePlan<128, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+        default: break;
+    }
+    if (g.big_r) return split_real_plan<RtBigPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
     return split_real_plan<RtPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
 }
 template <int N, typename T, int S1, int S2, class Op>
@@ -1121,7 +1133,7 @@ cudaError_t split_k_launch(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst,
         case 128: return cube_k<128, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
         default: break;
     }
-    if (g.big) return split_k_plan<RtBigPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+    if (g.big_k) return split_k_plan<RtBigPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
     return split_k_plan<RtPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
 }
 

@@ -321,7 +321,7 @@ class Engine:
     def get(self, name: str) -> np.ndarray:
         n = C.c_longlong(0)
         self._check(lib().ftsp_get_field(self.h, name.encode(), None, C.byref(n)), "get_field")
-        out = np.zeros(max(1, n.value), dtype=np.float64)
+        out = np.empty(max(1, n.value), dtype=np.float64)   # filled by the call
         self._check(lib().ftsp_get_field(self.h, name.encode(), out.ctypes.data, C.byref(n)), "get_field")
         return out[: n.value].view(np.complex128).reshape(-1, self.size)
 

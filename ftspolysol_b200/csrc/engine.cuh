@@ -1612,10 +1612,10 @@ struct Engine : EngineBase {
         prof_end(ev, "field_fft", units * sizeof(V) * (double)Vn);
         if (corr) {
             for (int f = 0; f < nf; ++f) {
-                k_combine<true><<<1, COMBINE_THREADS, 0, stream>>>(upart.p + (size_t)f * fparts, fparts, 1, ds->dmax + f);
+                launch_pass(k_combine<true>, dim3(1), COMBINE_THREADS, 0, (const double*)(upart.p + (size_t)f * fparts), (int)(fparts), 1, (double*)(ds->dmax + f));
                 ++launches;
             }
-            k_combine<false><<<1, COMBINE_THREADS, 0, stream>>>(upart.p + nparts, (int)nparts, 1, ds->corr + 2);
+            launch_pass(k_combine<false>, dim3(1), COMBINE_THREADS, 0, (const double*)(upart.p + nparts), (int)((int)nparts), 1, (double*)(ds->corr + 2));
             ++launches;
         }
     }
@@ -1707,7 +1707,7 @@ struct Engine : EngineBase {
         }, &ds->umax, (double)(c.nm + 1) * sizeof(V));
         DevScal* d = ds;
         const double uref = adaptive_u;
-        k_foreach<<<1, 32, 0, stream>>>(1, [=] __device__(size_t) {
+        one_warp(1, [=] __device__(size_t) {
             const double um = sqrt(d->umax);
             d->umax = um;
             d->dt_scale = (isfinite(um) && um > uref) ? uref / um : 1.0;
@@ -1871,7 +1871,7 @@ struct Engine : EngineBase {
             }, ds->lres);
             DevScal* d = ds;
             const double ratio = lr.fallback;
-            k_foreach<<<1, 32, 0, stream>>>(1, [=] __device__(size_t) {
+            one_warp(1, [=] __device__(size_t) {
                 const bool ok = isfinite(d->lres[0]) && d->lres[0] <= ratio * d->lres[1];
                 if (isfinite(d->lres[0]) && isfinite(d->lres[1])) {
                     d->lres_sum[0] += d->lres[0];
@@ -2112,6 +2112,15 @@ struct Engine : EngineBase {
         launch_pass(k_foreach<F>, dim3(std::max(1, blocks)), threads, 0, n, f);
         ++launches;
         prof_end(ev, "field_elementwise", bpe * (double)n);
+    }
+
+    // n <= 32 items by one warp (scalars of the step); a dependent launch like
+    // every kernel of the step, so that its launch latency overlaps the kernel
+    // before it
+    template <class F>
+    void one_warp(size_t n, F f)
+    {
+        launch_pass(k_foreach<F>, dim3(1), 32, 0, n, f);
     }
 
     // Blocks of kernel k resident at once on the current device (one wave),
@@ -2438,8 +2447,8 @@ struct Engine : EngineBase {
             DevScal* d = ds;
             const int* eF = expo.p;
             const int last = N - 1;
-            k_combine<false><<<2, COMBINE_THREADS, 0, stream>>>(qpart, cnt, 2, reinterpret_cast<double*>(&d->Q[isp]));
-            k_foreach<<<1, 32, 0, stream>>>(1, [=] __device__(size_t) {
+            launch_pass(k_combine<false>, dim3(2), COMBINE_THREADS, 0, (const double*)(qpart), (int)(cnt), 2, (double*)(reinterpret_cast<double*>(&d->Q[isp])));
+            one_warp(1, [=] __device__(size_t) {
                 const double2 Qs = dscale(d->Q[isp], invV);
                 d->factor[isp] = dscale(dinv(Qs), nv);
                 d->Q[isp] = make_double2(ldexp(Qs.x, eF[last]), ldexp(Qs.y, eF[last]));   // true Q
@@ -2810,6 +2819,8 @@ struct Engine : EngineBase {
             V* dBp = dB.p;
             float* slot = smax.p;
             const size_t slots = use_split ? smax.n : 0;
+            double* spp = spart.p;   // the stress partials start at zero
+            const size_t nsp = stress ? 12 * (size_t)stress_parts() : 0;
             if (ion_common) {
                 // the Boltzmann factors exp(-i z_j psi_s) are only summed here
                 // (Q_j); the combined ion charge is formed after the sweeps
@@ -2818,6 +2829,7 @@ struct Engine : EngineBase {
                 const T z0 = (T)ct.z[0];
                 reduce<6>(Vn, [=] __device__(size_t i, double* acc) {
                     for (size_t k = i; k < slots; k += Vn) slot[k] = 0.0f;
+                    for (size_t k = i; k < nsp; k += Vn) spp[k] = 0.0;
                     const V ps_ = __ldg(kBp + (size_t)M * Vn + i);
                     {
                         V w = __ldg(kBp + (size_t)t0 * Vn + i);
@@ -2850,7 +2862,7 @@ struct Engine : EngineBase {
                 IonTab ic{};
                 for (int j = 0; j < J; ++j) ic.nd[j] = c.ions[j].count / c.volume;
                 const double invV = 1.0 / (double)Vn;
-                k_foreach<<<1, 32, 0, stream>>>((size_t)J, [=] __device__(size_t j) {
+                one_warp((size_t)J, [=] __device__(size_t j) {
                     const double2 Q = dscale(d->Qion[j], invV);
                     d->Qion[j] = Q;
                     d->ion_factor[j] = dscale(dinv(Q), ic.nd[j]);
@@ -2859,6 +2871,7 @@ struct Engine : EngineBase {
             } else {
                 foreach(Vn, [=] __device__(size_t i) {
                     for (size_t k = i; k < slots; k += Vn) slot[k] = 0.0f;
+                    for (size_t k = i; k < nsp; k += Vn) spp[k] = 0.0;
                     const V ps_ = kBp[(size_t)M * Vn + i];
                     for (int k = 0; k < ncls; ++k) {
                         V w = kBp[(size_t)ct.type[k] * Vn + i];
@@ -2878,7 +2891,6 @@ struct Engine : EngineBase {
                 }, (double)(2 * (c.M + 1 + J) + (int)c.cls.size()) * sizeof(V));
             }
         }
-        if (stress) FTSP_CUDA(cudaMemsetAsync(spart.p, 0, sizeof(double) * 12 * (size_t)stress_parts(), stream));
         // 4. chain propagators of every species
         for (int isp = 0; isp < (int)c.sp.size(); ++isp) solve_species(isp, stress);
         if (!fx) charge_fold();
@@ -2943,7 +2955,7 @@ struct Engine : EngineBase {
             IonTab ic{};
             for (int j = 0; j < J; ++j) ic.nd[j] = c.ions[j].count / c.volume;
             const double invV = 1.0 / (double)Vn;
-            k_foreach<<<1, 32, 0, stream>>>((size_t)J, [=] __device__(size_t j) {
+            one_warp((size_t)J, [=] __device__(size_t j) {
                 const double2 Q = dscale(to_d(dBp[(size_t)(M + 1 + j) * Vn]), invV);
                 d->Qion[j] = Q;
                 d->ion_factor[j] = dscale(dinv(Q), ic.nd[j]);
@@ -3484,7 +3496,7 @@ struct Engine : EngineBase {
     void finalize_record(bool with_stress)
     {
         if (with_stress) {
-            k_combine<false><<<12, COMBINE_THREADS, 0, stream>>>(spart.p, stress_parts(), 12, ds->sconn);
+            launch_pass(k_combine<false>, dim3(12), COMBINE_THREADS, 0, (const double*)(spart.p), (int)(stress_parts()), 12, (double*)(ds->sconn));
             ++launches;
         }
         const int S = (int)c.sp.size(), J = (int)c.ions.size(), nm = c.nm;
@@ -3527,7 +3539,7 @@ struct Engine : EngineBase {
         const bool elec = c.elec;
         DevScal* d = ds;
         const bool ws = with_stress;
-        k_foreach<<<1, 32, 0, stream>>>(1, [=] __device__(size_t) {
+        one_warp(1, [=] __device__(size_t) {
             double2* rec = reinterpret_cast<double2*>(d->rec);
             int k = 0;
             double2 chem[MAXSP + MAXION];
@@ -3939,7 +3951,7 @@ struct Engine : EngineBase {
         });
         double* pend = avg.on ? avg.acc.p + (size_t)avg.nblk * (c.record_len() + 2) : nullptr;
         const int R2 = c.record_len() + 2;
-        k_foreach<<<1, 32, 0, stream>>>(1, [=] __device__(size_t) {
+        one_warp(1, [=] __device__(size_t) {
             if (d->bad_last && !d->exhausted) {
                 if (d->restarts >= cap) {
                     d->exhausted = 1;
@@ -3960,7 +3972,7 @@ struct Engine : EngineBase {
     {
         DevScal* d = ds;
         const int S = (int)c.sp.size(), R = c.record_len();
-        k_foreach<<<1, 32, 0, stream>>>(1, [=] __device__(size_t) {
+        one_warp(1, [=] __device__(size_t) {
             bool bad = d->nonfinite != 0 || d->corr[2] != 0.0 || d->exhausted != 0;
             for (int s = 0; s < S; ++s) bad |= !(isfinite(d->Q[s].x) && isfinite(d->Q[s].y));
             for (int i = 0; i < 2 * R; ++i) bad |= !isfinite(d->rec[i]);
@@ -3994,13 +4006,14 @@ struct Engine : EngineBase {
         const bool st = c.stress_on();
         eval(0, false);
         // save Q of the first evaluation for the finite check
-        FTSP_CUDA(cudaMemsetAsync(&ds->nonfinite, 0, sizeof(int), stream));
         {
             DevScal* d = ds;
             const int S = (int)c.sp.size();
-            k_foreach<<<1, 32, 0, stream>>>(1, [=] __device__(size_t) {
+            one_warp(1, [=] __device__(size_t) {
+                int bad = 0;
                 for (int s = 0; s < S; ++s)
-                    if (!isfinite(d->Q[s].x) || !isfinite(d->Q[s].y)) d->nonfinite = 1;
+                    if (!isfinite(d->Q[s].x) || !isfinite(d->Q[s].y)) bad = 1;
+                d->nonfinite = bad;
             });
             ++launches;
         }
@@ -4259,7 +4272,7 @@ struct Engine : EngineBase {
             }
         }
         double* out = reinterpret_cast<double*>(&ds->Q[0]);
-        k_combine<false><<<2, COMBINE_THREADS, 0, stream>>>(part.p, seg_pass_ctas(), 2, out);
+        launch_pass(k_combine<false>, dim3(2), COMBINE_THREADS, 0, (const double*)(part.p), (int)(seg_pass_ctas()), 2, (double*)(out));
         ++launches;
         double q[2];
         FTSP_CUDA(cudaMemcpyAsync(q, out, sizeof(q), cudaMemcpyDeviceToHost, stream));

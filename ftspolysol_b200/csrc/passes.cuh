@@ -1,4 +1,5 @@
-// FFT pass kernels with fused pointwise work.
+// FFT pass kernels with fused pointwise work: the run-time plans for grids
+// that the split-y passes (split_passes.cuh) do not take, and the ops of both.
 //
 // A 3-D transform of an m1 x m2 x m3 row-major grid (z fastest) is split
 // into passes that each read and write HBM once:

@@ -28,15 +28,14 @@
 // complex128, where the y transform became two more passes over memory.  The
 // tiles here are 8-40 KB, so several blocks share an SM and hide each
 // other's loads and barriers, and every grid takes two passes per segment.
-// Measured on one B200, whole calls before and after (the plane and line
-// passes of passes.cuh against these): chain of 50 segments at 128^3
-// complex128 3.56 -> 2.38 ms (72.7 -> 48.5 us per segment, floor 10.3 at the
-// measured copy rate); 40 segments at 90 x 125 x 100 complex128 5.33 -> 2.50
-// ms; step at 96^3 complex64, N = 32, 8.8 -> 3.7 ms; step at 64^3 complex64,
-// N = 50, 1.44 -> 1.17 ms.  Both passes are bound by issue slots and by the
-// latency of their five dependent phases, not by memory: at 128^3 complex64
-// the real-space pass issues 0.51 and the k-space pass 0.37 instructions per
-// cycle and scheduler over 12 us of active time.
+// Measured on one B200, whole calls with the plane and line passes of
+// passes.cuh and with these, in turn: chain of 50 segments at 128^3 complex128
+// 3.56 -> 1.98 ms (72.7 -> 40 us per segment, 10.3 at the measured copy rate);
+// 40 segments at 90 x 125 x 100 complex128 5.28 -> 2.00 ms; step at 96^3
+// complex64, N = 32, 8.7 -> 2.1 ms; step at 64^3 complex64, N = 50, 1.44 -> 1.15
+// ms.  Both passes are bound by issue slots and by the latency of their
+// dependent phases, not by memory: at 128^3 complex64 the real-space pass
+// issues 0.41 instructions per cycle and scheduler over 22 K active cycles.
 //
 // The radices come from a plan: RtPlan reads them from the geometry (a
 // uniform switch per phase; any extents that factor into two radices),
@@ -915,7 +914,9 @@ __global__ void __launch_bounds__(P::KNT, split_min_blocks<P, T, Op>(P::KNT))
 #undef FTSP_DIV
 
 // The k-space pass of a cube with m1 = XP * XQ in two exchanges instead of
-// four: a thread first holds the Y2 rows of XP points x = i + XQ p of one
+// four (128^3 complex64: 24.0 K -> 17.3 K active cycles, with its real-space
+// pass 26.5 -> 20.4 us per segment; 64-byte rows 23.3, 32-byte rows 24.6 with
+// the pair densities' share; the smaller cubes have too few threads for it): a thread first holds the Y2 rows of XP points x = i + XQ p of one
 // column (DFT over the rows, DFT over p, twiddle), then the XQ points of one
 // (p, row, column) for the second x stage, the op and its inverse; it writes
 // those back where it read them, so the pass has two barriers and the XP - 1

@@ -335,9 +335,10 @@ int ftsp_learn_set_weights(ftsp_handle* h, const float* w, int n);
 int ftsp_learn_grad(ftsp_handle* h, const float* x, const float* t, const float* m, int n, double* loss, float* grad);
 
 /* Launch geometry chosen for the handle's grid (autotune = 1): FFT radix
- * cap, strided tile width, how many alternatives were timed and the time of
- * one forward + inverse 3-D transform with the chosen and with the default
- * geometry.  compile_time = 1: every pass of this grid is a compile-time
+ * cap, tile width of the k-space pass, how many alternatives were timed and
+ * the time of one bond and one segment pass (grids whose extents have no two
+ * radices: of one forward + inverse 3-D transform) with the chosen and with
+ * the default geometry.  compile_time = 1: every pass of this grid is a compile-time
  * kernel and nothing was tuned.  No reference counterpart. */
 typedef struct ftsp_tune_info {
     int tuned, cached, compile_time;

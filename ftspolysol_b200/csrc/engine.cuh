@@ -1119,6 +1119,7 @@ struct Engine : EngineBase {
         if (x_threads > 256 || y_threads > 256 || z_threads > 256) throw std::runtime_error("grid dimension too large for the line passes");
         if (!sg.m1) split_setup(sg, m1, m2, m3, (int)sizeof(V));
         use_split = sg.ok;
+        if (use_split) geo_W = sg.W;   // the tile width that is tuned and reported
     }
 
     void allocate()
@@ -1267,9 +1268,9 @@ struct Engine : EngineBase {
             return;
         }
         TuneResult r{};
-        if (all_compile_time()) {
+        if (all_compile_time()) {   // the tiles it has: the next handle of the grid takes them from the cache
             r.max_bits = geo_max_bits;
-            r.W = geo_W;
+            r.W = geo_W; r.G = sg.G; r.cube = sg.cube;
             tune_cache()[key] = r;
             tune = r;
             return;

@@ -3706,7 +3706,10 @@ struct Engine : EngineBase {
     // (complex64: through the sweeps' scratch field, half a field at a time)
     // and copied straight to the caller.  Above 4 MiB the caller's pages are
     // touched by a few threads first: memory of that size comes fresh from
-    // the system, and its first touch costs more than the copy.  Measured,
+    // the system, and its first touch costs more than the copy.  The touch is
+    // an atomic add of zero, which maps the page and changes nothing: the
+    // buffer may still be the source of an upload in flight
+    // (ftsp_set_fields_async), and a failing call leaves it alone.  Measured,
     // complex64 into fresh memory: 128^3 18 ms (copy, then a host loop) -> 6,
     // 96^3 3.3 -> 2.0, 64^3 1.0 -> 0.65; a pinned staging buffer was no
     // faster and took 2-7 ms to allocate.
@@ -3716,7 +3719,7 @@ struct Engine : EngineBase {
         if (bytes >= ((size_t)4 << 20)) {
             const size_t pages = bytes / 4096;
             auto touch = [out](size_t a, size_t b) {
-                for (size_t i = a; i < b; ++i) *reinterpret_cast<volatile double*>(out + i * 512) = 0.0;
+                for (size_t i = a; i < b; ++i) __atomic_fetch_add(reinterpret_cast<unsigned long long*>(out + i * 512), 0ull, __ATOMIC_RELAXED);
             };
             const size_t nt = std::min(8u, std::max(1u, std::thread::hardware_concurrency()));
             std::vector<std::thread> pool;

@@ -3739,12 +3739,14 @@ struct Engine : EngineBase {
         } else {
             double2* d = reinterpret_cast<double2*>(G.p);
             const size_t chunk = std::max<size_t>(1, V_ / 2);
+            const long long of_step = launches;   // the conversions are no launches of the step
             for (size_t i0 = 0; i0 < n; i0 += chunk) {
                 const size_t m = std::min(chunk, n - i0);
                 const V* src = p + i0;
                 foreach(m, [=] __device__(size_t i) { d[i] = to_d(src[i]); });
                 FTSP_CUDA(cudaMemcpyAsync(out + 2 * i0, d, sizeof(double2) * m, cudaMemcpyDeviceToHost, stream));
             }
+            launches = of_step;
         }
         FTSP_CUDA(cudaStreamSynchronize(stream));
     }

@@ -46,3 +46,17 @@ def test_read_into_the_uploaded_buffer(prec):
             got = host.numpy().view(np.complex128).reshape(2, n)
             np.testing.assert_array_equal(got[0], ref["omega"])
             np.testing.assert_array_equal(got[1], ref["psi"])
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_reads_are_not_launches_of_the_step(prec):
+    from ftspolysol_b200 import Engine, FP32, FP64
+    case = solution((16, 15, 12))
+    om, ps = case.initial_fields()
+    with Engine(derive(case), precision=FP64 if prec == "fp64" else FP32) as e:
+        e.set_fields(om, ps)
+        e.step()
+        n = e.launches()
+        for name in ("omega", "rho_type", "psi_s"):
+            e.get(name)
+        assert e.launches() == n

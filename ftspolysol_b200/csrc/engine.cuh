@@ -1038,7 +1038,7 @@ struct Engine : EngineBase {
         }
         if (ev_staged) cudaEventDestroy(ev_staged);
         if (ev_installed) cudaEventDestroy(ev_installed);
-        astage.release();
+        astage.release(); ostage.release();
         Buf<V>* vb[] = {&tw1, &tw2, &tw3, &omega, &psi, &omega_bar, &psi_bar, &drift, &drift_bar, &dpsi, &dpsi_bar,
                         &kA, &kB, &dB, &kC, &rho_p, &rho_c, &ion_rho, &E, &qF, &Fst, &G, &H};
         for (auto* b : vb) b->release();
@@ -1149,7 +1149,7 @@ struct Engine : EngineBase {
         for (auto& s : c.sp) Nmax = std::max(Nmax, s.N);
         qF.alloc(Vn * Nmax);
         if (c.stress_on()) Fst.alloc(Vn * Nmax);
-        G.alloc(std::max<size_t>(Vn, 2)); H.alloc(Vn);   // G: also one FP64 value of copy_out at least
+        G.alloc(Vn); H.alloc(Vn);
         part.alloc((size_t)std::max(RED_BLOCKS, std::max(c.m1, c.m1 * c.m2)) * 32);
         expo.alloc((size_t)2 * Nmax);
         pmax.alloc((size_t)2 * std::max(c.m1, c.m1 * c.m2));
@@ -3703,8 +3703,9 @@ struct Engine : EngineBase {
     }
 
     // n device values to host memory as FP64 pairs: converted on the device
-    // (complex64: through the sweeps' scratch field, half a field at a time)
-    // and copied straight to the caller.  Above 4 MiB the caller's pages are
+    // (complex64: through a staging buffer, so that a read changes nothing
+    // that a step uses, also one in flight on another stream) and copied
+    // straight to the caller.  Above 4 MiB the caller's pages are
     // touched by a few threads first: memory of that size comes fresh from
     // the system, and its first touch costs more than the copy.  The touch is
     // an atomic add of zero, which maps the page and changes nothing: the
@@ -3713,6 +3714,7 @@ struct Engine : EngineBase {
     // complex64 into fresh memory: 128^3 18 ms (copy, then a host loop) -> 6,
     // 96^3 3.3 -> 2.0, 64^3 1.0 -> 0.65; a pinned staging buffer was no
     // faster and took 2-7 ms to allocate.
+    Buf<double2> ostage;
     void copy_out(const V* p, size_t n, double* out)
     {
         const size_t bytes = n * sizeof(double2);
@@ -3737,8 +3739,10 @@ struct Engine : EngineBase {
         if constexpr (!F32) {
             FTSP_CUDA(cudaMemcpyAsync(out, p, bytes, cudaMemcpyDeviceToHost, stream));
         } else {
-            double2* d = reinterpret_cast<double2*>(G.p);
-            const size_t chunk = std::max<size_t>(1, V_ / 2);
+            // the buffer that set_fields left, or 4 MiB where it was never called
+            if (!stage.p && !ostage.p) ostage.alloc(std::min<size_t>(V_, (size_t)1 << 18));
+            double2* d = stage.p ? stage.p : ostage.p;
+            const size_t chunk = stage.p ? stage.n : ostage.n;
             const long long of_step = launches;   // the conversions are no launches of the step
             for (size_t i0 = 0; i0 < n; i0 += chunk) {
                 const size_t m = std::min(chunk, n - i0);

@@ -60,3 +60,27 @@ def test_reads_are_not_launches_of_the_step(prec):
         for name in ("omega", "rho_type", "psi_s"):
             e.get(name)
         assert e.launches() == n
+
+
+def test_a_read_leaves_a_step_in_flight_alone():
+    """A read while the batch steps returns fields of no one time, but the
+    steps go on as without it."""
+    from ftspolysol_b200 import Engine, FP32, SCHEME_SI
+    from ftspolysol_b200.engine import Batch
+    case = solution((64, 64, 64), 20)
+    om, ps = case.initial_fields()
+    out = []
+    for read in (False, True):
+        e = Engine(derive(case), precision=FP32, scheme=SCHEME_SI, noise=True, seed=3)
+        e.set_fields(om, ps)
+        b = Batch([e], 2)
+        b.step(20)
+        if read:
+            for _ in range(4):
+                e.get("rho_type")
+        b.sync()
+        out.append((e.get("omega"), e.get("psi")))
+        b.close()
+        e.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)

@@ -20,14 +20,16 @@ INCLUDE = os.path.join(ROOT, "include")
 LIB = os.path.join(HERE, "libftsp.so")
 
 SOURCES = ["engine_f32.cu", "engine_f64.cu", "split_real_f32.cu", "split_real_f64.cu", "split_k_f32.cu", "split_k_f64.cu",
-           "abi.cu"]
+           "line_f32.cu", "line_f64.cu", "abi.cu"]
 HOST_SOURCES = ["host_model.cpp", "host_io.cpp", "host_run.cpp"]
 HEADERS = ["fft_core.cuh", "passes.cuh", "chain_pairs.cuh", "split_passes.cuh", "learned.cuh", "engine.cuh", "host_model.h", "host_io.h"]
 MAIN = os.path.join(HERE, "ftsp_main")
 HOST_FLAGS = ["-O2", "-std=c++17", "-Xcompiler", "-fPIC,-O2,-Wall"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--extended-lambda", "-Xcompiler", "-fPIC,-O2",
-         "-Xptxas", "-warn-spills", "-split-compile", "0"]
+         "-Xptxas", "-warn-spills"]
+# Kernels compiled in parallel, except where they call functions (line_*.cu)
+PARALLEL = ["-split-compile", "0"]
 
 
 def nvcc() -> str:
@@ -58,6 +60,8 @@ def build(force: bool = False, verbose: bool = False, extra=None) -> str:
         obj = os.path.join(objdir, os.path.splitext(src)[0] + ".o")
         objs.append(obj)
         flags = ARCH + FLAGS if src.endswith(".cu") else HOST_FLAGS
+        if src.endswith(".cu") and not src.startswith("line_"):
+            flags = flags + PARALLEL
         cmd = [nvcc()] + flags + ["-I", INCLUDE, "-I", CSRC, "-c", os.path.join(CSRC, src), "-o", obj]
         if extra:
             cmd += list(extra)

@@ -714,7 +714,7 @@ extern "C" int ftsp_propagate_chain_noalloc(int m1, int m2, int m3, double L1, d
         // launch geometry of the runtime-plan passes (complex128)
         int dev_smem = 0;
         FTSP_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        constexpr int EP = 16, EL = 8;
+        constexpr int EP = LINE_EP<double>, EL = LINE_EL<double>;
         auto round32 = [](int t) { return std::max(32, (t + 31) / 32 * 32); };
         PlaneGeom pg{};
         pg.m1 = m1; pg.m2 = m2; pg.m3 = m3; pg.P = m3 + 1;
@@ -746,9 +746,6 @@ extern "C" int ftsp_propagate_chain_noalloc(int m1, int m2, int m3, double L1, d
         const double2* tw1 = dtab->tw[0];
         const double2* tw2 = dtab->tw[1];
         const double2* tw3 = dtab->tw[2];
-        auto smem_attr = [&](auto kernel, size_t bytes) {
-            if (bytes > 48 * 1024) FTSP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-        };
         // real-space pass of one segment (split-y pass, plane, or y / z-line / y)
         auto seg = [&](auto s1c, auto s2c, const double2* src, double2* dst, const auto& op) {
             constexpr int S1 = decltype(s1c)::value, S2 = decltype(s2c)::value;
@@ -758,24 +755,15 @@ extern "C" int ftsp_propagate_chain_noalloc(int m1, int m2, int m3, double L1, d
                 return;
             }
             if (plane_ok) {
-                auto k = k_plane<double, EP, S1, S2, Op>;
-                smem_attr(k, plane_smem);
-                k<<<dim3(m1, 1), plane_threads, plane_smem, stream>>>(pg, src, dst, V, tw2, tw3, op);
+                FTSP_CUDA((plane_launch<double, EP, S1, S2, Op>(pg, src, dst, 1, V, tw2, tw3, plane_threads, plane_smem, op, stream)));
                 return;
             }
-            if (S1 != 0) {
-                auto k = k_strided<double, EL, 1, 0, S1, OpLoadOne<double>>;
-                smem_attr(k, y_smem);
-                k<<<dim3(m1 * (m3 / W), 1), y_threads, y_smem, stream>>>(gy, nullptr, const_cast<double2*>(src), V, tw2, OpLoadOne<double>{src});
-            }
-            auto kz = k_zline<double, EL, S1, S2, Op>;
-            smem_attr(kz, z_smem);
-            kz<<<dim3(m1 * m2 / B, 1), z_threads, z_smem, stream>>>(gz, src, dst, V, tw3, op);
-            if (S2 != 0) {
-                auto k = k_strided<double, EL, 1, 0, S2, OpLoadOne<double>>;
-                smem_attr(k, y_smem);
-                k<<<dim3(m1 * (m3 / W), 1), y_threads, y_smem, stream>>>(gy, nullptr, dst, V, tw2, OpLoadOne<double>{dst});
-            }
+            using Load = OpLoadOne<double>;   // y-lines, in place
+            if constexpr (S1 != 0)
+                FTSP_CUDA((strided_launch<double, EL, 1, 0, S1, Load>(gy, nullptr, const_cast<double2*>(src), 1, V, tw2, y_threads, y_smem, Load{src}, stream)));
+            FTSP_CUDA((zline_launch<double, EL, S1, S2, Op>(gz, src, dst, 1, V, tw3, z_threads, z_smem, op, stream)));
+            if constexpr (S2 != 0)
+                FTSP_CUDA((strided_launch<double, EL, 1, 0, S2, Load>(gy, nullptr, dst, 1, V, tw2, y_threads, y_smem, Load{dst}, stream)));
         };
         OpBond<double, true, false> ob{};
         ob.phix = dtab->phi;
@@ -788,9 +776,7 @@ extern "C" int ftsp_propagate_chain_noalloc(int m1, int m2, int m3, double L1, d
                 FTSP_CUDA((split_k_launch<double, -1, +1, OB>(sg, Gb, Gb, V, 1, ob, stream)));
                 return;
             }
-            auto kb = k_strided<double, EL, 0, -1, +1, OB>;
-            smem_attr(kb, x_smem);
-            kb<<<dim3(m2 * (m3 / W), 1), x_threads, x_smem, stream>>>(gx, Gb, Gb, V, tw1, ob);
+            FTSP_CUDA((strided_launch<double, EL, 0, -1, +1, OB>(gx, Gb, Gb, 1, V, tw1, x_threads, x_smem, ob, stream)));
         };
 
         const double2* wp = reinterpret_cast<const double2*>(w);

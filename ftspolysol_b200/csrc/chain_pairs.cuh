@@ -194,11 +194,13 @@ struct PairVec<double> {
     }
 };
 
+// Two blocks per SM asked for in complex64: with 128 registers the loads of
+// four pairs are in flight, with the 101 of the compiler's own choice fewer
+// (59 and 68 us at 128^3, N = 16); complex128 takes 102 us either way.
 template <typename T>
-__global__ void __launch_bounds__(256) k_pair_density_vec(size_t n, PairTable tb, const cplx<T>* __restrict__ u,
-                                                          const cplx<T>* __restrict__ E, const int* __restrict__ eF,
-                                                          int N, const double2* __restrict__ factor, cplx<T>* rho,
-                                                          cplx<T>* rho_charge)
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 0)
+    k_pair_density_vec(size_t n, PairTable tb, const cplx<T>* __restrict__ u, const cplx<T>* __restrict__ E,
+                       const int* __restrict__ eF, int N, const double2* __restrict__ factor, cplx<T>* rho, cplx<T>* rho_charge)
 {
     using V = cplx<T>;
     using PV = PairVec<T>;

@@ -776,6 +776,57 @@ struct OpStore {
     __device__ __forceinline__ void end(double*, size_t) {}
 };
 
+// Elements per thread of the run-time passes: plane, lines.
+template <typename T> constexpr int LINE_EP = sizeof(T) == 4 ? 32 : 16;
+template <typename T> constexpr int LINE_EL = sizeof(T) == 4 ? 16 : 8;
+
+// The run-time passes of an engine (and of the allocation-free chain call).
+#define FTSP_PLANE(PRE, T, S1, S2, ...)                                                                                     \
+    PRE cudaError_t plane_launch<T, LINE_EP<T>, S1, S2, __VA_ARGS__>(const PlaneGeom&, const cplx<T>*, cplx<T>*, int, size_t,     \
+                                                                     const cplx<T>*, const cplx<T>*, int, size_t,                 \
+                                                                     const __VA_ARGS__&, cudaStream_t);
+#define FTSP_STRIDED(PRE, T, DIM, S1, S2, ...)                                                                              \
+    PRE cudaError_t strided_launch<T, LINE_EL<T>, DIM, S1, S2, __VA_ARGS__>(const LineGeom&, const cplx<T>*, cplx<T>*, int,       \
+                                                                            size_t, const cplx<T>*, int, size_t,                  \
+                                                                            const __VA_ARGS__&, cudaStream_t);
+#define FTSP_ZLINE(PRE, T, S1, S2, ...)                                                                                     \
+    PRE cudaError_t zline_launch<T, LINE_EL<T>, S1, S2, __VA_ARGS__>(const LineGeom&, const cplx<T>*, cplx<T>*, int, size_t,      \
+                                                                     const cplx<T>*, int, size_t, const __VA_ARGS__&, cudaStream_t);
+#define FTSP_PROP(PRE, T, S1, S2, KIND)       \
+    FTSP_PLANE(PRE, T, S1, S2, OpProp<T, KIND>) \
+    FTSP_ZLINE(PRE, T, S1, S2, OpProp<T, KIND>)
+#define FTSP_LINE_ALL(PRE, T)                               \
+    FTSP_PROP(PRE, T, 0, -1, FWD_START)                     \
+    FTSP_PROP(PRE, T, 1, -1, FWD_MID)                       \
+    FTSP_PROP(PRE, T, 1, 0, FWD_LAST)                       \
+    FTSP_PROP(PRE, T, 0, 0, FWD_SINGLE)                     \
+    FTSP_PROP(PRE, T, 0, 1, BWD_START)                      \
+    FTSP_PROP(PRE, T, -1, 1, BWD_MID)                       \
+    FTSP_PROP(PRE, T, -1, 0, BWD_LAST)                      \
+    FTSP_PROP(PRE, T, 0, 0, BWD_SINGLE)                     \
+    FTSP_STRIDED(PRE, T, 0, -1, 1, OpBond<T, true, false>)  \
+    FTSP_STRIDED(PRE, T, 0, 1, -1, OpBond<T, false, true>)  \
+    FTSP_STRIDED(PRE, T, 0, 1, -1, OpBond<T, false, false>) \
+    FTSP_STRIDED(PRE, T, 1, 0, 1, OpLoadOne<T>)             \
+    FTSP_STRIDED(PRE, T, 1, 0, -1, OpLoadOne<T>)            \
+    FTSP_PLANE(PRE, T, 0, 1, OpLoadN<T>)                    \
+    FTSP_PLANE(PRE, T, 0, -1, OpLoadN<T>)                   \
+    FTSP_ZLINE(PRE, T, 0, 1, OpLoadN<T>)                    \
+    FTSP_ZLINE(PRE, T, 0, -1, OpLoadN<T>)                   \
+    FTSP_STRIDED(PRE, T, 0, 0, 1, OpLoadN<T>)               \
+    FTSP_STRIDED(PRE, T, 0, 0, -1, OpLoadN<T>)              \
+    FTSP_STRIDED(PRE, T, 1, 0, 1, OpLoadN<T>)               \
+    FTSP_STRIDED(PRE, T, 1, 0, -1, OpLoadN<T>)              \
+    FTSP_PLANE(PRE, T, 0, -1, OpIncrement<T, false>)        \
+    FTSP_PLANE(PRE, T, 0, -1, OpIncrement<T, true>)         \
+    FTSP_STRIDED(PRE, T, 0, -1, 1, OpPrecond<T>)            \
+    FTSP_PLANE(PRE, T, 1, 0, OpStore<T>)                    \
+    FTSP_PLANE(PRE, T, 1, 0, OpUpdate<T>)
+#ifndef FTSP_LINE_INSTANCES
+FTSP_LINE_ALL(extern template, float)
+FTSP_LINE_ALL(extern template, double)
+#endif
+
 // ---------------------------------------------------------------------------
 // Engine
 // ---------------------------------------------------------------------------
@@ -952,8 +1003,7 @@ struct Engine : EngineBase {
     int plane_threads = 0, x_threads = 0, y_threads = 0, z_threads = 0;
     size_t plane_smem = 0, x_smem = 0, y_smem = 0, z_smem = 0;
     static constexpr bool F32 = sizeof(T) == 4;
-    static constexpr int EP = F32 ? 32 : 16;   // elements per thread, runtime-plan plane pass
-    static constexpr int EL = F32 ? 16 : 8;    // elements per thread, runtime-plan line passes
+    static constexpr int EP = LINE_EP<T>, EL = LINE_EL<T>;
     Buf<FftPlan1> plans;                       // device-memory plans: x, y, z
 
     // device buffers
@@ -2185,9 +2235,7 @@ struct Engine : EngineBase {
     template <int S1, int S2, class Op>
     void plane(const V* src, V* dst, int nf, const Op& op)
     {
-        auto kp = k_plane<T, EP, S1, S2, Op>;
-        set_smem(kp, plane_smem);
-        kp<<<dim3(c.m1, nf), plane_threads, plane_smem, stream>>>(pg, src, dst, V_, tw2.p, tw3.p, op);
+        FTSP_CUDA((plane_launch<T, EP, S1, S2, Op>(pg, src, dst, nf, V_, tw2.p, tw3.p, plane_threads, plane_smem, op, stream)));
         ++launches;
     }
 
@@ -2201,13 +2249,8 @@ struct Engine : EngineBase {
         if constexpr (op_has_src<Op>::value) {
             throw std::runtime_error("an op with a source map needs the split passes");
         } else {
-            const LineGeom& g = DIM == 1 ? gy : gx;
-            auto k = k_strided<T, EL, DIM, S1, S2, Op>;
-            const size_t smem = DIM == 1 ? y_smem : x_smem;
-            set_smem(k, smem);
-            const int outer = DIM == 1 ? c.m1 : c.m2;
-            k<<<dim3(outer * (c.m3 / g.W), nf), DIM == 1 ? y_threads : x_threads, smem, stream>>>(g, src, dst, V_,
-                                                                                                DIM == 1 ? tw2.p : tw1.p, op);
+            FTSP_CUDA((strided_launch<T, EL, DIM, S1, S2, Op>(DIM == 1 ? gy : gx, src, dst, nf, V_, DIM == 1 ? tw2.p : tw1.p,
+                                                              DIM == 1 ? y_threads : x_threads, DIM == 1 ? y_smem : x_smem, op, stream)));
             ++launches;
         }
     }
@@ -2215,9 +2258,7 @@ struct Engine : EngineBase {
     template <int S1, int S2, class Op>
     void zline(const V* src, V* dst, int nf, const Op& op)
     {
-        auto k = k_zline<T, EL, S1, S2, Op>;
-        set_smem(k, z_smem);
-        k<<<dim3(c.m1 * c.m2 / gz.B, nf), z_threads, z_smem, stream>>>(gz, src, dst, V_, tw3.p, op);
+        FTSP_CUDA((zline_launch<T, EL, S1, S2, Op>(gz, src, dst, nf, V_, tw3.p, z_threads, z_smem, op, stream)));
         ++launches;
     }
 
@@ -2927,7 +2968,7 @@ struct Engine : EngineBase {
             ld.Vn = Vn;
             for (size_t k = 0; k < fold_type.size(); ++k)
                 if (fold_type[k] >= 0) ld.zf += fold_z[k];   // one type: at most one species folds
-            yz_forward(kC.p, 3, ld);
+            split_real<0, -1>(nullptr, kC.p, 3, ld);
             const double invV = 1.0 / (double)Vn;
             OpKScale<T> op{};
             op.kst = dB.p;

@@ -300,6 +300,47 @@ __global__ void __launch_bounds__(256, 2) k_strided(LineGeom g, const cplx<T>* s
     op.end(reinterpret_cast<double*>(tile), blockIdx.x + (size_t)blockIdx.y * gridDim.x);
 }
 
+// ---- launches of the run-time passes ----
+// Compiled in line_f32.cu and line_f64.cu (FTSP_LINE_ALL in engine.cuh): the
+// radix stages are functions, and a compilation that takes the functions of a
+// file one by one (-split-compile) costs these passes up to 1.6 times (bond
+// pass at 486 x 64 x 64 complex64 72 us, 117 with it; 243 x 16 x 20 27 and 35).
+template <class K>
+inline cudaError_t pass_smem(K kernel, size_t bytes)
+{
+    return bytes > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) : cudaSuccess;
+}
+template <typename T, int E, int S1, int S2, class Op>
+cudaError_t plane_launch(const PlaneGeom& g, const cplx<T>* src, cplx<T>* dst, int nf, size_t fstride, const cplx<T>* twy,
+                         const cplx<T>* twz, int threads, size_t smem, const Op& op, cudaStream_t stream)
+{
+    auto k = k_plane<T, E, S1, S2, Op>;
+    const cudaError_t e = pass_smem(k, smem);
+    if (e != cudaSuccess) return e;
+    k<<<dim3(g.m1, nf), threads, smem, stream>>>(g, src, dst, fstride, twy, twz, op);
+    return cudaGetLastError();
+}
+template <typename T, int E, int DIM, int S1, int S2, class Op>
+cudaError_t strided_launch(const LineGeom& g, const cplx<T>* src, cplx<T>* dst, int nf, size_t fstride, const cplx<T>* tw,
+                           int threads, size_t smem, const Op& op, cudaStream_t stream)
+{
+    auto k = k_strided<T, E, DIM, S1, S2, Op>;
+    const cudaError_t e = pass_smem(k, smem);
+    if (e != cudaSuccess) return e;
+    k<<<dim3((DIM == 1 ? g.m1 : g.m2) * (g.m3 / g.W), nf), threads, smem, stream>>>(g, src, dst, fstride, tw, op);
+    return cudaGetLastError();
+}
+template <typename T, int E, int S1, int S2, class Op>
+cudaError_t zline_launch(const LineGeom& g, const cplx<T>* src, cplx<T>* dst, int nf, size_t fstride, const cplx<T>* tw,
+                         int threads, size_t smem, const Op& op, cudaStream_t stream)
+{
+    auto k = k_zline<T, E, S1, S2, Op>;
+    const cudaError_t e = pass_smem(k, smem);
+    if (e != cudaSuccess) return e;
+    k<<<dim3(g.m1 * g.m2 / g.B, nf), threads, smem, stream>>>(g, src, dst, fstride, tw, op);
+    return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------
 // Pointwise ops
 // ---------------------------------------------------------------------------

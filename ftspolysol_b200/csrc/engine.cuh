@@ -1020,7 +1020,14 @@ struct Engine : EngineBase {
     Buf<V> kC;           // (M + 3) * V : rho_type, rho_c_poly, rho_c_ion, psi-drift part
     Buf<V> rho_p, rho_c, ion_rho;
     Buf<V> E;            // class tables exp(-W_c)
-    Buf<V> qF, Fst, G, H;
+    Buf<V> qF, Fst;
+    // Scratch within an evaluation or a transform, one block: `scr` holds the
+    // half-transformed fields of fft3 and of the fused evaluation; its last two
+    // fields are the sweeps' G and H (no fft3 runs during a sweep).
+    Buf<V> scr;
+    struct {
+        V* p = nullptr;
+    } G, H;
     Buf<double> part;    // reduction partials
     Buf<int> expo;       // propagator renormalisation exponents: forward [Nmax], backward [Nmax]
     Buf<T> si_G;         // semi-implicit linear-response coefficients G(k) (analytic): modes, then psi
@@ -1029,7 +1036,6 @@ struct Engine : EngineBase {
     Buf<float> pmax;     // per-CTA propagator maxima, two slots (ping-pong by segment parity)
     SplitGeom sg{};      // split-y passes of the chain sweeps (split_passes.cuh)
     Buf<V> split_tw;     // their twiddle tables
-    Buf<V> fscr;         // half-transformed fields between the two passes of fft3
     bool use_split = false;
     Buf<float> smax;     // their propagator maxima: per species, forward [N], backward [N]; zeroed by eval
     std::vector<size_t> smax0;   // first slot of each species
@@ -1090,12 +1096,12 @@ struct Engine : EngineBase {
         if (ev_installed) cudaEventDestroy(ev_installed);
         astage.release(); ostage.release();
         Buf<V>* vb[] = {&tw1, &tw2, &tw3, &omega, &psi, &omega_bar, &psi_bar, &drift, &drift_bar, &dpsi, &dpsi_bar,
-                        &kA, &kB, &dB, &kC, &rho_p, &rho_c, &ion_rho, &E, &qF, &Fst, &G, &H};
+                        &kA, &kB, &dB, &kC, &rho_p, &rho_c, &ion_rho, &E, &qF, &Fst, &scr};
         for (auto* b : vb) b->release();
         plans.release();
         kx.release(); ky.release(); kz.release(); phi.release(); gam.release(); gion.release(); eta.release();
         part.release(); spart.release(); stage.release(); expo.release(); pmax.release();
-        split_tw.release(); smax.release(); fscr.release();
+        split_tw.release(); smax.release();
         pair_ix.release(); pair_wt.release(); pair_run.release();
         si_G.release(); si_inc.release(); ck.release();
         avg.acc.release();
@@ -1189,7 +1195,7 @@ struct Engine : EngineBase {
         // may run under stream capture, where nothing can be allocated)
         if (c.scheme == FTSP_SCHEME_SI) upart.alloc(2 * (size_t)(use_split ? c.m1 * sg.Y2 : c.m1) * (nm + 1));   // most blocks of any tiling
         eta.alloc((size_t)(nm + 1) * Vn);
-        kA.alloc((size_t)2 * (nm + 1) * Vn);   // upper half: scratch of the fused evaluation's first pass
+        kA.alloc((size_t)(nm + 1) * Vn);
         kB.alloc((size_t)(M + 1 + J) * Vn);
         dB.alloc((size_t)(M + 1 + J) * Vn);
         kC.alloc((size_t)(M + 3) * Vn);
@@ -1199,7 +1205,18 @@ struct Engine : EngineBase {
         for (auto& s : c.sp) Nmax = std::max(Nmax, s.N);
         qF.alloc(Vn * Nmax);
         if (c.stress_on()) Fst.alloc(Vn * Nmax);
-        G.alloc(Vn); H.alloc(Vn);
+        {
+            // fft3 takes as many fields as its widest batch of an evaluation
+            // (those of the learned preconditioner, nm + 1 or 2, fit too), the
+            // fused evaluation two; a field starts on a 256-byte boundary
+            const int Jb = ion_common ? 1 : J;
+            const int before = eval_fused_ok() ? 2 : use_split ? std::max({M + 3, M + 1 + Jb, nm + 1}) - 2 : 0;
+            const size_t align = 256 / sizeof(V);
+            const size_t g = ((size_t)before * Vn + align - 1) / align * align, pitch = (Vn + align - 1) / align * align;
+            scr.alloc(g + pitch + Vn);
+            G.p = scr.p + g;
+            H.p = G.p + pitch;
+        }
         part.alloc((size_t)std::max(RED_BLOCKS, std::max(c.m1, c.m1 * c.m2)) * 32);
         expo.alloc((size_t)2 * Nmax);
         pmax.alloc((size_t)2 * std::max(c.m1, c.m1 * c.m2));
@@ -1210,9 +1227,6 @@ struct Engine : EngineBase {
         }
         smax.alloc(std::max<size_t>(1, slots));
         split_tw.alloc((size_t)3 * c.m1 + c.m2 + 2 * c.m3);
-        // as many fields as the widest batch of the evaluation that runs fft3
-        // (the learned preconditioner, the other user, allocates its own)
-        if (use_split && !eval_fused_ok()) fscr.alloc(Vn * (size_t)std::max({M + 3, M + 1 + J, nm + 1}));
         spart.alloc((size_t)c.m2 * c.m3 * 12);
         if (c.restart_interval > 0) ck.alloc((size_t)(std::max(1, c.nm) + 1) * V_);
         FTSP_CUDA(cudaMalloc(&ds, sizeof(DevScal)));
@@ -1813,7 +1827,6 @@ struct Engine : EngineBase {
         lr.nb = lr.batch / mlp::GRAD_THREADS;
         const size_t Vn = V_;
         lr.A.alloc(nf * Vn); lr.B.alloc(nf * Vn); lr.Pw.alloc(Vn); lr.Pp.alloc(Vn);
-        if (use_split && !fscr.p) fscr.alloc(std::max(nf, 2) * Vn);   // transforms of du and of the spectral powers
         lr.GL.alloc(nf * Vn); lr.dw.alloc(nf * Vn); lr.du.alloc(nf * Vn); lr.fk.alloc(2 * Vn);
         lr.w.alloc(lr.np); lr.m1.alloc(lr.np); lr.m2.alloc(lr.np);
         lr.partial.alloc((size_t)lr.nb * lr.np); lr.lpart.alloc(2 * (size_t)lr.nb); lr.loss.alloc(2);
@@ -2278,8 +2291,8 @@ struct Engine : EngineBase {
         cudaEvent_t ev = prof_begin();
         if (use_split) {
             // either sign runs the real-space pass first: natural order in and out
-            split_real<0, S>(nullptr, fscr.p, nf, in);
-            split_k<S, 0>(fscr.p, nullptr, nf, OpStore<T>{dst});
+            split_real<0, S>(nullptr, scr.p, nf, in);
+            split_k<S, 0>(scr.p, nullptr, nf, OpStore<T>{dst});
             prof_end(ev, "field_fft", 4.0 * nf * sizeof(V) * (double)V_);
             return;
         }
@@ -2772,13 +2785,13 @@ struct Engine : EngineBase {
         const bool elec = c.elec;
         const bool fx = eval_fused_ok();
         if (fx) {
-            // 1-2 fused: yz forward of omega and psi (into the scratch half of
-            // kA); one x-pencil pass: x forward, the k-space omega and psi
+            // 1-2 fused: yz forward of omega and psi (into the scratch fields);
+            // one x-pencil pass: x forward, the k-space omega and psi
             // stored in kA, W_type = gamma O Gamma omega / V, psi_s = Gamma
             // psi / V and the psi drift's k^2 psi / (4 pi l_B V) (from psi's
             // transform a second time), x inverse into kB; yz inverse
             cudaEvent_t ev = prof_begin();
-            V* kAx = kA.p + (size_t)(nm + 1) * Vn;
+            V* kAx = scr.p;
             OpLoadN<T> in{};
             in.s[0] = om;
             in.s[1] = ps;

@@ -1033,7 +1033,7 @@ struct Engine : EngineBase {
     Buf<T> si_G;         // semi-implicit linear-response coefficients G(k) (analytic): modes, then psi
     Buf<V> si_inc;       // semi-implicit increments (nm + 1 fields)
     Buf<V> ck;           // device checkpoint of (omega, psi) for rollback
-    Buf<float> pmax;     // per-CTA propagator maxima, two slots (ping-pong by segment parity)
+    Buf<float> pmax;     // run-time passes: per-CTA propagator maxima, two slots (ping-pong by segment parity)
     SplitGeom sg{};      // split-y passes of the chain sweeps (split_passes.cuh)
     Buf<V> split_tw;     // their twiddle tables
     bool use_split = false;
@@ -1219,13 +1219,13 @@ struct Engine : EngineBase {
         }
         part.alloc((size_t)std::max(RED_BLOCKS, std::max(c.m1, c.m1 * c.m2)) * 32);
         expo.alloc((size_t)2 * Nmax);
-        pmax.alloc((size_t)2 * std::max(c.m1, c.m1 * c.m2));
+        if (!use_split) pmax.alloc((size_t)2 * std::max(c.m1, c.m1 * c.m2));
         size_t slots = 0;
         for (auto& s : c.sp) {
             smax0.push_back(slots);
             slots += 2 * (size_t)s.N;
         }
-        smax.alloc(std::max<size_t>(1, slots));
+        smax.alloc(use_split ? slots : 0);
         split_tw.alloc((size_t)3 * c.m1 + c.m2 + 2 * c.m3);
         spart.alloc((size_t)c.m2 * c.m3 * 12);
         if (c.restart_interval > 0) ck.alloc((size_t)(std::max(1, c.nm) + 1) * V_);
@@ -2449,11 +2449,12 @@ struct Engine : EngineBase {
             r.nparts = nparts;
             r.s = s;
             r.N = N;
-            r.pmax_cur = pm(s);
-            r.pmax_prev = pm(s + 1);   // the pass before: segment s-1 (forward) or s+1 (backward), other parity
             if (use_split) {
                 r.pmax_cur = smax.p + smax0[isp] + s;
                 r.pmax_prev = r.pmax_cur - 1;
+            } else {
+                r.pmax_cur = pm(s);
+                r.pmax_prev = pm(s + 1);   // the pass before: segment s-1 (forward) or s+1 (backward), other parity
             }
             return r;
         };

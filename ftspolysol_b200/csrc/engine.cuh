@@ -1258,7 +1258,7 @@ struct Engine : EngineBase {
         }
     };
     struct TuneResult {
-        int max_bits = 0, W = 0, G = 0, cube = 0, candidates = 0;
+        int max_bits = 0, W = 0, G = 0, plane = 0, xct = 0, candidates = 0;
         double best_ms = 0.0, default_ms = 0.0;
         bool tuned = false, cached = false;
     };
@@ -1274,7 +1274,10 @@ struct Engine : EngineBase {
     }
     TuneResult tune{};
 
-    bool all_compile_time() const { return use_split && (sg.cube == 32 || sg.cube == 64 || sg.cube == 128); }
+    bool all_compile_time() const
+    {
+        return use_split && sg.plane == c.m1 && sg.xct == c.m1 && (c.m1 == 32 || c.m1 == 64 || c.m1 == 128);
+    }
 
     double time_fft(int reps)
     {
@@ -1307,13 +1310,14 @@ struct Engine : EngineBase {
         return (double)ms / reps;
     }
 
-    // other tiles for the split passes (cube: side of a compile-time plan, which
-    // brings its own tiles); false: they do not fit
-    bool retile(int groups, int W, int cube)
+    // other tiles for the split passes (plane, xct: the compile-time plans to run,
+    // which bring their own tiles); false: they do not fit
+    bool retile(int groups, int W, int plane, int xct)
     {
         SplitGeom g = sg;
         if (!split_tiles(g, (int)sizeof(V), groups, W)) return false;
-        g.cube = cube;
+        g.plane = plane;
+        g.xct = xct;
         sg = g;
         geo_W = W;
         return true;
@@ -1327,14 +1331,14 @@ struct Engine : EngineBase {
         if (it != tune_cache().end()) {
             tune = it->second;
             tune.cached = true;
-            if (use_split) retile(tune.G, tune.W, tune.cube);
+            if (use_split) retile(tune.G, tune.W, tune.plane, tune.xct);
             else setup_geometry(tune.max_bits, tune.W);
             return;
         }
         TuneResult r{};
         if (all_compile_time()) {   // the tiles it has: the next handle of the grid takes them from the cache
             r.max_bits = geo_max_bits;
-            r.W = geo_W; r.G = sg.G; r.cube = sg.cube;
+            r.W = geo_W; r.G = sg.G; r.plane = sg.plane; r.xct = sg.xct;
             tune_cache()[key] = r;
             tune = r;
             return;
@@ -1343,20 +1347,20 @@ struct Engine : EngineBase {
         if (use_split) {
             FTSP_CUDA(cudaMemsetAsync(E.p, 0, sizeof(V) * V_, stream));
             r.max_bits = geo_max_bits;
-            r.W = sg.W; r.G = sg.G; r.cube = sg.cube;
+            r.W = sg.W; r.G = sg.G; r.plane = sg.plane; r.xct = sg.xct;
             r.best_ms = r.default_ms = time_fft(3);
             const int G0 = sg.G;
             for (int g : {G0, G0 > 1 ? 1 : 2})
                 for (int bytes : {32, 64, 128}) {
-                    if (sg.Y2 % g || !retile(g, std::max(1, bytes / (int)sizeof(V)), 0)) continue;
+                    if (sg.Y2 % g || !retile(g, std::max(1, bytes / (int)sizeof(V)), 0, 0)) continue;
                     const double t = time_fft(3);
                     ++r.candidates;
                     if (t < r.best_ms) {
                         r.best_ms = t;
-                        r.W = sg.W; r.G = g; r.cube = 0;
+                        r.W = sg.W; r.G = g; r.plane = r.xct = 0;
                     }
                 }
-            retile(r.G, r.W, r.cube);
+            retile(r.G, r.W, r.plane, r.xct);
             r.tuned = true;
             tune_cache()[key] = r;
             tune = r;

@@ -56,7 +56,8 @@ struct SplitGeom {
     int m1, m2, m3;
     int ok;                  // the extents factor (see split_setup)
     int big_r, big_k;        // passes with radices that need RtBigPlan
-    int cube;                // side of the CubePlan to run, 0: a run-time plan
+    int plane;               // side of the yz plane whose compile-time real-space plan runs, 0: a run-time plan
+    int xct;                 // x extent whose compile-time k-space plan runs, 0: a run-time plan
     int Y1, Y2;
     // real-space pass: m3 = zA * zB, G row groups (y0 .. y0 + G - 1) per block
     int zA, zB, G, rows;     // rows = G * Y1
@@ -187,16 +188,20 @@ constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes
             g.Y2 = t;
         }
     }
+    // compile-time plans: the square planes of the production cubes, with any x
+    // extent; the x extents of the cubes, with their plane or (32, 64, 128) any
+    // rows of 4 or 8 and whole tiles
+    g.plane = m2 == m3 && (m3 == 32 || m3 == 48 || m3 == 64 || m3 == 96 || m3 == 128) ? m3 : 0;
+    g.xct = g.plane == m1 ? m1 : (m1 == 32 || m1 == 64 || m1 == 128) && (g.Y2 == 4 || g.Y2 == 8) && m3 % 4 == 0 ? m1 : 0;
     // real space: as many row groups per block as leave two blocks per SM
     int G = 1;
-    for (int t = 2; t <= g.Y2; ++t)
+    for (int t = 2; t <= g.Y2 && !g.plane; ++t)
         if (g.Y2 % t == 0 && m1 * (g.Y2 / t) >= 296 && t * g.Y1 * m3 <= 1024 && t * split_max(g.Y1 * g.zA, m3) <= 256) G = t;
     // k space: 32 bytes of every row (one memory sector)
     int W = split_max(1, 32 / value_bytes);
     while (W > 1 && (W / 2 >= m3 || (long long)m1 * g.Y2 * W * value_bytes > 72 * 1024)) W /= 2;
     g.big_r = g.zA > 16 || g.zB > 10 || g.Y1 > 16;
     g.big_k = g.xA > 16 || g.xB > 10 || g.Y2 > 16;
-    g.cube = m1 == m2 && m2 == m3 && (m1 == 32 || m1 == 48 || m1 == 64 || m1 == 96 || m1 == 128) ? m1 : 0;
     g.ok = split_tiles(g, value_bytes, G, W) ? 1 : 0;
     return g.ok != 0;
 }
@@ -205,7 +210,7 @@ constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes
 // RtPlan takes everything from the geometry argument, gives a thread one
 // butterfly per phase and exchanges between two buffers (one barrier each).
 struct RtPlan {
-    static constexpr bool CT = false;
+    static constexpr bool CT = false, PLANE = false;
     static constexpr bool INPLACE = false;
     static constexpr SplitGeom G = SplitGeom{};
     static constexpr int RNT = 256, KNT = SPLIT_NT;
@@ -228,22 +233,53 @@ constexpr int split_nt(int base, int a, int b)   // threads: a phase of `base` b
     const int nt = split_round32(base);
     return a % nt == 0 && b % nt == 0 ? nt : split_round32(split_max(base, split_max(a, b)));
 }
-constexpr SplitGeom split_cube(int n, int value_bytes)
+constexpr SplitGeom split_box(int m1, int n, int value_bytes)   // m1 planes of n x n points
 {
     SplitGeom g{};
-    split_setup(g, n, n, n, value_bytes);
+    split_setup(g, m1, n, n, value_bytes);
     g.r_threads = split_nt(split_max(g.rows * g.zB, g.G * n), g.rows * g.zA, g.rows * g.zA);
-    g.k_threads = split_nt(g.C * g.xB, g.C * g.xA, n * g.W);
+    g.k_threads = split_nt(g.C * g.xB, g.C * g.xA, m1 * g.W);
     return g;
 }
+constexpr SplitGeom split_cube(int n, int value_bytes) { return split_box(n, n, value_bytes); }
+// The real-space pass takes it for any number of N x N planes (it uses m1 for
+// nothing but its grid).
 template <int N, typename T>
 struct CubePlan {
-    static constexpr bool CT = true;
+    static constexpr bool CT = true, PLANE = true;
     static constexpr bool INPLACE = true;
     static constexpr SplitGeom G = split_cube(N, 2 * (int)sizeof(T));
     static constexpr int RNT = G.r_threads, KNT = G.k_threads;
     static constexpr int AMAX = 16, BMAX = 10;
     template <typename T2> static constexpr int rmin = 1;
+    static_assert(G.G == 1, "one row group per block on every grid with this plane");
+};
+// The k-space pass of m1 = X points along x and rows of Y2 = 4 or 8 at compile
+// time, m2, m3 and Y1 from the geometry argument (m3 a multiple of the tile
+// width).
+template <int X, int Y2, typename T>
+struct XPlan {
+    static constexpr bool CT = true, PLANE = false;
+    static constexpr bool INPLACE = true;
+    // Threads: as in the cubes, but a thread per butterfly of the widest phase
+    // where a thread had four of a phase or 256 bytes of values (steps with
+    // N = 16, the cubes' rule and this one: 128 x 32 x 32 complex64 617 and 384
+    // us, complex128 739 and 571, 128 x 64 x 64 complex128 1225 and 1026; the
+    // others lose by it: 128 x 64 x 64 complex64 736 and 849, 32 x 64 x 64 344
+    // and 362)
+    static constexpr SplitGeom threads(SplitGeom g)
+    {
+        const int nt = g.k_threads, widest = split_max(g.C * g.xA, g.m1 * g.W);
+        const int rows = (g.m1 * g.W + nt - 1) / nt, mid = (g.C * g.xA + nt - 1) / nt;
+        const int values = split_max(split_max(rows * g.Y2, mid * g.xB), (g.C * g.xB + nt - 1) / nt * g.xA);
+        if (split_max(rows, mid) >= 4 || values * 2 * (int)sizeof(T) >= 256) g.k_threads = split_round32(widest);
+        return g;
+    }
+    static constexpr SplitGeom G = threads(split_box(X, Y2 == 4 ? 32 : 64, 2 * (int)sizeof(T)));
+    static constexpr int RNT = G.r_threads, KNT = G.k_threads;
+    static constexpr int AMAX = 16, BMAX = 10;
+    template <typename T2> static constexpr int rmin = 1;
+    static_assert(G.Y2 == Y2 && G.m1 == X, "representative grid");
 };
 
 // Values of the twiddle tables, in the order tza, tzb, txa, txb, ty, tx
@@ -533,6 +569,8 @@ __device__ __forceinline__ void split_phase(int items, Ga gather, Fi finish)
 
 // geometry member: a constant of the plan, or the kernel argument's
 #define FTSP_PL(m) (P::CT ? P::G.m : g.m)
+// the same of the members that depend on the yz plane
+#define FTSP_PP(m) (P::PLANE ? P::G.m : g.m)
 // quotient by a geometry member with its magic-number divisor
 #define FTSP_DIV(i, m, f) (P::CT ? (int)((unsigned)(i) / (unsigned)split_max(1, P::G.m)) : (int)fdiv(i, g.f))
 
@@ -775,8 +813,8 @@ __global__ void __launch_bounds__(P::KNT, split_min_blocks<P, T, Op>(P::KNT))
     constexpr int NT = P::KNT;
     constexpr bool IP = P::INPLACE;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int m1 = FTSP_PL(m1), m2 = FTSP_PL(m2), m3 = FTSP_PL(m3), Y1 = FTSP_PL(Y1), Y2 = FTSP_PL(Y2), xA = FTSP_PL(xA), xB = FTSP_PL(xB);
-    const int W = FTSP_PL(W), C = FTSP_PL(C), pc = FTSP_PL(pc), kt = FTSP_PL(kt), nzb = FTSP_PL(nzb);
+    const int m1 = FTSP_PL(m1), m2 = FTSP_PP(m2), m3 = FTSP_PP(m3), Y1 = FTSP_PP(Y1), Y2 = FTSP_PL(Y2), xA = FTSP_PL(xA), xB = FTSP_PL(xB);
+    const int W = FTSP_PL(W), C = FTSP_PL(C), pc = FTSP_PL(pc), kt = FTSP_PL(kt), nzb = FTSP_PP(nzb);
     const int nthr = P::CT ? NT : (int)blockDim.x;
     V* b0 = reinterpret_cast<V*>(smem_raw);
     V* b1 = IP ? b0 : b0 + kt;
@@ -784,7 +822,7 @@ __global__ void __launch_bounds__(P::KNT, split_min_blocks<P, T, Op>(P::KNT))
     V* tb = ta + m1;
     const int tid = threadIdx.x;
     const int f = blockIdx.y;
-    const int k1 = FTSP_DIV(blockIdx.x, nzb, fnzb);
+    const int k1 = P::PLANE ? (int)(blockIdx.x / (unsigned)split_max(1, P::G.nzb)) : (int)fdiv(blockIdx.x, g.fnzb);
     const int z0 = (blockIdx.x - k1 * nzb) * W;
     const size_t plane = (size_t)m2 * m3;
     const size_t inner = (size_t)k1 * Y2 * m3 + z0;
@@ -792,7 +830,7 @@ __global__ void __launch_bounds__(P::KNT, split_min_blocks<P, T, Op>(P::KNT))
     V* dp = dst + (size_t)f * fstride + inner;
     const size_t fbase = (size_t)f * fstride;
     // the last tile of a row may be partial
-    const bool whole = P::CT ? P::G.m3 % split_max(1, P::G.W) == 0 : false;
+    const bool whole = P::CT ? !P::PLANE || P::G.m3 % split_max(1, P::G.W) == 0 : false;
     for (int j = tid; j < m1; j += nthr) {
         ta[j] = reinterpret_cast<const V*>(g.txa)[j];
         tb[j] = reinterpret_cast<const V*>(g.txb)[j];
@@ -911,6 +949,7 @@ __global__ void __launch_bounds__(P::KNT, split_min_blocks<P, T, Op>(P::KNT))
 }
 
 #undef FTSP_PL
+#undef FTSP_PP
 #undef FTSP_DIV
 
 // The k-space pass of a cube with m1 = XP * XQ in two exchanges instead of
@@ -1078,7 +1117,7 @@ cudaError_t split_real_plan(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst
                             cudaStream_t stream)
 {
     const SplitGeom& p = P::CT ? P::G : g;
-    return split_launch(k_split_real<T, P, S1, S2, Op>, dim3(p.m1 * (p.Y2 / p.G), nf), p.r_threads,
+    return split_launch(k_split_real<T, P, S1, S2, Op>, dim3(g.m1 * (p.Y2 / p.G), nf), p.r_threads,
                         split_real_smem<P, cplx<T>>(p), stream, g, src, dst, fstride, op);
 }
 template <class P, typename T, int S1, int S2, class Op>
@@ -1086,28 +1125,29 @@ cudaError_t split_k_plan(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst, s
                          cudaStream_t stream)
 {
     const SplitGeom& p = P::CT ? P::G : g;
-    return split_launch(k_split_k<T, P, S1, S2, Op>, dim3(p.Y1 * p.nzb, nf), p.k_threads, split_k_smem<P, cplx<T>>(p),
-                        stream, g, src, dst, fstride, op);
+    SplitGeom a = g;
+    if (P::CT) {   // its tile width, not the one of the run-time plans
+        a.nzb = g.m3 / p.W;
+        a.fnzb = make_fastdiv(a.nzb);
+    }
+    return split_launch(k_split_k<T, P, S1, S2, Op>, dim3(g.Y1 * a.nzb, nf), p.k_threads, split_k_smem<P, cplx<T>>(p),
+                        stream, a, src, dst, fstride, op);
 }
 // blocks of one field of the real-space pass
 inline int split_real_blocks(const SplitGeom& g) { return g.m1 * (g.Y2 / g.G); }
 
-// The production cubes run their compile-time plans (where g says so); passes
-// with one transform (the ends of a sweep, the field transforms) only at 96 and
-// 128, where they are not a matter of launch latency.
+// The planes and x extents of the production cubes run their compile-time plans
+// (where g says so); real-space passes with one transform (the ends of a sweep,
+// the field transforms) only at 96 and 128, where they are not a matter of
+// launch latency.
 template <typename T, int S1, int S2, class Op>
 cudaError_t split_real_launch(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst, size_t fstride, int nf, const Op& op,
                               cudaStream_t stream)
 {
-    if constexpr (S1 != 0 && S2 != 0) switch (g.cube) {
+    switch (g.plane) {
         case 32: return split_real_plan<CubePlan<32, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
         case 48: return split_real_plan<CubePlan<48, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
         case 64: return split_real_plan<CubePlan<64, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
-        case 96: return split_real_plan<CubePlan<96, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
-        case 128: return split_real_plan<CubePlan<128, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
-        default: break;
-    }
-    else switch (g.cube) {
         case 96: return split_real_plan<CubePlan<96, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
         case 128: return split_real_plan<CubePlan<128, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
         default: break;
@@ -1126,13 +1166,27 @@ template <typename T, int S1, int S2, class Op>
 cudaError_t split_k_launch(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst, size_t fstride, int nf, const Op& op,
                            cudaStream_t stream)
 {
-    if constexpr (S1 != 0 && S2 != 0) switch (g.cube) {
-        case 32: return split_k_plan<CubePlan<32, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
-        case 48: return split_k_plan<CubePlan<48, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
-        case 64: return split_k_plan<CubePlan<64, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
-        case 96: return cube_k<96, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
-        case 128: return cube_k<128, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
-        default: break;
+    if constexpr (S1 != 0 && S2 != 0) {
+        if (g.plane == g.xct) switch (g.xct) {   // cubes
+            case 32: return split_k_plan<CubePlan<32, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            case 48: return split_k_plan<CubePlan<48, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            case 64: return split_k_plan<CubePlan<64, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            case 96: return cube_k<96, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            case 128: return cube_k<128, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            default: break;
+        }
+        if (g.xct && g.Y2 == 4) switch (g.xct) {
+            case 32: return split_k_plan<XPlan<32, 4, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            case 64: return split_k_plan<XPlan<64, 4, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            case 128: return split_k_plan<XPlan<128, 4, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            default: break;
+        }
+        if (g.xct && g.Y2 == 8) switch (g.xct) {
+            case 32: return split_k_plan<XPlan<32, 8, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            case 64: return split_k_plan<XPlan<64, 8, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            case 128: return split_k_plan<XPlan<128, 8, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            default: break;
+        }
     }
     if (g.big_k) return split_k_plan<RtBigPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
     return split_k_plan<RtPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);

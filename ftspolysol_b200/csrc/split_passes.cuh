@@ -155,9 +155,6 @@ constexpr bool split_tiles(SplitGeom& g, int value_bytes, int G, int W)
     g.C = g.Y2 * g.W;
     g.k_threads = split_round32(split_max(g.C * g.xA, m1 * g.W));
     if (g.k_threads > SPLIT_NT) g.k_threads = SPLIT_NT;
-    // both buffers of both passes within the shared memory of a block
-    if ((2LL * g.rt + 2 * m3 + g.rows) * value_bytes > 225 * 1024 || (2LL * m1 * (g.C + banks) + 2 * m1) * value_bytes > 225 * 1024)
-        return false;
     best = 1 << 30;
     for (int p = g.C; p < g.C + banks; ++p) {
         const int c = bank_cost(64, banks, g.W, p, 1) + bank_cost(64, banks, g.C, p, 1) +
@@ -168,6 +165,8 @@ constexpr bool split_tiles(SplitGeom& g, int value_bytes, int G, int W)
         }
     }
     g.kt = m1 * g.pc;
+    // both buffers of both passes within the shared memory of a block
+    if ((2LL * g.rt + 2 * m3 + g.rows) * value_bytes > 225 * 1024 || (2LL * g.kt + 2 * m1) * value_bytes > 225 * 1024) return false;
     g.nzb = (m3 + g.W - 1) / g.W;
     g.fC = make_fastdiv(g.C); g.fW = make_fastdiv(g.W); g.fnzb = make_fastdiv(g.nzb);
     return true;
@@ -202,8 +201,13 @@ constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes
     while (W > 1 && (W / 2 >= m3 || (long long)m1 * g.Y2 * W * value_bytes > 72 * 1024)) W /= 2;
     g.big_r = g.zA > 16 || g.zB > 10 || g.Y1 > 16;
     g.big_k = g.xA > 16 || g.xB > 10 || g.Y2 > 16;
-    g.ok = split_tiles(g, value_bytes, G, W) ? 1 : 0;
-    return g.ok != 0;
+    // narrower tiles of a long x
+    while (!split_tiles(g, value_bytes, G, W)) {
+        if (W == 1) return false;
+        W /= 2;
+    }
+    g.ok = 1;
+    return true;
 }
 
 // ---- plans ----
@@ -1137,9 +1141,7 @@ cudaError_t split_k_plan(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst, s
 inline int split_real_blocks(const SplitGeom& g) { return g.m1 * (g.Y2 / g.G); }
 
 // The planes and x extents of the production cubes run their compile-time plans
-// (where g says so); real-space passes with one transform (the ends of a sweep,
-// the field transforms) only at 96 and 128, where they are not a matter of
-// launch latency.
+// (where g says so); the k-space half of the plain transforms is run-time.
 template <typename T, int S1, int S2, class Op>
 cudaError_t split_real_launch(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst, size_t fstride, int nf, const Op& op,
                               cudaStream_t stream)

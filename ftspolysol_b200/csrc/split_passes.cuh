@@ -1190,6 +1190,13 @@ cudaError_t split_k_launch(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst,
             default: break;
         }
     }
+    if constexpr (S1 != 0 && S2 == 0) {
+        if (g.plane == g.xct) switch (g.xct) {
+            case 96: return split_k_plan<CubePlan<96, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            case 128: return split_k_plan<CubePlan<128, T>, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
+            default: break;
+        }
+    }
     if (g.big_k) return split_k_plan<RtBigPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
     return split_k_plan<RtPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
 }

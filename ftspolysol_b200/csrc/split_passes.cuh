@@ -50,12 +50,13 @@
 namespace ftsp {
 
 constexpr int SPLIT_NT = 512;   // largest block
+constexpr int SPLIT_NT_HUGE = 256;   // of RtHugePlan
 constexpr int SPLIT_RADICES[] = {1, 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 24, 25, 32};
 
 struct SplitGeom {
     int m1, m2, m3;
     int ok;                  // the extents factor (see split_setup)
-    int big_r, big_k;        // passes with radices that need RtBigPlan
+    int big_r, big_k;        // passes with radices that need RtBigPlan (1) or RtHugePlan (2)
     int plane;               // side of the yz plane whose compile-time real-space plan runs, 0: a run-time plan
     int xct;                 // x extent whose compile-time k-space plan runs, 0: a run-time plan
     int Y1, Y2;
@@ -83,10 +84,11 @@ constexpr bool split_radix(int r)
     return false;
 }
 // n = a * b, a >= b, as even as possible, a at most amax, b at most bmax
-constexpr bool split_pair(int n, int amax, int bmax, int& a, int& b)
+constexpr bool split_pair(int n, int amax, int bmax, int& a, int& b, bool with27 = false)
 {
     for (int x = 1; x <= amax; ++x)
-        if (n % x == 0 && x * x >= n && n / x <= bmax && split_radix(x) && split_radix(n / x)) {
+        if (n % x == 0 && x * x >= n && n / x <= bmax && (split_radix(x) || (with27 && x == 27)) &&
+            (split_radix(n / x) || (with27 && n / x == 27))) {
             a = x;
             b = n / x;
             return true;
@@ -154,7 +156,8 @@ constexpr bool split_tiles(SplitGeom& g, int value_bytes, int G, int W)
     g.W = W;
     g.C = g.Y2 * g.W;
     g.k_threads = split_round32(split_max(g.C * g.xA, m1 * g.W));
-    if (g.k_threads > SPLIT_NT) g.k_threads = SPLIT_NT;
+    const int most = g.big_k == 2 ? SPLIT_NT_HUGE : SPLIT_NT;
+    if (g.k_threads > most) g.k_threads = most;
     best = 1 << 30;
     for (int p = g.C; p < g.C + banks; ++p) {
         const int c = bank_cost(64, banks, g.W, p, 1) + bank_cost(64, banks, g.C, p, 1) +
@@ -176,12 +179,21 @@ constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes
 {
     g.m1 = m1; g.m2 = m2; g.m3 = m3;
     g.ok = 0;
+    const bool square = m2 == m3 && (m3 == 32 || m3 == 48 || m3 == 64 || m3 == 96 || m3 == 128);
+    g.big_k = 0;
     // the butterfly pair around the op (radix B) holds the op's operands
-    // beside its values: 10 at most, except in RtBigPlan
+    // beside its values: 10 at most, except in RtBigPlan and RtHugePlan
     if (!split_pair(m3, 16, 10, g.zA, g.zB) || !split_pair(m1, 16, 10, g.xA, g.xB) || !split_pair(m2, 16, 16, g.Y1, g.Y2)) {
-        if (!split_pair(m3, 32, 16, g.zA, g.zB) || !split_pair(m1, 32, 16, g.xA, g.xB) || !split_pair(m2, 32, 16, g.Y1, g.Y2))
-            return false;
-        if (g.Y1 > 16) {   // the long half of y in the pass whose tiles are narrower
+        if (!split_pair(m3, 32, 16, g.zA, g.zB) || !split_pair(m1, 32, 16, g.xA, g.xB) || !split_pair(m2, 32, 16, g.Y1, g.Y2)) {
+            // two radices above 16, or 27, along x only, where the real-space
+            // pass has a compile-time plan (steps with N = 16, with it and with
+            // the run-time passes: 243 x 32 x 32 complex64 0.78 and 2.5 ms, 640 x
+            // 64 x 64 complex128 7.3 and 13.6)
+            if (!square || !split_pair(m3, 16, 10, g.zA, g.zB) || !split_pair(m1, 32, 32, g.xA, g.xB, true) ||
+                !split_pair(m2, 16, 16, g.Y1, g.Y2))
+                return false;
+            g.big_k = 2;
+        } else if (g.Y1 > 16) {   // the long half of y in the pass whose tiles are narrower
             const int t = g.Y1;
             g.Y1 = g.Y2;
             g.Y2 = t;
@@ -190,7 +202,7 @@ constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes
     // compile-time plans: the square planes of the production cubes, with any x
     // extent; the x extents of the cubes, with their plane or (32, 64, 128) any
     // rows of 4 or 8 and whole tiles
-    g.plane = m2 == m3 && (m3 == 32 || m3 == 48 || m3 == 64 || m3 == 96 || m3 == 128) ? m3 : 0;
+    g.plane = square ? m3 : 0;
     g.xct = g.plane == m1 ? m1 : (m1 == 32 || m1 == 64 || m1 == 128) && (g.Y2 == 4 || g.Y2 == 8) && m3 % 4 == 0 ? m1 : 0;
     // real space: as many row groups per block as leave two blocks per SM
     int G = 1;
@@ -200,7 +212,7 @@ constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes
     int W = split_max(1, 32 / value_bytes);
     while (W > 1 && (W / 2 >= m3 || (long long)m1 * g.Y2 * W * value_bytes > 72 * 1024)) W /= 2;
     g.big_r = g.zA > 16 || g.zB > 10 || g.Y1 > 16;
-    g.big_k = g.xA > 16 || g.xB > 10 || g.Y2 > 16;
+    if (!g.big_k) g.big_k = g.xA > 16 || g.xB > 10 || g.Y2 > 16;
     // narrower tiles of a long x
     while (!split_tiles(g, value_bytes, G, W)) {
         if (W == 1) return false;
@@ -227,6 +239,14 @@ struct RtPlan {
 // keep their registers.
 struct RtBigPlan : RtPlan {
     static constexpr int AMAX = 32, BMAX = 16;
+    template <typename T> static constexpr int rmin = 1;
+};
+// The k-space pass of x extents with two radices above 16 or one of 27 (486 = 27
+// x 18, 640 = 32 x 20): a thread holds up to 32 points and the op's operands, so
+// blocks are half as large.
+struct RtHugePlan : RtPlan {
+    static constexpr int KNT = SPLIT_NT_HUGE;
+    static constexpr int AMAX = 33, BMAX = 33;
     template <typename T> static constexpr int rmin = 1;
 };
 // A cube of N points a side at compile time.  One buffer: a phase reads,
@@ -430,6 +450,42 @@ __device__ __forceinline__ void dft25(V* u)
     }
 }
 
+// 27 = 9 x 3 with the twiddles w27^(j k)
+template <int S, typename V>
+__device__ __forceinline__ void dft27(V* u)
+{
+    using R = typename RealOf<V>::type;
+    // cos and sin of 2 pi j / 27 for the products j = 0 .. 16
+    constexpr double c[17] = {1.0, 0.97304487057982383883, 0.89363264032341224819, 0.7660444431189780352,
+                              0.59715859170278616485, 0.3960797660391568237, 0.17364817766693034885,
+                              -0.058144828910475828539, -0.2868032327110902531, -0.5, -0.68624163786873358573,
+                              -0.83548781141293641965, -0.93969262078590838405, -0.99323835774194298855,
+                              -0.99323835774194298855, -0.93969262078590838405, -0.83548781141293641965};
+    constexpr double sn[17] = {0.0, 0.23061587074244017845, 0.44879918020046217279, 0.64278760968653932632,
+                               0.80212319275504378508, 0.91821610688027401476, 0.98480775301220805937,
+                               0.99830815827126820805, 0.95798951231548887444, 0.86602540378443864676,
+                               0.72737364157304869599, 0.54950897807080603526, 0.34202014332566873304,
+                               0.11609291412523022968, -0.11609291412523022968, -0.34202014332566873304,
+                               -0.54950897807080603526};
+    V a[3][9];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) a[j][k] = u[j + 3 * k];
+        dft9<S>(a[j]);
+#pragma unroll
+        for (int k = 1; k < 9; ++k)
+            if (j > 0) a[j][k] = crot<S>(a[j][k], R(c[j * k]), R(sn[j * k]));
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        V b[3] = {a[0][k], a[1][k], a[2][k]};
+        dft3<S>(b);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) u[k + 9 * t] = b[t];
+    }
+}
+
 // cos(2 pi m / 32)
 __host__ __device__ constexpr double cos32(int m)
 {
@@ -483,6 +539,7 @@ __device__ __forceinline__ void dft_any(V* u)
     else if constexpr (R == 20) dft_coprime<S, 4, 5>(u);
     else if constexpr (R == 24) dft_coprime<S, 8, 3>(u);
     else if constexpr (R == 25) dft25<S>(u);
+    else if constexpr (R == 27) dft27<S>(u);
     else if constexpr (R == 32) dft32<S>(u);
     else dftR<S, R>(u);
 }
@@ -521,6 +578,9 @@ __device__ __forceinline__ void by_radix(int r, F&& f)
                 else if (r == 24) f(RadixTag<24>{});
                 else if (r == 25) f(RadixTag<25>{});
                 else if (r == 32) f(RadixTag<32>{});
+            }
+            if constexpr (MAX > 32) {
+                if (r == 27) f(RadixTag<27>{});
             }
             break;
         }
@@ -1197,6 +1257,7 @@ cudaError_t split_k_launch(const SplitGeom& g, const cplx<T>* src, cplx<T>* dst,
             default: break;
         }
     }
+    if (g.big_k == 2) return split_k_plan<RtHugePlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
     if (g.big_k) return split_k_plan<RtBigPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
     return split_k_plan<RtPlan, T, S1, S2>(g, src, dst, fstride, nf, op, stream);
 }

@@ -3,7 +3,7 @@ square planes of the production cubes with other x extents (one row, odd,
 large), the x extents 32, 64 and 128 with rows of 4 and 8 and whole tiles of
 columns, and their neighbours that must take the run-time plans (m3 no
 multiple of 4, rows of 6); x extents so long that the tiles of the k-space pass
-get narrower.
+get narrower; x extents with two radices above 16 or one of 27.
 
 Chain propagation against numpy FFTs (complex128, 1e-12 of the field's largest
 modulus), densities and record of an asymmetric chain (both sweeps, stress
@@ -22,7 +22,9 @@ pytestmark = pytest.mark.gpu
 
 CHAINS = [(64, 32, 32), (128, 32, 32), (1, 32, 32), (45, 32, 32), (256, 32, 32), (32, 64, 64), (125, 64, 64), (128, 64, 64),
           (10, 48, 48), (27, 96, 96), (2, 128, 128), (64, 128, 128), (32, 20, 12), (64, 16, 4), (128, 24, 20), (32, 80, 8),
-          (64, 40, 36), (128, 72, 12), (32, 20, 15), (64, 48, 20), (128, 36, 8), (512, 32, 32), (512, 30, 8), (480, 64, 6), (400, 120, 4)]
+          (64, 40, 36), (128, 72, 12), (32, 20, 15), (64, 48, 20), (128, 36, 8), (512, 32, 32), (512, 30, 8), (480, 64, 6), (400, 120, 4),
+          (243, 32, 32), (324, 48, 48), (486, 32, 32), (500, 32, 32), (576, 32, 32), (625, 32, 32), (640, 32, 32), (729, 32, 32),
+          (800, 32, 32)]
 
 
 @pytest.mark.parametrize("m", CHAINS, ids=lambda m: "%dx%dx%d" % m)
@@ -41,7 +43,8 @@ def test_chain(m):
     assert abs(Q - ref.mean()) / abs(ref.mean()) < 1e-12
 
 
-@pytest.mark.parametrize("m", [(64, 32, 32), (32, 64, 64), (20, 64, 64), (128, 16, 12), (3, 128, 128), (5, 96, 96), (512, 30, 8)],
+@pytest.mark.parametrize("m", [(64, 32, 32), (32, 64, 64), (20, 64, 64), (128, 16, 12), (3, 128, 128), (5, 96, 96), (512, 30, 8), (243, 32, 32),
+                               (640, 32, 32)],
                          ids=lambda m: "%dx%dx%d" % m)
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_both_sweeps(m, prec):

@@ -1681,10 +1681,10 @@ struct Engine : EngineBase {
         prof_end(ev, "field_fft", units * sizeof(V) * (double)Vn);
         if (corr) {
             for (int f = 0; f < nf; ++f) {
-                launch_pass(k_combine<true>, dim3(1), COMBINE_THREADS, 0, (const double*)(upart.p + (size_t)f * fparts), (int)(fparts), 1, (double*)(ds->dmax + f));
+                launch_pass(k_combine<true>, dim3(1), COMBINE_THREADS, 0, upart.p + (size_t)f * fparts, fparts, 1, ds->dmax + f);
                 ++launches;
             }
-            launch_pass(k_combine<false>, dim3(1), COMBINE_THREADS, 0, (const double*)(upart.p + nparts), (int)((int)nparts), 1, (double*)(ds->corr + 2));
+            launch_pass(k_combine<false>, dim3(1), COMBINE_THREADS, 0, upart.p + nparts, (int)nparts, 1, ds->corr + 2);
             ++launches;
         }
     }
@@ -2226,14 +2226,9 @@ struct Engine : EngineBase {
     // ---- pass launchers ----
     // Launches a pass kernel with programmatic dependent launch (the kernel
     // waits for its predecessor with griddepcontrol.wait).
-    bool use_pdl = true;
     template <class K, class... Args>
     void launch_pass(K kernel, dim3 grid, int threads, size_t smem, Args... args)
     {
-        if (!use_pdl) {
-            kernel<<<grid, threads, smem, stream>>>(args...);
-            return;
-        }
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = grid;
         cfg.blockDim = dim3(threads);
@@ -2507,7 +2502,7 @@ struct Engine : EngineBase {
             DevScal* d = ds;
             const int* eF = expo.p;
             const int last = N - 1;
-            launch_pass(k_combine<false>, dim3(2), COMBINE_THREADS, 0, (const double*)(qpart), (int)(cnt), 2, (double*)(reinterpret_cast<double*>(&d->Q[isp])));
+            launch_pass(k_combine<false>, dim3(2), COMBINE_THREADS, 0, qpart, cnt, 2, reinterpret_cast<double*>(&d->Q[isp]));
             one_warp(1, [=] __device__(size_t) {
                 const double2 Qs = dscale(d->Q[isp], invV);
                 d->factor[isp] = dscale(dinv(Qs), nv);
@@ -3556,7 +3551,7 @@ struct Engine : EngineBase {
     void finalize_record(bool with_stress)
     {
         if (with_stress) {
-            launch_pass(k_combine<false>, dim3(12), COMBINE_THREADS, 0, (const double*)(spart.p), (int)(stress_parts()), 12, (double*)(ds->sconn));
+            launch_pass(k_combine<false>, dim3(12), COMBINE_THREADS, 0, spart.p, stress_parts(), 12, ds->sconn);
             ++launches;
         }
         const int S = (int)c.sp.size(), J = (int)c.ions.size(), nm = c.nm;
@@ -4341,7 +4336,7 @@ struct Engine : EngineBase {
             }
         }
         double* out = reinterpret_cast<double*>(&ds->Q[0]);
-        launch_pass(k_combine<false>, dim3(2), COMBINE_THREADS, 0, (const double*)(part.p), (int)(seg_pass_ctas()), 2, (double*)(out));
+        launch_pass(k_combine<false>, dim3(2), COMBINE_THREADS, 0, part.p, seg_pass_ctas(), 2, out);
         ++launches;
         double q[2];
         FTSP_CUDA(cudaMemcpyAsync(q, out, sizeof(q), cudaMemcpyDeviceToHost, stream));

@@ -321,8 +321,7 @@ inline std::vector<V> split_tables(const SplitGeom& g, Tw tw)
     put(g.m1, g.xA, g.xB);
     put(g.m1, g.xB, g.xA);
     put(g.m2, g.Y1, g.Y2);
-    put(g.m1, g.m1, 2);
-    t.erase(t.end() - 2 * g.m1, t.end() - g.m1);   // the row of first powers
+    for (int j = 0; j < g.m1; ++j) t.push_back(tw(g.m1, j));
     return t;
 }
 template <class V>

@@ -172,9 +172,9 @@ def step_roofline(prop_bytes, field, steps, npts, s_c, steps_per_s_gpu, peak):
 
 def committed_traffic():
     """Per-launch DRAM bytes of the propagator passes from the committed ncu
-    summary (profiles/propagator_passes_128cube_N50.md, lines 'traffic <kind> <bytes>')."""
+    summary (profiles/split_passes_128cube.md, lines 'traffic <kind> <bytes>')."""
     out = {}
-    path = os.path.join(ROOT, "profiles", "propagator_passes_128cube_N50.md")
+    path = os.path.join(ROOT, "profiles", "split_passes_128cube.md")
     if os.path.exists(path):
         for line in open(path):
             p = line.split()

@@ -1128,7 +1128,8 @@ struct Engine : EngineBase {
         if (bytes > 48 * 1024) FTSP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     }
 
-    // Launch geometry of the runtime-plan passes.  max_bits: largest
+    // Launch geometry: plans of the run-time passes, tiles of the split passes
+    // where the grid has them.  max_bits: largest
     // power-of-two radix (as a bit count) of the FFT plans (0: the default,
     // 4 for complex64 and 3 for complex128); W: z-columns per tile of the
     // strided line passes (0: the largest divisor of m3 within the register
@@ -1248,8 +1249,10 @@ struct Engine : EngineBase {
     // of one field.  Timed with CUDA events (one warm-up, then the mean of
     // three); the fastest is kept.
     // Results are cached per (grid, precision, device) for the process, so a
-    // set of replicas of the same grid tunes once.  Grids whose passes are
-    // all compile-time kernels (32/64/128 cubes) have nothing to tune.
+    // set of replicas of the same grid tunes once.  Where the default plans are
+    // compile-time kernels of both passes (cubes, planes and x extents of
+    // split_setup) they compete with the run-time tiles; the 32, 64 and 128
+    // cubes are not tuned.
     struct TuneKey {
         int m1, m2, m3, f32, dev;
         bool operator<(const TuneKey& o) const

@@ -4,8 +4,8 @@
 // A 3-D transform of an m1 x m2 x m3 row-major grid (z fastest) is split
 // into passes that each read and write HBM once:
 //   * plane pass   : one x-plane (m2 x m3) per CTA, z- and y-transforms in
-//                    shared memory (used when the plane fits: complex64 up
-//                    to 128^2, complex128 up to 96^2);
+//                    shared memory (used when the plane fits a block: 227
+//                    KB and 512 threads of 32 or 16 values);
 //   * z-line pass  : B contiguous z-rows per CTA;
 //   * strided pass : an n x W tile of lines along y or x, W contiguous
 //                    z-columns wide, so every load and store is a W-element
@@ -28,9 +28,10 @@ namespace ftsp {
 // stream-serialisation attribute starts while the previous kernel drains;
 // griddepcontrol.wait holds it until that kernel has completed and its
 // writes are visible, so only the prologue (constant twiddles into shared
-// memory, index set-up) overlaps.  launch_dependents lets the next pass be
-// scheduled once this CTA has issued its last global reads.  Both are no-ops
-// for launches without the attribute.
+// memory, index set-up) overlaps.  launch_dependents lets the next kernel be
+// scheduled: the split passes call it as soon as their own wait is over, the
+// others once a block has issued its last global reads.  Both are no-ops for
+// launches without the attribute.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -17,29 +17,37 @@
 // value (y0, k1): each tile of either pass reads and writes the same rows, so
 // a pass may run in place.
 //
-// Each 1-D transform along z (x) is two register butterflies, m = A * B (inverse along z: radix A, then B; forward in
-// reversed order, B then A), so the op sits between two radix-B butterflies
-// of the same thread and a pass is five register phases with four
-// shared-memory exchanges, whatever the length:
+// Each 1-D transform along z (x) is two register butterflies, m = A * B
+// (inverse along z: radix A, then B; forward in reversed order, B then A), so
+// the op sits between two radix-B butterflies of the same thread and a pass is
+// five register phases with four shared-memory exchanges, whatever the length:
 //     Y1 | A | B op B | A | Y1      (real space; Y2 | A | B op B | A | Y2)
+// (k_cube_k, the k-space pass of the 96 and 128 cubes, has three phases and two
+// exchanges.)
 //
 // Why split: one yz plane per block (k_plane) leaves one block of few warps
 // per SM on planes of mixed radix and does not fit at all above 112^2 in
 // complex128, where the y transform became two more passes over memory.  The
-// tiles here are 8-40 KB, so several blocks share an SM and hide each
-// other's loads and barriers, and every grid takes two passes per segment.
+// tiles here are 8-40 KB (k_cube_k at 128: 74 KB; long extents more, up to the
+// 225 KB of a block), so several blocks share an SM and hide each other's loads
+// and barriers, and every grid whose extents have two radices takes two passes
+// per segment.
 // Measured on one B200, whole calls with the plane and line passes of
 // passes.cuh and with these, in turn: chain of 50 segments at 128^3 complex128
-// 3.56 -> 1.98 ms (72.7 -> 40 us per segment, 10.3 at the measured copy rate);
+// 3.56 -> 1.98 ms (72.7 -> 40 us per segment; its six field transfers, one of
+// them the stored propagator's, take 31 at the measured copy rate);
 // 40 segments at 90 x 125 x 100 complex128 5.28 -> 2.00 ms; step at 96^3
 // complex64, N = 32, 8.7 -> 2.1 ms; step at 64^3 complex64, N = 50, 1.44 -> 1.15
-// ms.  Both passes are bound by issue slots and by the latency of their
-// dependent phases, not by memory: at 128^3 complex64 the real-space pass
-// issues 0.41 instructions per cycle and scheduler over 22 K active cycles.
+// ms.  A pass alone is bound by issue slots and by the latency of its dependent
+// phases: at 128^3 complex64 the real-space pass issues 0.41 instructions per
+// cycle and scheduler over 22 K active cycles.  In a step graph the passes
+// overlap: 101 MB in 20.4 us per segment there, 0.75 of the copy rate.
 //
 // The radices come from a plan: RtPlan reads them from the geometry (a
 // uniform switch per phase; any extents that factor into two radices),
-// CubePlan has every size at compile time (the production cubes).
+// CubePlan has every size at compile time (real space: the square planes of the
+// production cubes with any x extent; k space: the cubes), XPlan the x extents
+// 32, 64 and 128.
 #pragma once
 
 #include "passes.cuh"

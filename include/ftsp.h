@@ -81,9 +81,9 @@ typedef struct ftsp_config {
                                     rollback after a non-finite step (the
                                     reference's Ntmp / max_nan_restarts recovery,
                                     complexLangevin.cu:583-636); 0: off          */
-    int autotune;                /* 1: time the launch-geometry alternatives of the
-                                    runtime-plan passes at creation (cached per
-                                    grid in the process); no reference counterpart */
+    int autotune;                /* 1: time the launch-geometry alternatives at
+                                    creation (cached per grid in the process); no
+                                    reference counterpart                      */
     int max_restarts;            /* rollbacks allowed (restart_interval > 0) before a
                                     non-finite step becomes final: the reference's
                                     max_nan_restarts (param.h:74,
@@ -334,12 +334,15 @@ int ftsp_learn_set_weights(ftsp_handle* h, const float* w, int n);
  * target weights (loss = sum m (z - t)^2 / sum m).  For gradient checks. */
 int ftsp_learn_grad(ftsp_handle* h, const float* x, const float* t, const float* m, int n, double* loss, float* grad);
 
-/* Launch geometry chosen for the handle's grid (autotune = 1): FFT radix
- * cap, tile width of the k-space pass, how many alternatives were timed and
- * the time of one bond and one segment pass (grids whose extents have no two
- * radices: of one forward + inverse 3-D transform) with the chosen and with
- * the default geometry.  compile_time = 1: every pass of this grid is a compile-time
- * kernel and nothing was tuned.  No reference counterpart. */
+/* Launch geometry chosen for the handle's grid (autotune = 1): radix cap of
+ * the run-time FFT passes (without effect on a grid that runs the split
+ * passes, whose extents have two radices), tile width of the k-space (x) pass,
+ * how many alternatives were timed and the time of one bond and one segment
+ * pass (grids without split passes: of one forward + inverse 3-D transform)
+ * with the chosen and with the default geometry.  compile_time = 1: the passes
+ * of the sweeps and of the fused evaluation are compile-time kernels of this
+ * cube (32, 64 or 128) and nothing was tuned; the k-space half of the plain
+ * transforms is a run-time pass at 32 and 64.  No reference counterpart. */
 typedef struct ftsp_tune_info {
     int tuned, cached, compile_time;
     int max_radix, tile_width, candidates;

@@ -1,7 +1,7 @@
-"""Compile-time (production-size) kernels against the oracle.
+"""Production-size and ragged grids against the oracle.
 
-Grids whose extents are 32, 64 or 128 run the specialised passes (plane,
-strided, z-line); other 2/3/5-smooth grids run the runtime-plan passes.
+All of them run the split passes: compile-time plans where the yz plane or
+the x extent is one of the production cubes', run-time plans elsewhere.
 FP64 tolerance 1e-10 (fields, relative to the field's max modulus; records
 relative with a 1e-3 floor); complex64 tolerance 1e-5 on fields and 2e-3 on
 records (FP64 reductions over complex64 fields).

@@ -21,7 +21,7 @@ def case_of(m):
                 counterions={"number": "auto_neutralize", "valence": 1.0}, dt=0.01, init_seed=4)
 
 
-@pytest.mark.parametrize("m", [(32, 32, 32), (64, 64, 64), (20, 18, 15)], ids=lambda m: "%dx%dx%d" % m)
+@pytest.mark.parametrize("m", [(32, 32, 32), (64, 64, 64), (20, 18, 15), (64, 32, 32), (128, 16, 12)], ids=lambda m: "%dx%dx%d" % m)
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_handles_of_one_grid(m, prec):
     from ftspolysol_b200 import Engine, FP32, FP64, SCHEME_SI

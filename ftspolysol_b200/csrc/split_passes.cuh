@@ -209,9 +209,14 @@ constexpr bool split_setup(SplitGeom& g, int m1, int m2, int m3, int value_bytes
     }
     // compile-time plans: the square planes of the production cubes, with any x
     // extent; the x extents of the cubes, with their plane or (32, 64, 128) any
-    // rows of 4 or 8 and whole tiles
+    // rows of 4 or 8 and whole tiles.  128 x 8 in complex64 has half the threads
+    // of the run-time plan and pays beside a run-time real-space pass only where
+    // its blocks cover the SMs (steps with N = 16, run-time and this plan: 64
+    // blocks, 128 x 64 x 32, 745 and 870 us; 135 blocks, 128 x 72 x 60, 985 and
+    // 1039; 200 blocks, 128 x 80 x 80, 1507 and 1295)
     g.plane = square ? m3 : 0;
-    g.xct = g.plane == m1 ? m1 : (m1 == 32 || m1 == 64 || m1 == 128) && (g.Y2 == 4 || g.Y2 == 8) && m3 % 4 == 0 ? m1 : 0;
+    const bool few = m1 == 128 && g.Y2 == 8 && value_bytes == 8 && !square && g.Y1 * (m3 / 4) < 148;
+    g.xct = g.plane == m1 ? m1 : (m1 == 32 || m1 == 64 || m1 == 128) && (g.Y2 == 4 || g.Y2 == 8) && m3 % 4 == 0 && !few ? m1 : 0;
     // real space: as many row groups per block as leave two blocks per SM
     int G = 1;
     for (int t = 2; t <= g.Y2 && !g.plane; ++t)

@@ -43,7 +43,7 @@ def test_chain(m):
     assert abs(Q - ref.mean()) / abs(ref.mean()) < 1e-12
 
 
-@pytest.mark.parametrize("m", [(64, 32, 32), (32, 64, 64), (20, 64, 64), (128, 16, 12), (3, 128, 128), (5, 96, 96), (512, 30, 8), (243, 32, 32),
+@pytest.mark.parametrize("m", [(64, 32, 32), (32, 64, 64), (20, 64, 64), (128, 16, 12), (128, 72, 72), (3, 128, 128), (5, 96, 96), (512, 30, 8), (243, 32, 32),
                                (640, 32, 32)],
                          ids=lambda m: "%dx%dx%d" % m)
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])

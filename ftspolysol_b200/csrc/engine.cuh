@@ -3796,10 +3796,14 @@ struct Engine : EngineBase {
         if constexpr (!F32) {
             FTSP_CUDA(cudaMemcpyAsync(out, p, bytes, cudaMemcpyDeviceToHost, stream));
         } else {
-            // the buffer that set_fields left, or 4 MiB where it was never called
-            if (!stage.p && !ostage.p) ostage.alloc(std::min<size_t>(V_, (size_t)1 << 18));
-            double2* d = stage.p ? stage.p : ostage.p;
-            const size_t chunk = stage.p ? stage.n : ostage.n;
+            // the buffer that set_fields or set_fields_async left (an upload through
+            // the latter has been installed on this stream before, and none is
+            // queued before this call returns), or 16 MiB where neither was called;
+            // pieces of 4 MiB cost 2 ms more per field of 128^3
+            Buf<double2>& buf = stage.p ? stage : astage.p ? astage : ostage;
+            if (!buf.p) buf.alloc(std::min<size_t>(V_, (size_t)1 << 20));
+            double2* d = buf.p;
+            const size_t chunk = buf.n;
             const long long of_step = launches;   // the conversions are no launches of the step
             for (size_t i0 = 0; i0 < n; i0 += chunk) {
                 const size_t m = std::min(chunk, n - i0);
